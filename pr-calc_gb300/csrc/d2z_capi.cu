@@ -201,7 +201,8 @@ using namespace prc;
 struct prc_d2z_ctx {
   int N = 0, H = 0, nr = 0, B = 0, flags = 0, dev = 0, sms = 0;
   int win_var = 0;   // window-pass variant (prc_d2z_tune)
-  int slots_b = 0;   // radius slots allocated
+  int slots_b = 0;   // radius slots allocated (one more than B for an odd B of paired sweeps)
+  int waves = 1;     // CTA waves of the window and z passes (batches: kBatchWaves)
   long long NN = 0, slot_f2 = 0;
   double box = 0, A = 0, dinit = 1;
   std::vector<double> R, Bb;
@@ -302,6 +303,11 @@ int grid_for(int items, int per_cta, int occ, int sms) {
   return (int)(need < cap ? need : cap);
 }
 
+// A context alone runs its passes as one wave of resident CTAs.  Where kernels
+// of several streams share the GPU, a CTA that has to wait for its place
+// would start its whole share late; smaller shares even that out.
+constexpr int kBatchWaves = 4;
+
 template <class T> int dalloc(T** p, size_t count, const char* what) {
   cudaError_t e = cudaMalloc((void**)p, count * sizeof(T));
   if (e != cudaSuccess) {
@@ -340,6 +346,31 @@ void free_all(prc_d2z_ctx* c) {
   c->pev.clear();
 }
 
+// Radii per sweep.  Sweeps on pairs of radii (fft2.cuh) take an even number:
+// an odd radius batch is rounded up, or down when the extra slot could not be
+// allocated.  The pair kernels are left for the single-radius ones by the
+// faithful window, by a tuned window variant, and where there is one radius
+// or one slot.
+bool paired(const prc_d2z_ctx* c) {
+  return c->ksl.pair && !(c->flags & PRC_FLAG_FAITHFUL_WINDOW) && c->win_var == 0 && c->nr > 1 && c->slots_b > 1;
+}
+int sweep_len(const prc_d2z_ctx* c) {
+  if (!paired(c) || c->B % 2 == 0) return c->B;
+  return c->B + 1 <= c->slots_b ? c->B + 1 : c->B - 1;
+}
+
+// Radius slots for a radius batch of B into *out: with one more for an odd
+// batch of a size with pair kernels, if that can be had.
+int alloc_slots(const prc_d2z_ctx* c, int B, float2** out, int* n) {
+  if (c->ksl.pair && c->nr > 1 && B % 2 == 1) {
+    *n = B + 1;
+    if (cudaMalloc((void**)out, (size_t)c->slot_f2 * *n * sizeof(float2)) == cudaSuccess) return PRC_OK;
+    cudaGetLastError();
+  }
+  *n = B;
+  return dalloc(out, (size_t)c->slot_f2 * B, "radius slots");
+}
+
 // main-array segment of a column pass along x (rows ix) or y (rows iy)
 TileSeg mseg(const prc_d2z_ctx* c, const float2* in, float2* out, bool xpass) {
   TileSeg s;
@@ -369,16 +400,30 @@ TileSeg qseg(const prc_d2z_ctx* c, const float2* in, float2* out, bool transpose
   return s;
 }
 
+// The main array of pair slots as the inverse y pass sees it: blocks of XB
+// planes, rows of XB * H contiguous elements.
+void pair_rows(const KernelSet& ks, TileSeg* s) {
+  const int N = ks.N, w = ks.pair_xb * (N / 2);
+  s->row_stride = w;
+  s->outer_stride = N * w;
+  s->n_outer = N / ks.pair_xb;
+  s->tpo = w / ks.pair_tile_w;
+}
+
 // one column pass over the main array and the Nyquist plane
-void run_tile(prc_d2z_ctx* c, int mode, TileSeg s0, TileSeg s1, int gy, int nb = 1, int r0 = 0, int first = 0) {
+// (pair: TM_WIN or TM_INV on pair slots; gy then counts pairs)
+void run_tile(prc_d2z_ctx* c, int mode, TileSeg s0, TileSeg s1, int gy, int nb = 1, int r0 = 0, int first = 0,
+              bool pair = false) {
   TileArgs a;
   memset(&a, 0, sizeof(a));
   const bool faithful = mode == TM_WIN && (c->flags & PRC_FLAG_FAITHFUL_WINDOW);
   const int wv = faithful ? 0 : c->win_var;  // the faithful window runs on variant 0's tiles
-  if (mode == TM_WIN || mode == TM_ACC) {  // these passes may use narrower tiles
-    const int tw = mode == TM_WIN ? c->ksl.tile_w_winv[wv] : c->ksl.tile_w_acc;
+  if (pair || mode == TM_WIN || mode == TM_ACC) {  // these passes may use narrower tiles
+    const int tw = pair ? (mode == TM_WIN ? c->ksl.pair_tile_w_win : c->ksl.pair_tile_w)
+                        : mode == TM_WIN ? c->ksl.tile_w_winv[wv] : c->ksl.tile_w_acc;
     s0.tpo = (s0.nyq ? c->N : c->H) / tw;
     s1.tpo = (s1.nyq ? c->N : c->H) / tw;
+    if (pair && mode == TM_INV) pair_rows(c->ksl, &s0);
   }
   a.seg[0] = s0;
   a.seg[1] = s1;
@@ -396,25 +441,27 @@ void run_tile(prc_d2z_ctx* c, int mode, TileSeg s0, TileSeg s1, int gy, int nb =
     for (int b = 0; b < nb; ++b) a.kr[b] = (float)c->R[r0 + b];
   } else if (mode == TM_WIN || mode == TM_ACC) {
     for (int b = 0; b < nb; ++b) a.kr[b] = c->kr[r0 + b];
+    if (pair && nb % 2) a.kr[nb] = a.kr[nb - 1];  // the last pair's second half: any radius (its barrier never wins)
   }
   const int tiles = s0.n_outer * s0.tpo + s1.n_outer * s1.tpo;
-  const int occ = (mode == TM_ACC) ? c->ksl.occ_tile_acc
+  const int occ = pair ? (mode == TM_WIN ? c->ksl.occ_pair_win : c->ksl.occ_pair_inv)
+                : (mode == TM_ACC) ? c->ksl.occ_tile_acc
                 : faithful         ? c->ksl.occ_win_faithful
                 : (mode == TM_WIN) ? c->ksl.occ_winv[wv] : c->ksl.occ_tile;
-  dim3 grid(grid_for(tiles, 1, occ, c->sms), gy, 1);
+  dim3 grid(grid_for(tiles, 1, occ * (mode == TM_WIN ? c->waves : 1), c->sms), gy, 1);
   if (mode == TM_WIN && c->N <= 128) {
     // fewer tiles than two waves of resident CTAs: the sweep's radii are
     // split over blockIdx.y as well (the kernels of grids up to 128 read
     // their radius range from it)
     const long long want = 2LL * occ * c->sms;
-    if (tiles < want) grid.y = (unsigned)std::min<long long>(nb, (want + tiles - 1) / tiles);
+    if (tiles < want) grid.y = (unsigned)std::min<long long>(pair ? (nb + 1) / 2 : nb, (want + tiles - 1) / tiles);
   }
   const int kind = mode == TM_FWD ? PRC_KIND_COL_FWD
                  : mode == TM_INV ? PRC_KIND_COL_INV
                  : mode == TM_WIN ? PRC_KIND_WIN_X : PRC_KIND_ADJ_X;
   {
     Prof pf(c, kind);
-    c->ks->tile(c->ksl, mode, grid, c->st, a);
+    (pair ? c->ks->pair_tile : c->ks->tile)(c->ksl, mode, grid, c->st, a);
   }
   c->launches++;
 }
@@ -458,8 +505,10 @@ void enqueue_sweeps(prc_d2z_ctx* c, float* d_z, uint8_t* d_am, double* sig, floa
                     uint8_t* am_out = nullptr, bool withhold = false) {
   const int N = c->N, H = c->H;
   const long long NN = c->NN;
-  for (int r0 = 0; r0 < c->nr; r0 += c->B) {
-    const int nb = (c->nr - r0 < c->B) ? c->nr - r0 : c->B;
+  const int B = sweep_len(c);
+  for (int r0 = 0; r0 < c->nr; r0 += B) {
+    const int nb = (c->nr - r0 < B) ? c->nr - r0 : B;
+    const bool pair = paired(c) && nb > 1;
     SweepArgs sa;
     memset(&sa, 0, sizeof(sa));
     sa.slots = c->slots;
@@ -478,14 +527,19 @@ void enqueue_sweeps(prc_d2z_ctx* c, float* d_z, uint8_t* d_am, double* sig, floa
     sa.first = (r0 == 0);
     sa.as = c->as;
     for (int b = 0; b < nb; ++b) sa.cb[b] = c->cb[r0 + b];
+    if (pair && nb % 2) sa.cb[nb] = NAN;  // never wins
     float2* U = c->slots;
+    float2* UQ = U + NN * H * (pair ? 2 : 1);  // Nyquist plane (of the first pair or radius)
     // window + inverse x pass: spectrum -> slots (Nyquist plane transposed)
-    run_tile(c, TM_WIN, mseg(c, c->spec, U, true), qseg(c, c->spec + NN * H, U + NN * H, true), 1, nb, r0);
+    run_tile(c, TM_WIN, mseg(c, c->spec, U, true), qseg(c, c->spec + NN * H, UQ, true), 1, nb, r0, 0, pair);
     // inverse y pass of every slot, in place
-    run_tile(c, TM_INV, mseg(c, U, U, false), qseg(c, U + NN * H, U + NN * H, false), nb);
+    run_tile(c, TM_INV, mseg(c, U, U, false), qseg(c, UQ, UQ, false), pair ? (nb + 1) / 2 : nb, 1, 0, 0, pair);
     {
       Prof pf(c, PRC_KIND_C2R_Z);
-      c->ks->c2r_z(c->ksl, grid_for(N * N, c->ksl.c2r_lines, c->ksl.occ_c2r, c->sms), c->st, sa);
+      if (pair)
+        c->ks->pair_c2r(c->ksl, grid_for(N * N, c->ksl.pair_lines, c->ksl.occ_pair_c2r * c->waves, c->sms), c->st, sa);
+      else
+        c->ks->c2r_z(c->ksl, grid_for(N * N, c->ksl.c2r_lines, c->ksl.occ_c2r, c->sms), c->st, sa);
     }
     c->launches++;
   }
@@ -569,8 +623,15 @@ void batch_enqueue(prc_d2z_batch* b, const float* const* delta, float* const* zr
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // A box joins a grouped launch when its size has grouped kernels and it asks
-// for nothing they leave out (the faithful window runs per box).
-bool groupable(const prc_d2z_ctx* c) { return c->ksl.grouped && !(c->flags & PRC_FLAG_FAITHFUL_WINDOW); }
+// for nothing they leave out: the faithful window and a single radius (or
+// slot) run per box.  (A tuned window variant is not used there.)
+bool groupable(const prc_d2z_ctx* c) {
+  return c->ksl.grouped && !(c->flags & PRC_FLAG_FAITHFUL_WINDOW) && c->nr > 1 && c->slots_b > 1;
+}
+// radii per sweep of a grouped box (its window variant does not matter)
+int grouped_len(const prc_d2z_ctx* c) {
+  return c->B % 2 == 0 ? c->B : c->B + 1 <= c->slots_b ? c->B + 1 : c->B - 1;
+}
 
 // Groups of equal grid size, their sweeps and the layout of their tables.
 // Sizes without grouped kernels keep per-box launches (no group).
@@ -595,15 +656,18 @@ int batch_group_setup(prc_d2z_batch* b) {
       if (b->ctx[i]->N == N && groupable(b->ctx[i])) {
         g.boxes.push_back(i);
         const prc_d2z_ctx* c = b->ctx[i];
-        g.nsweeps = std::max(g.nsweeps, (c->nr + c->B - 1) / c->B);
+        g.nsweeps = std::max(g.nsweeps, (c->nr + grouped_len(c) - 1) / grouped_len(c));
       }
     for (int sw = 0; sw < g.nsweeps; ++sw) {
       std::vector<int> bx;
       for (int i : g.boxes)
-        if (b->ctx[i]->nr > sw * b->ctx[i]->B) bx.push_back(i);
-      auto nb_of = [&](int i) { return std::min(b->ctx[i]->B, b->ctx[i]->nr - sw * b->ctx[i]->B); };
-      // most radii first: the boxes with more than y radii in the sweep are a
-      // prefix, which the inverse y pass's slot y takes
+        if (b->ctx[i]->nr > sw * grouped_len(b->ctx[i])) bx.push_back(i);
+      auto nb_of = [&](int i) {
+        const int B = grouped_len(b->ctx[i]);
+        return std::min(B, b->ctx[i]->nr - sw * B);
+      };
+      // most radii first: the boxes with more than y pairs in the sweep are a
+      // prefix, which the inverse y pass's pair y takes
       std::stable_sort(bx.begin(), bx.end(), [&](int x, int y) { return nb_of(x) > nb_of(y); });
       std::vector<int> nbs;
       for (int i : bx) nbs.push_back(nb_of(i));
@@ -673,14 +737,15 @@ void batch_group_fill(prc_d2z_batch* b, const float* const* delta, float* const*
         const int i = g.sw_box[sw][k];
         const prc_d2z_ctx* c = b->ctx[i];
         const long long NN = c->NN, H = c->H;
-        const int r0 = sw * c->B, nb = g.sw_nb[sw][k];
+        const int r0 = sw * grouped_len(c), nb = g.sw_nb[sw][k];
         float2* U = c->slots;
         BoxCol w, v;
         memset(&w, 0, sizeof w);
         memset(&v, 0, sizeof v);
-        w.in0 = c->spec, w.out0 = U, w.in1 = c->spec + NN * H, w.out1 = U + NN * H, w.nb = nb;
+        w.in0 = c->spec, w.out0 = U, w.in1 = c->spec + NN * H, w.out1 = U + 2 * NN * H, w.nb = nb;
         for (int q = 0; q < nb; ++q) w.kr[q] = c->kr[r0 + q];
-        v.in0 = U, v.out0 = U, v.in1 = U + NN * H, v.out1 = U + NN * H, v.nb = nb;
+        if (nb % 2) w.kr[nb] = w.kr[nb - 1];  // as in run_tile
+        v.in0 = U, v.out0 = U, v.in1 = U + 2 * NN * H, v.out1 = U + 2 * NN * H, v.nb = nb;
         memcpy(h + g.o_win[sw] + k * sizeof(BoxCol), &w, sizeof w);
         memcpy(h + g.o_inv[sw] + k * sizeof(BoxCol), &v, sizeof v);
         BoxLine L;
@@ -690,6 +755,7 @@ void batch_group_fill(prc_d2z_batch* b, const float* const* delta, float* const*
         L.argmax = L.argmax_out = argmax ? argmax[i] : nullptr;
         L.nb = nb, L.r0 = r0, L.first = (sw == 0), L.as = c->as;
         for (int q = 0; q < nb; ++q) L.cb[q] = c->cb[r0 + q];
+        if (nb % 2) L.cb[nb] = NAN;  // never wins
         memcpy(h + g.o_line[sw] + k * sizeof(BoxLine), &L, sizeof L);
       }
     }
@@ -708,7 +774,7 @@ void batch_enqueue_grouped(prc_d2z_batch* b, const float* const* delta, float* c
     const BatchGroup& g = b->groups[gi];
     const prc_d2z_ctx* c0 = b->ctx[g.boxes[0]];
     const KernelSet& ks = c0->ksl;
-    const int N = g.N, H = N / 2, sms = c0->sms, nbox = (int)g.boxes.size();
+    const int N = g.N, H = N / 2, sms = c0->sms, nbox = (int)g.boxes.size(), waves = c0->waves;
     const long long NN = c0->NN;
     float2* S0 = c0->spec;
     float2* U0 = c0->slots;
@@ -717,9 +783,11 @@ void batch_enqueue_grouped(prc_d2z_batch* b, const float* const* delta, float* c
     auto cols = [&](int mode, TileSeg s0, TileSeg s1, size_t o, int nboxes, int gy, const int* nvb) {
       TileArgs a;
       memset(&a, 0, sizeof(a));
-      if (mode == TM_WIN) {
-        s0.tpo = H / ks.tile_w_mb_win;
-        s1.tpo = N / ks.tile_w_mb_win;
+      if (mode != TM_FWD) {
+        const int tw = mode == TM_WIN ? ks.pair_tile_w_win : ks.pair_tile_w;
+        s0.tpo = H / tw;
+        s1.tpo = N / tw;
+        if (mode == TM_INV) pair_rows(ks, &s0);
       }
       a.seg[0] = s0;
       a.seg[1] = s1;
@@ -730,8 +798,9 @@ void batch_enqueue_grouped(prc_d2z_batch* b, const float* const* delta, float* c
       if (nvb)
         for (int y = 0; y < gy; ++y) a.nvb[y] = nvb[y];
       const int tpb = s0.n_outer * s0.tpo + s1.n_outer * s1.tpo;
-      const int occ = mode == TM_WIN ? ks.occ_mb_win : ks.occ_mb_tile;
-      ks.tile_mb(ks, mode, dim3(grid_for(tpb * (nvb ? nvb[0] : nboxes), 1, occ, sms), gy, 1), g.st, a);
+      const int occ = mode == TM_WIN ? ks.occ_mb_win : mode == TM_INV ? ks.occ_mb_inv : ks.occ_mb_tile;
+      ks.tile_mb(ks, mode, dim3(grid_for(tpb * (nvb ? nvb[0] : nboxes), 1, occ * (mode == TM_WIN ? waves : 1), sms), gy, 1),
+                 g.st, a);
       ++launches;
     };
     cols(TM_FWD, mseg(c0, S0, S0, false), qseg(c0, S0 + NN * (H + 1), S0 + NN * H, true), g.o_fy, nbox, 1, nullptr);
@@ -739,15 +808,16 @@ void batch_enqueue_grouped(prc_d2z_batch* b, const float* const* delta, float* c
     for (int sw = 0; sw < g.nsweeps; ++sw) {
       const int ns = (int)g.sw_box[sw].size();
       const std::vector<int>& nbs = g.sw_nb[sw];
-      cols(TM_WIN, mseg(c0, S0, U0, true), qseg(c0, S0 + NN * H, U0 + NN * H, true), g.o_win[sw], ns, 1, nullptr);
+      float2* UQ = U0 + 2 * NN * H;
+      cols(TM_WIN, mseg(c0, S0, U0, true), qseg(c0, S0 + NN * H, UQ, true), g.o_win[sw], ns, 1, nullptr);
+      const int np = (nbs[0] + 1) / 2;
       int nvb[kMaxBatch];
-      for (int y = 0; y < nbs[0]; ++y) {
+      for (int y = 0; y < np; ++y) {
         int k = 0;
-        while (k < ns && nbs[k] > y) ++k;
+        while (k < ns && nbs[k] > 2 * y) ++k;
         nvb[y] = k;
       }
-      cols(TM_INV, mseg(c0, U0, U0, false), qseg(c0, U0 + NN * H, U0 + NN * H, false), g.o_inv[sw], ns, nbs[0],
-           nvb);
+      cols(TM_INV, mseg(c0, U0, U0, false), qseg(c0, UQ, UQ, false), g.o_inv[sw], ns, np, nvb);
       SweepArgs sa;
       memset(&sa, 0, sizeof(sa));
       sa.slot_stride = c0->slot_f2;
@@ -756,7 +826,7 @@ void batch_enqueue_grouped(prc_d2z_batch* b, const float* const* delta, float* c
       sa.argmax = argmax ? argmax[g.sw_box[sw][0]] : nullptr;
       sa.box = reinterpret_cast<const BoxLine*>(b->d_tab + g.o_line[sw]);
       sa.nbox = ns;
-      ks.c2r_z_mb(ks, grid_for(N * N * ns, ks.c2r_lines, ks.occ_mb_c2r, sms), g.st, sa);
+      ks.c2r_z_mb(ks, grid_for(N * N * ns, ks.pair_lines, ks.occ_mb_c2r * waves, sms), g.st, sa);
       launches += 2;
     }
     launches += 1;
@@ -845,7 +915,7 @@ int prc_d2z_create(const prc_d2z_desc* d, prc_d2z_ctx** out) {
   }
   const long long n3l = (long long)c->NN * c->N;
   if ((st = dalloc(&c->spec, (size_t)c->slot_f2, "spectrum")) != PRC_OK ||
-      (st = dalloc(&c->slots, (size_t)c->slot_f2 * c->B, "radius slots")) != PRC_OK ||
+      (st = alloc_slots(c, c->B, &c->slots, &c->slots_b)) != PRC_OK ||
       (st = dalloc(&c->tw, (size_t)c->N, "twiddles")) != PRC_OK ||
       (st = dalloc(&c->sig, (size_t)c->nr, "sigma accumulators")) != PRC_OK ||
       (st = dalloc(&c->dB, (size_t)c->nr, "barrier gradient")) != PRC_OK ||
@@ -1416,10 +1486,11 @@ int prc_d2z_tune(prc_d2z_ctx* c, int radius_batch, int win_variant) {
     if ((st = set_device(c)) != PRC_OK) return st;
     PRC_CU(cudaStreamSynchronize(c->st), "prc_d2z_tune");
     float2* ns = nullptr;
-    if ((st = dalloc(&ns, (size_t)c->slot_f2 * B, "radius slots")) != PRC_OK) return st;
+    int n = 0;
+    if ((st = alloc_slots(c, B, &ns, &n)) != PRC_OK) return st;
     cudaFree(c->slots);
     c->slots = ns;
-    c->slots_b = B;
+    c->slots_b = n;
   }
   c->B = B;
   c->win_var = win_variant;
@@ -1478,6 +1549,7 @@ int prc_d2z_batch_create(int n_boxes, const prc_d2z_desc* descs, int n_streams, 
     prc_d2z_desc d = descs[i];
     d.stream = b->streams[k % n_streams];
     int st = prc_d2z_create(&d, &b->ctx[i]);
+    if (st == PRC_OK && n_streams > 1) b->ctx[i]->waves = kBatchWaves;
     if (st != PRC_OK) {
       batch_free(b);
       delete b;

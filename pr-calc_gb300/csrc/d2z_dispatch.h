@@ -34,12 +34,18 @@ struct KernelSet {
   void (*c2r_z)(const KernelSet&, int grid, cudaStream_t, const SweepArgs&);
   void (*adj_z)(const KernelSet&, int grid, cudaStream_t, const AdjArgs&);
   void (*c2r_plain)(const KernelSet&, int grid, cudaStream_t, const AdjArgs&);
+  // pairs of radii (fft2.cuh), when compiled for this size (pair = 1): planes
+  // per block of a pair slot, tile widths, lines per CTA step, resident CTAs
+  int pair;
+  int pair_xb, pair_tile_w, pair_tile_w_win, pair_lines;
+  int occ_pair_inv, occ_pair_win, occ_pair_c2r;
+  void (*pair_tile)(const KernelSet&, int mode, dim3 grid, cudaStream_t, const TileArgs&);  // TM_INV, TM_WIN
+  void (*pair_c2r)(const KernelSet&, int grid, cudaStream_t, const SweepArgs&);
   // grouped launches (several boxes of this size per launch), when compiled
-  // for this size (grouped = 1): forward z pass, column passes (TM_FWD,
-  // TM_INV, TM_WIN with window variant 0), inverse z pass
+  // for this size (grouped = 1): forward z pass, forward column passes, and
+  // the sweep's passes on pairs of radii (TM_WIN, TM_INV, inverse z)
   int grouped;
-  int tile_w_mb_win;
-  int occ_mb_tile, occ_mb_win, occ_mb_c2r, occ_mb_r2c;
+  int occ_mb_tile, occ_mb_inv, occ_mb_win, occ_mb_c2r, occ_mb_r2c;
   void (*r2c_z_mb)(const KernelSet&, int grid, cudaStream_t, const BoxR2c* box, int nbox, const float2* tw);
   void (*tile_mb)(const KernelSet&, int mode, dim3 grid, cudaStream_t, const TileArgs&);
   void (*c2r_z_mb)(const KernelSet&, int grid, cudaStream_t, const SweepArgs&);

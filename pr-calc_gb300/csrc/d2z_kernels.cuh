@@ -130,7 +130,7 @@ struct TileArgs {
   float dk, kmax;          // faithful window: dk = 2 pi / box and kmax = dk * N, in float
   float kr[kMaxBatch];     // dk * R_b (faithful window: R_b)
   // grouped launches: the boxes (sorted by nb, largest first), their count,
-  // and per slot y of the inverse y pass the number of boxes with nb > y
+  // and per pair y of the inverse y pass the number of boxes with more pairs
   const BoxCol* box;
   int nbox;
   int nvb[kMaxBatch];

@@ -5,6 +5,7 @@
 #include "d2z_dispatch.h"
 #include "d2z_kernels.cuh"
 #include "d2z_lines.cuh"
+#include "d2z_lines2.cuh"
 
 namespace prc {
 
@@ -111,19 +112,11 @@ template <int N> struct ColLaunch<N, true> {
       default: k_col<N, TM_ACC><<<grid, CA::THREADS, CSA, st>>>(a); break;
     }
   }
-  // grouped launches (several boxes of this size per launch; window variant 0)
+  // grouped forward column passes (several boxes of this size per launch)
   static constexpr bool GROUPED = N <= 256 && PCfg<N>::on;
-  using W0 = typename Win<0>::K;
-  static constexpr size_t WS0 = (size_t)W0::smem_f2 * sizeof(float2);
-  template <int MODE> static void* fn_mb() { return reinterpret_cast<void*>(&k_col<N, MODE, 0, true>); }
-  static void launch_mb(int mode, dim3 grid, cudaStream_t st, const TileArgs& a) {
-    if constexpr (GROUPED) {
-      switch (mode) {
-        case TM_FWD: k_col<N, TM_FWD, 0, true><<<grid, THREADS, CS, st>>>(a); break;
-        case TM_INV: k_col<N, TM_INV, 0, true><<<grid, THREADS, CS, st>>>(a); break;
-        default: k_col<N, TM_WIN, 0, true><<<grid, W0::THREADS, WS0, st>>>(a); break;
-      }
-    }
+  static void* fn_mb() { return reinterpret_cast<void*>(&k_col<N, TM_FWD, 0, true>); }
+  static void launch_mb(dim3 grid, cudaStream_t st, const TileArgs& a) {
+    if constexpr (GROUPED) k_col<N, TM_FWD, 0, true><<<grid, THREADS, CS, st>>>(a);
   }
 };
 
@@ -135,7 +128,6 @@ template <int N, bool PAIR = PCfg<N>::on> struct C2rLaunch {
   static constexpr int NFN = 1;
   static void* fn(int) { return reinterpret_cast<void*>(&k_c2r_z<N>); }
   static void launch(int grid, cudaStream_t st, const SweepArgs& a) { k_c2r_z<N><<<grid, THREADS, BYTES, st>>>(a); }
-  static void launch_mb(int, cudaStream_t, const SweepArgs&) {}
 };
 template <int N> struct C2rLaunch<N, true> {
   static constexpr int THREADS = PK<N>::THREADS, NG = PK<N>::NG;
@@ -152,15 +144,43 @@ template <int N> struct C2rLaunch<N, true> {
       else k_c2r_zp<N, false, false><<<grid, THREADS, BYTES, st>>>(a);
     }
   }
+};
+
+// The sweep's passes on pairs of radii (grids with both a column and a z-line
+// plan): window + inverse x, inverse y, inverse z; MB: grouped launches.
+template <int N, bool ON = C2Cfg<N>::on> struct PairLaunch {
+  static constexpr bool on = false;
+};
+template <int N> struct PairLaunch<N, true> {
+  static constexpr bool on = true;
+  using KW = CK2<N, TM_WIN>;
+  using KI = CK2<N, TM_INV>;
+  using KZ = PK2<N>;
+  template <bool MB> static void* win_fn() { return reinterpret_cast<void*>(&k_col2<N, TM_WIN, MB>); }
+  template <bool MB> static void* inv_fn() { return reinterpret_cast<void*>(&k_col2<N, TM_INV, MB>); }
+  template <bool AM, bool SIG, bool MB> static void* z_fn() { return reinterpret_cast<void*>(&k_c2r_zp2<N, AM, SIG, MB>); }
+  template <bool MB> static void tile(int mode, dim3 grid, cudaStream_t st, const TileArgs& a) {
+    if (mode == TM_WIN) k_col2<N, TM_WIN, MB><<<grid, KW::THREADS, KW::bytes, st>>>(a);
+    else k_col2<N, TM_INV, MB><<<grid, KI::THREADS, KI::bytes, st>>>(a);
+  }
+  static void c2r(int grid, cudaStream_t st, const SweepArgs& a) {
+    if (a.sig_acc) {
+      if (a.argmax) k_c2r_zp2<N, true, true><<<grid, KZ::THREADS, KZ::bytes, st>>>(a);
+      else k_c2r_zp2<N, false, true><<<grid, KZ::THREADS, KZ::bytes, st>>>(a);
+    } else {
+      if (a.argmax) k_c2r_zp2<N, true, false><<<grid, KZ::THREADS, KZ::bytes, st>>>(a);
+      else k_c2r_zp2<N, false, false><<<grid, KZ::THREADS, KZ::bytes, st>>>(a);
+    }
+  }
   // grouped: a.argmax != null means every box of the launch records its argmax
-  template <bool AM> static void* f_mb() { return reinterpret_cast<void*>(&k_c2r_zp<N, AM, false, true>); }
-  static void launch_mb(int grid, cudaStream_t st, const SweepArgs& a) {
-    if (a.argmax) k_c2r_zp<N, true, false, true><<<grid, THREADS, BYTES, st>>>(a);
-    else k_c2r_zp<N, false, false, true><<<grid, THREADS, BYTES, st>>>(a);
+  static void c2r_mb(int grid, cudaStream_t st, const SweepArgs& a) {
+    if (a.argmax) k_c2r_zp2<N, true, false, true><<<grid, KZ::THREADS, KZ::bytes, st>>>(a);
+    else k_c2r_zp2<N, false, false, true><<<grid, KZ::THREADS, KZ::bytes, st>>>(a);
   }
 };
 
 template <int N> struct Launchers {
+  using PL = PairLaunch<N>;
   using CL = ColLaunch<N>;
   using CR = C2rLaunch<N>;
   using LL = LK<N>;
@@ -195,19 +215,35 @@ template <int N> struct Launchers {
     }
     ks->occ_tile_win = ks->occ_winv[0];
     ks->tile_w_win = ks->tile_w_winv[0];
+    if constexpr (PL::on) {
+      void* w = PL::template win_fn<false>();
+      void* v = PL::template inv_fn<false>();
+      void* z[4] = {PL::template z_fn<false, false, false>(), PL::template z_fn<true, false, false>(),
+                    PL::template z_fn<false, true, false>(), PL::template z_fn<true, true, false>()};
+      if ((e = smem(w, PL::KW::bytes)) != cudaSuccess) return e;
+      if ((e = smem(v, PL::KI::bytes)) != cudaSuccess) return e;
+      for (void* f : z)
+        if ((e = smem(f, PL::KZ::bytes)) != cudaSuccess) return e;
+      if ((e = occ(&ks->occ_pair_win, w, PL::KW::THREADS, PL::KW::bytes)) != cudaSuccess) return e;
+      if ((e = occ(&ks->occ_pair_inv, v, PL::KI::THREADS, PL::KI::bytes)) != cudaSuccess) return e;
+      if ((e = occ(&ks->occ_pair_c2r, z[1], PL::KZ::THREADS, PL::KZ::bytes)) != cudaSuccess) return e;
+    }
     if constexpr (CL::GROUPED) {
-      void* fm = CL::template fn_mb<TM_FWD>();
-      void* im = CL::template fn_mb<TM_INV>();
-      void* wm = CL::template fn_mb<TM_WIN>();
+      void* fm = CL::fn_mb();
+      void* im = PL::template inv_fn<true>();
+      void* wm = PL::template win_fn<true>();
+      void* z0 = PL::template z_fn<false, false, true>();
+      void* z1 = PL::template z_fn<true, false, true>();
       if ((e = smem(fm, CL::CS)) != cudaSuccess) return e;
-      if ((e = smem(im, CL::CS)) != cudaSuccess) return e;
-      if ((e = smem(wm, CL::WS0)) != cudaSuccess) return e;
-      if ((e = smem(CR::template f_mb<false>(), CR::BYTES)) != cudaSuccess) return e;
-      if ((e = smem(CR::template f_mb<true>(), CR::BYTES)) != cudaSuccess) return e;
+      if ((e = smem(im, PL::KI::bytes)) != cudaSuccess) return e;
+      if ((e = smem(wm, PL::KW::bytes)) != cudaSuccess) return e;
+      if ((e = smem(z0, PL::KZ::bytes)) != cudaSuccess) return e;
+      if ((e = smem(z1, PL::KZ::bytes)) != cudaSuccess) return e;
       if ((e = smem(&k_r2c_z<N, true>, LS)) != cudaSuccess) return e;
-      if ((e = occ(&ks->occ_mb_tile, im, CL::THREADS, CL::CS)) != cudaSuccess) return e;
-      if ((e = occ(&ks->occ_mb_win, wm, CL::W0::THREADS, CL::WS0)) != cudaSuccess) return e;
-      if ((e = occ(&ks->occ_mb_c2r, CR::template f_mb<true>(), CR::THREADS, CR::BYTES)) != cudaSuccess) return e;
+      if ((e = occ(&ks->occ_mb_tile, fm, CL::THREADS, CL::CS)) != cudaSuccess) return e;
+      if ((e = occ(&ks->occ_mb_inv, im, PL::KI::THREADS, PL::KI::bytes)) != cudaSuccess) return e;
+      if ((e = occ(&ks->occ_mb_win, wm, PL::KW::THREADS, PL::KW::bytes)) != cudaSuccess) return e;
+      if ((e = occ(&ks->occ_mb_c2r, z1, PL::KZ::THREADS, PL::KZ::bytes)) != cudaSuccess) return e;
       if ((e = occ(&ks->occ_mb_r2c, &k_r2c_z<N, true>, LL::THREADS, LS)) != cudaSuccess) return e;
     }
     if ((e = smem(CL::faithful_fn(), CL::FS)) != cudaSuccess) return e;
@@ -233,10 +269,19 @@ template <int N> struct Launchers {
     if constexpr (CL::GROUPED) k_r2c_z<N, true><<<grid, LL::THREADS, LS, st>>>(nullptr, 1.f, nullptr, nullptr, tw, box, nbox);
   }
   static void tile_mb(const KernelSet&, int mode, dim3 grid, cudaStream_t st, const TileArgs& a) {
-    CL::launch_mb(mode, grid, st, a);
+    if constexpr (CL::GROUPED) {
+      if (mode == TM_FWD) CL::launch_mb(grid, st, a);
+      else PL::template tile<true>(mode, grid, st, a);
+    }
   }
   static void c2r_z_mb(const KernelSet&, int grid, cudaStream_t st, const SweepArgs& a) {
-    if constexpr (CL::GROUPED) CR::launch_mb(grid, st, a);
+    if constexpr (CL::GROUPED) PL::c2r_mb(grid, st, a);
+  }
+  static void pair_tile(const KernelSet&, int mode, dim3 grid, cudaStream_t st, const TileArgs& a) {
+    if constexpr (PL::on) PL::template tile<false>(mode, grid, st, a);
+  }
+  static void pair_c2r(const KernelSet&, int grid, cudaStream_t st, const SweepArgs& a) {
+    if constexpr (PL::on) PL::c2r(grid, st, a);
   }
   static void tile(const KernelSet&, int mode, dim3 grid, cudaStream_t st, const TileArgs& a) {
     CL::launch(mode, grid, st, a);
@@ -266,9 +311,17 @@ template <int N> struct Launchers {
     ks.c2r_z = &c2r_z;
     ks.adj_z = &adj_z;
     ks.c2r_plain = &c2r_plain;
+    if constexpr (PL::on) {
+      ks.pair = 1;
+      ks.pair_xb = PairSlot<N>::XB;
+      ks.pair_tile_w = PL::KI::T;
+      ks.pair_tile_w_win = PL::KW::T;
+      ks.pair_lines = PL::KZ::NG;
+      ks.pair_tile = &pair_tile;
+      ks.pair_c2r = &pair_c2r;
+    }
     if constexpr (CL::GROUPED) {
       ks.grouped = 1;
-      ks.tile_w_mb_win = CL::W0::T;
       ks.r2c_z_mb = &r2c_z_mb;
       ks.tile_mb = &tile_mb;
       ks.c2r_z_mb = &c2r_z_mb;

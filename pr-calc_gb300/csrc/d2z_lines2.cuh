@@ -1,0 +1,281 @@
+// d2z_lines2.cuh — the inverse z pass on pairs of radii: k_c2r_zp's packing,
+// transform, barrier and running max (d2z_lines.cuh) for two radii per step
+// with the packed arithmetic of fft2.cuh, from the pair slots of d2z_cols2.cuh.
+//
+// A warp works alone on 32 / G lines: every lane copies the sixteen-byte
+// elements that it needs itself (its mirror pairs X[k], X[H-k]) with cp.async
+// into its own column of a staging area, the next step's as soon as this
+// step's are in registers, and the copies complete on the warp's mbarrier.
+// So no CTA barrier separates the steps, and the warps of an SM drift apart:
+// one transforms while others wait for copies.  The transform's exchange runs
+// in the warp's own buffer, padded by one element every PD positions so that
+// the first stage's stores (stride: the first radix) hit distinct banks.
+#pragma once
+#include "d2z_cols2.cuh"
+#include "d2z_lines.cuh"
+
+namespace prc {
+
+// PD: padding period, MINB: resident CTAs per SM
+template <int N> struct P2Cfg { static constexpr bool on = false; };
+template <> struct P2Cfg<32> { static constexpr bool on = true; static constexpr int PD = 8, MINB = 5; };
+template <> struct P2Cfg<64> { static constexpr bool on = true; static constexpr int PD = 8, MINB = 6; };
+template <> struct P2Cfg<96> { static constexpr bool on = true; static constexpr int PD = 24, MINB = 4; };
+template <> struct P2Cfg<128> { static constexpr bool on = true; static constexpr int PD = 8, MINB = 5; };
+template <> struct P2Cfg<192> { static constexpr bool on = true; static constexpr int PD = 24, MINB = 4; };
+template <> struct P2Cfg<256> { static constexpr bool on = true; static constexpr int PD = 16, MINB = 3; };
+template <> struct P2Cfg<384> { static constexpr bool on = true; static constexpr int PD = 24, MINB = 4; };
+template <> struct P2Cfg<512> { static constexpr bool on = true; static constexpr int PD = 16, MINB = 3; };
+template <> struct P2Cfg<768> { static constexpr bool on = true; static constexpr int PD = 24, MINB = 4; };
+template <> struct P2Cfg<1024> { static constexpr bool on = true; static constexpr int PD = 16, MINB = 3; };
+
+template <int N> struct PK2 {
+  using P = typename PCfg<N>::P;
+  static constexpr int H = N / 2, E = P::E, G = H / E, PD = P2Cfg<N>::PD, MINB = P2Cfg<N>::MINB;
+  static constexpr int THREADS = 128, NG = THREADS / G;  // lines per CTA step
+  static_assert(THREADS >= kMaxBatch && NG * G == THREADS, "per-radius sums need a thread per radius");
+  static_assert(PlanRun<P>::L == H && E % 2 == 0 && G >= 2 && G <= 32 && 32 % G == 0, "paired line shape");
+  static constexpr int TW = (PlanRun<P>::TW + 1) & ~1;
+  // 16-byte elements of one line's exchange buffer: padded, and G bank groups
+  // on from the next line's where several lines share a wavefront
+  static constexpr int pads = H + H / PD;
+  static constexpr int LS = G >= 8 ? pads : pads + ((G - pads % 8) % 8 + 8) % 8;
+  // quarter of the N-table, stage twiddles, exchange buffers, every lane's E staged elements,
+  // every line's X[H/2]
+  static constexpr int QT = N / 4 + 2;  // e^{2 pi i k/N}, k <= N/4 (even, for alignment)
+  static constexpr size_t bytes = (size_t)(QT + TW) * 8 + (size_t)(NG * LS + E * THREADS + NG) * 16;
+};
+
+// Offsets add except where reads of a 12-point plan (PD = 24) meet a lane's
+// position t: there each is formed by itself (Stages2x: get_pos).
+template <int PD> struct PairLine {
+  static constexpr bool READ_POS = PD == 24;
+  ulonglong2* b;
+  static __device__ __forceinline__ constexpr int off(int p) { return p + p / PD; }
+  __device__ __forceinline__ Cx2 get(int h, int cp) const {
+    const ulonglong2 q = b[h + off(cp)];
+    return {q.x, q.y};
+  }
+  __device__ __forceinline__ Cx2 get_pos(int p) const {
+    const ulonglong2 q = b[off(p)];
+    return {q.x, q.y};
+  }
+  __device__ __forceinline__ void put(int h, int cp, Cx2 v) const { b[h + off(cp)] = make_ulonglong2(v.re, v.im); }
+};
+
+// arrival of this thread at the barrier once all its cp.async so far are done
+__device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
+  const unsigned b = (unsigned)__cvta_generic_to_shared(bar);
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(b) : "memory");
+}
+
+// AM, SIG and MB as in k_c2r_zp.  Steps (line group, pair) of a warp run
+// pair-fastest.  A wait that runs out of polls sets *a.err and ends the warp's
+// work; its own copies are waited for (cp.async.wait_all) before it leaves.
+// a.withhold (a test hook) makes the first warp of CTA 0 skip its first copies
+// and their arrival, so that its first wait runs out with nothing in flight.
+template <int N, bool AM, bool SIG, bool MB = false>
+__global__ void __launch_bounds__(PK2<N>::THREADS, PK2<N>::MINB) k_c2r_zp2(const __grid_constant__ SweepArgs a) {
+  static_assert(!(MB && SIG), "no per-radius sums in grouped launches");
+  using KK = PK2<N>;
+  using P = typename KK::P;
+  using L = PairSlot<N>;
+  constexpr int H = N / 2, E = KK::E, G = KK::G, NG = KK::NG, EH = E / 2, LS = KK::LS, TH = KK::THREADS;
+  constexpr long long NN = (long long)N * N;
+  static_assert(NN % NG == 0 && (NG % L::XB == 0 || L::XB % NG == 0), "whole line groups");
+  extern __shared__ float4 smem4[];
+  float2* tw = reinterpret_cast<float2*>(smem4);
+  float2* tws = tw + KK::QT;
+  ulonglong2* xbuf = reinterpret_cast<ulonglong2*>(tws + KK::TW);
+  ulonglong2* stage = xbuf + NG * LS + threadIdx.x;  // element i of this lane at stage[i * TH]
+  ulonglong2* mid = xbuf + NG * LS + E * TH + threadIdx.x / G;
+  load_tw(tw, a.tw, N / 4 + 1);
+  PlanRun<P>::template fill<2>(tws, a.tw);
+  __shared__ double red[kMaxBatch];
+  __shared__ float s_cb[kMaxBatch];
+  if constexpr (!MB) stage_params_all(s_cb, a.cb);
+  if (threadIdx.x < kMaxBatch) red[threadIdx.x] = 0.0;
+  const int g = threadIdx.x / G, t = threadIdx.x % G;
+  const GroupSync<G> sync(g);
+  const int partner = (G - t) & (G - 1);
+  constexpr int lgpb = (int)(NN / NG);  // line groups of one box
+  const long long lg_all = MB ? (long long)lgpb * a.nbox : lgpb;
+  const int nsteps_l = (int)((lg_all - blockIdx.x + gridDim.x - 1) / gridDim.x);
+  auto box_of = [&](int lg) { return MB ? (int)(((long long)blockIdx.x + (long long)lg * gridDim.x) / lgpb) : 0; };
+  // this lane group's line of line group lg: the block's planes first, then iy
+  // (their pieces are neighbours in the slot); with SIG in file order, as in
+  // k_c2r_zp, so that a warp adds up the same lines
+  auto line_of = [&](int lg, int bx, int& ix, int& iy) {
+    const int s = (int)((long long)blockIdx.x + (long long)lg * gridDim.x - (long long)bx * lgpb) * NG + g;
+    const int xi = SIG ? 0 : s % L::XB, q = SIG ? s : s / L::XB;
+    iy = q % N;
+    ix = SIG ? q / N : (q / N) * L::XB + xi;
+  };
+
+  __shared__ __align__(8) uint64_t s_bar[TH / 32];
+  uint64_t* const bar = &s_bar[threadIdx.x >> 5];
+  if ((threadIdx.x & 31) == 0) {
+    mbar_init(bar, 32);
+    mbar_init_fence();
+  }
+  __syncthreads();
+
+  // copies of step (line group lg of this CTA, pair p): lane t's pairs (X[k],
+  // X[H-k]), k = t + G*m, m < E/2; lane 0 takes the Nyquist element for X[H]
+  // and X[H/2] besides
+  const bool withheld = a.withhold && blockIdx.x == 0 && threadIdx.x < 32;
+  auto issue = [&](int lg, int p) {
+    if (lg < nsteps_l && !(withheld && lg == 0 && p == 0)) {
+      const int bx = box_of(lg);
+      int ix, iy;
+      line_of(lg, bx, ix, iy);
+      const ulonglong2* slot =
+          reinterpret_cast<const ulonglong2*>(MB ? a.box[bx].slots : a.slots) + (long long)p * a.slot_stride;
+      const ulonglong2* nyq = slot + NN * H + (long long)iy * N + ix;
+      // position t + x, x a multiple of G, lies along(x) after position t
+      static_assert(G % L::T == 0 || L::T % G == 0, "a lane's positions split");
+      const ulonglong2* line = slot + L::at(ix, iy, 0);
+      const ulonglong2* lo = line + L::along(t);
+      const ulonglong2* hi = line + L::along(G - t);  // t > 0
+#pragma unroll
+      for (int m = 0; m < EH; ++m) {
+        cp_async16(stage + m * TH, lo + L::along(G * m));
+        cp_async16(stage + (EH + m) * TH,
+                   t ? hi + L::along(H - G * (m + 1)) : (m ? line + L::along(H - G * m) : nyq));
+      }
+      if (t == 0) cp_async16(mid, line + L::along(H / 2));
+      cp_async_arrive(bar);
+    }
+  };
+
+  issue(0, 0);
+  float2 zr[E];
+  uint32_t am[AM ? EH : 1];  // argmax bytes of cells 2p, 2p+1 of elements 2j (low half) and 2j+1
+  int lg = 0, p = 0;         // current step
+  for (int i = 0; lg < nsteps_l; ++i) {
+    const int bx = box_of(lg);
+    const BoxLine* bp = MB ? a.box + bx : nullptr;
+    const int np = ((MB ? bp->nb : a.nb) + 1) >> 1;
+    const int p_next = (p + 1 < np) ? p + 1 : 0;
+    const int lg_next = (p + 1 < np) ? lg : lg + 1;
+    if (p == 0) {
+      if (MB ? bp->first : a.first) {
+#pragma unroll
+        for (int m = 0; m < E; ++m) zr[m] = make_float2(0.f, 0.f);
+        if constexpr (AM) {
+#pragma unroll
+          for (int j = 0; j < EH; ++j) am[j] = 0xFFFFFFFFu;
+        }
+      } else {
+        int ix, iy;
+        line_of(lg, bx, ix, iy);
+        const long long l = (long long)ix * N + iy;
+        const float2* zline = reinterpret_cast<const float2*>((MB ? bp->zreion : a.zreion) + l * N);
+#pragma unroll
+        for (int m = 0; m < E; ++m) zr[m] = zline[t + G * m];
+        if constexpr (AM) {
+          const uint16_t* aline = reinterpret_cast<const uint16_t*>((MB ? bp->argmax : a.argmax) + l * N);
+#pragma unroll
+          for (int j = 0; j < EH; ++j)
+            am[j] = (uint32_t)aline[t + G * (2 * j)] | ((uint32_t)aline[t + G * (2 * j + 1)] << 16);
+        }
+      }
+    }
+    // step i is the barrier's i-th phase
+    const bool late = !mbar_wait(bar, (unsigned)(i & 1), (withheld && i == 0) ? kWithheldPolls : kWaitPolls);
+    if (__any_sync(0xffffffffu, late)) {
+      if ((threadIdx.x & 31) == 0 && a.err) *reinterpret_cast<volatile int*>(a.err) = 1;  // may be mapped host memory
+      break;
+    }
+    Cx2 v[E];
+#pragma unroll
+    for (int m = 0; m < EH; ++m) {
+      const ulonglong2 q = stage[m * TH], qp = stage[(EH + m) * TH];
+      Cx2 x = {q.x, q.y}, xp = {qp.x, qp.y};
+      if (m == 0 && t == 0) x.im = xp.im = 0;
+      const Cx2 xe = {add2(x.re, xp.re), sub2(x.im, xp.im)};
+      const Cx2 xo = ctwid<true>(Cx2{sub2(x.re, xp.re), add2(x.im, xp.im)}, tw[t + G * m]);
+      v[m] = {sub2(xe.re, xo.im), add2(xe.im, xo.re)};
+      // Z[H-k] to the lane that owns it (lane G-t, register E-1-m)
+      const float2 mr = unpack2(add2(xe.re, xo.im)), mi = unpack2(sub2(xo.re, xe.im));
+      v[E - 1 - m].re = pack2(__shfl_sync(0xffffffffu, mr.x, partner, G), __shfl_sync(0xffffffffu, mr.y, partner, G));
+      v[E - 1 - m].im = pack2(__shfl_sync(0xffffffffu, mi.x, partner, G), __shfl_sync(0xffffffffu, mi.y, partner, G));
+    }
+    if (t == 0) {
+      // lane 0 received its own mirrors Z[G*(E-m)] one register low
+#pragma unroll
+      for (int j = E - 1; j > EH; --j) v[j] = v[j - 1];
+      const ulonglong2 q = *mid;
+      const Cx2 x = {q.x, q.y};
+      const Cx2 xe = {add2(x.re, x.re), sub2(x.im, x.im)};
+      const Cx2 xo = ctwid<true>(Cx2{sub2(x.re, x.re), add2(x.im, x.im)}, tw[H / 2]);
+      v[EH] = {sub2(xe.re, xo.im), add2(xe.im, xo.re)};
+    }
+    // the staged elements are in registers (the shuffles have used them), and
+    // the previous exchange of this warp has been read
+    sync();
+    issue(lg_next, p_next);
+    const PairLine<KK::PD> buf{xbuf + g * LS};
+    PlanRun2x<P>::template run<true>(v, buf, t, tws, sync);
+    const f32x2 as = dup2(MB ? bp->as : a.as);
+    const f32x2 cb = MB ? pack2(__ldg(&bp->cb[2 * p]), __ldg(&bp->cb[2 * p + 1])) : pack2(s_cb[2 * p], s_cb[2 * p + 1]);
+    const uint32_t rid = (uint32_t)((MB ? bp->r0 : a.r0) + 2 * p);
+    f32x2 ss = 0;
+#pragma unroll
+    for (int m = 0; m < E; ++m) {
+      const float2 z0 = unpack2(fma2(as, v[m].re, cb)), z1 = unpack2(fma2(as, v[m].im, cb));
+      if constexpr (AM) {
+        const int sh = 16 * (m & 1);
+        auto win = [&](float z, float& best, uint32_t r, int s) {
+          if (z > best) {
+            best = z;
+            am[m >> 1] = (am[m >> 1] & ~(0xFFu << s)) | (r << s);
+          }
+        };
+        win(z0.x, zr[m].x, rid, sh);
+        win(z0.y, zr[m].x, rid + 1, sh);
+        win(z1.x, zr[m].y, rid, sh + 8);
+        win(z1.y, zr[m].y, rid + 1, sh + 8);
+      } else {
+        // fmaxf: as in k_c2r_zp
+        zr[m].x = fmaxf(fmaxf(zr[m].x, z0.x), z0.y);
+        zr[m].y = fmaxf(fmaxf(zr[m].y, z1.x), z1.y);
+      }
+      if constexpr (SIG) ss = fma2(v[m].re, v[m].re, fma2(v[m].im, v[m].im, ss));
+    }
+    if constexpr (SIG) {
+      float2 s = unpack2(ss);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+        s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+      }
+      if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&red[2 * p], (double)s.x);
+        atomicAdd(&red[2 * p + 1], (double)s.y);  // (the filler of an odd sweep: never read)
+      }
+    }
+    if (p == np - 1) {
+      int ix, iy;
+      line_of(lg, bx, ix, iy);
+      const long long l = (long long)ix * N + iy;
+      float2* zout = reinterpret_cast<float2*>((MB ? bp->zreion_out : a.zreion_out) + l * N);
+#pragma unroll
+      for (int m = 0; m < E; ++m) zout[t + G * m] = zr[m];
+      if constexpr (AM) {
+        uint16_t* aout = reinterpret_cast<uint16_t*>((MB ? bp->argmax_out : a.argmax_out) + l * N);
+#pragma unroll
+        for (int m = 0; m < E; ++m) aout[t + G * m] = (uint16_t)(am[m >> 1] >> (16 * (m & 1)));
+      }
+    }
+    lg = lg_next;
+    p = p_next;
+  }
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+  if constexpr (SIG) {
+    __syncthreads();
+    if (threadIdx.x < a.nb) atomicAdd(&a.sig_acc[a.r0 + threadIdx.x], red[threadIdx.x]);
+  }
+}
+
+}  // namespace prc
