@@ -826,7 +826,7 @@ void batch_enqueue_grouped(prc_d2z_batch* b, const float* const* delta, float* c
       sa.argmax = argmax ? argmax[g.sw_box[sw][0]] : nullptr;
       sa.box = reinterpret_cast<const BoxLine*>(b->d_tab + g.o_line[sw]);
       sa.nbox = ns;
-      ks.c2r_z_mb(ks, grid_for(N * N * ns, ks.pair_lines, ks.occ_mb_c2r * waves, sms), g.st, sa);
+      ks.c2r_z_mb(ks, grid_for(N * N * ns, ks.mb_lines, ks.occ_mb_c2r * waves, sms), g.st, sa);
       launches += 2;
     }
     launches += 1;

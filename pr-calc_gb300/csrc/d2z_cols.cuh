@@ -172,6 +172,7 @@ __global__ void __launch_bounds__(ColK<N, MODE, V>::type::THREADS, ColK<N, MODE,
   __shared__ float s_kr[kMaxBatch];
   if constexpr (MODE == TM_WIN || MODE == TM_ACC) stage_params(s_kr, a.kr);
   PlanRun<P>::template fill<1>(tws, a.tw);
+  pdl_wait();
   __syncthreads();
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, c = lane & (T - 1);
   int t;
@@ -239,7 +240,7 @@ __global__ void __launch_bounds__(ColK<N, MODE, V>::type::THREADS, ColK<N, MODE,
     const float2* p = base + (long long)t * rs + c;
     const long long step = (long long)G * rs;
 #pragma unroll
-    for (int m = 0; m < E; ++m) v[m] = __ldg(p + m * step);
+    for (int m = 0; m < E; ++m) v[m] = p[m * step];
   };
   auto gstore = [&](const Where& w, float2* dst, const float2 (&v)[E]) {
     if (w.sn ? a.seg[1].transpose : a.seg[0].transpose) {
@@ -420,6 +421,7 @@ __global__ void __launch_bounds__(ColK<N, MODE, V>::type::THREADS, ColK<N, MODE,
       }
     }
   }
+  pdl_release();
 }
 
 }  // namespace prc

@@ -160,6 +160,7 @@ __global__ void __launch_bounds__(CK2<N, MODE>::THREADS, CK2<N, MODE>::MINB) k_c
   __shared__ float s_kr[kMaxBatch];
   if constexpr (MODE == TM_WIN && !MB) stage_params_all(s_kr, a.kr);
   PlanRun<P>::template fill<1>(tws, a.tw);
+  pdl_wait();
   __syncthreads();
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, c = lane & (T - 1);
   using F = ColFft<N, P>;
@@ -332,7 +333,7 @@ __global__ void __launch_bounds__(CK2<N, MODE>::THREADS, CK2<N, MODE>::MINB) k_c
         Cx2 v[E];
 #pragma unroll
         for (int m = 0; m < E; ++m) {
-          const ulonglong2 q = __ldg(p + m * step);
+          const ulonglong2 q = p[m * step];
           v[m] = {q.x, q.y};
         }
         reuse();
@@ -429,6 +430,7 @@ __global__ void __launch_bounds__(CK2<N, MODE>::THREADS, CK2<N, MODE>::MINB) k_c
     }
     cp_async_wait<0>();
   }
+  pdl_release();
 }
 
 }  // namespace prc

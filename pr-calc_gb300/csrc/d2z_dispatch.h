@@ -45,6 +45,7 @@ struct KernelSet {
   // for this size (grouped = 1): forward z pass, forward column passes, and
   // the sweep's passes on pairs of radii (TM_WIN, TM_INV, inverse z)
   int grouped;
+  int mb_lines;  // lines per CTA step of the inverse z pass
   int occ_mb_tile, occ_mb_inv, occ_mb_win, occ_mb_c2r, occ_mb_r2c;
   void (*r2c_z_mb)(const KernelSet&, int grid, cudaStream_t, const BoxR2c* box, int nbox, const float2* tw);
   void (*tile_mb)(const KernelSet&, int mode, dim3 grid, cudaStream_t, const TileArgs&);

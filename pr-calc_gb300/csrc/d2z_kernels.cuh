@@ -182,6 +182,20 @@ struct SweepArgs {
 enum TileMode { TM_FWD = 0, TM_INV = 1, TM_WIN = 2, TM_ACC = 3 };
 
 // ------------------------------------------------------------ helpers
+// Programmatic dependent launch: the passes of a step are launched with the
+// attribute that lets a kernel's CTAs start while the previous kernel of the
+// stream drains.  A CTA that has done its work allows the successor to start
+// (pdl_release; at the beginning of the CTA instead, the successor's CTAs sat
+// in the slots that this kernel's own still needed: 128^3 x 32 279 against 247
+// us).  The successor fills its tables; before it touches anything that another kernel writes
+// or reads it waits until the previous kernel has finished (pdl_wait; at once
+// when launched without the attribute).  Every kernel of the chain waits, so
+// all earlier ones have finished too.  Data of the previous kernel is read with
+// ordinary loads, not through the read-only path: it may still be written
+// while this kernel has begun.
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ int fsq(int f, int n) {
   const int a = (f <= (n >> 1)) ? f : n - f;
   return a * a;
@@ -723,7 +737,7 @@ __device__ __forceinline__ void line_c2r(float2 (&v)[LK<N>::E], float2 xh, float
 // MB (grouped launch): the lines of nbox boxes of this grid size, line l of
 // box l / N^2 with box i's input, spectrum and divisor from box[i].
 template <int N, bool MB = false>
-__global__ void __launch_bounds__(LK<N>::THREADS, LK<N>::MINB) k_r2c_z(const float* __restrict__ delta, float dinit,
+__global__ void __launch_bounds__(LK<N>::THREADS, LK<N>::MINB) k_r2c_z(const float* delta, float dinit,
                                                              float2* S, float2* Qt, const float2* twg,
                                                              const BoxR2c* box, int nbox) {
   using KK = LK<N>;
@@ -733,6 +747,7 @@ __global__ void __launch_bounds__(LK<N>::THREADS, LK<N>::MINB) k_r2c_z(const flo
   float2* tws = tw + N;
   load_tw(tw, twg, N);
   PlanRun<typename KK::P>::template fill<2>(tws, twg);
+  pdl_wait();
   __syncthreads();
   const int g = threadIdx.x / G, t = threadIdx.x % G;
   float2* gbuf = tws + KK::TW + g * KK::gsize;
@@ -759,7 +774,7 @@ __global__ void __launch_bounds__(LK<N>::THREADS, LK<N>::MINB) k_r2c_z(const flo
     const float2* src = reinterpret_cast<const float2*>(dsrc + (long long)(valid ? l : 0) * N);
 #pragma unroll
     for (int m = 0; m < E; ++m) {
-      float2 q = valid ? __ldg(src + t + G * m) : make_float2(0.f, 0.f);
+      float2 q = valid ? src[t + G * m] : make_float2(0.f, 0.f);
       v[m] = make_float2(__fdiv_rn(q.x, dv), __fdiv_rn(q.y, dv));
     }
     const float xh = line_r2c<N>(v, gbuf, t, tw, tws, sync);
@@ -773,6 +788,7 @@ __global__ void __launch_bounds__(LK<N>::THREADS, LK<N>::MINB) k_r2c_z(const flo
       }
     }
   }
+  pdl_release();
 }
 
 // ============================================================ inverse z pass

@@ -11,6 +11,23 @@ namespace prc {
 
 static_assert(kWinVariants == kMaxWinVariants, "window variant table size");
 
+// Launch with the programmatic-dependent-launch attribute; only for kernels
+// that call pdl_wait before they touch the previous kernel's data.
+template <class... P, class... A>
+void launch_pdl(void (*f)(P...), dim3 grid, int threads, size_t bytes, cudaStream_t st, const A&... args) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid;
+  c.blockDim = dim3((unsigned)threads);
+  c.dynamicSmemBytes = bytes;
+  c.stream = st;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  cudaLaunchKernelEx(&c, f, static_cast<P>(args)...);
+}
+
 // Column passes: k_col (one lane per column) where CCfg<N> has a plan, else
 // k_tile (shared-memory staged tiles).
 template <int N, bool COL = CCfg<N>::on> struct ColLaunch;
@@ -106,7 +123,7 @@ template <int N> struct ColLaunch<N, true> {
   }
   static void launch(int mode, dim3 grid, cudaStream_t st, const TileArgs& a) {
     switch (mode) {
-      case TM_FWD: k_col<N, TM_FWD><<<grid, THREADS, CS, st>>>(a); break;
+      case TM_FWD: launch_pdl(&k_col<N, TM_FWD>, grid, THREADS, CS, st, a); break;
       case TM_INV: k_col<N, TM_INV><<<grid, THREADS, CS, st>>>(a); break;
       case TM_WIN: launch_win<0>(a.win_var, grid, st, a); break;
       default: k_col<N, TM_ACC><<<grid, CA::THREADS, CSA, st>>>(a); break;
@@ -116,7 +133,7 @@ template <int N> struct ColLaunch<N, true> {
   static constexpr bool GROUPED = N <= 256 && PCfg<N>::on;
   static void* fn_mb() { return reinterpret_cast<void*>(&k_col<N, TM_FWD, 0, true>); }
   static void launch_mb(dim3 grid, cudaStream_t st, const TileArgs& a) {
-    if constexpr (GROUPED) k_col<N, TM_FWD, 0, true><<<grid, THREADS, CS, st>>>(a);
+    if constexpr (GROUPED) launch_pdl(&k_col<N, TM_FWD, 0, true>, grid, THREADS, CS, st, a);
   }
 };
 
@@ -156,26 +173,27 @@ template <int N> struct PairLaunch<N, true> {
   using KW = CK2<N, TM_WIN>;
   using KI = CK2<N, TM_INV>;
   using KZ = PK2<N>;
+  using KZM = PK2<N, true>;
   template <bool MB> static void* win_fn() { return reinterpret_cast<void*>(&k_col2<N, TM_WIN, MB>); }
   template <bool MB> static void* inv_fn() { return reinterpret_cast<void*>(&k_col2<N, TM_INV, MB>); }
   template <bool AM, bool SIG, bool MB> static void* z_fn() { return reinterpret_cast<void*>(&k_c2r_zp2<N, AM, SIG, MB>); }
   template <bool MB> static void tile(int mode, dim3 grid, cudaStream_t st, const TileArgs& a) {
-    if (mode == TM_WIN) k_col2<N, TM_WIN, MB><<<grid, KW::THREADS, KW::bytes, st>>>(a);
-    else k_col2<N, TM_INV, MB><<<grid, KI::THREADS, KI::bytes, st>>>(a);
+    if (mode == TM_WIN) launch_pdl(&k_col2<N, TM_WIN, MB>, grid, KW::THREADS, KW::bytes, st, a);
+    else launch_pdl(&k_col2<N, TM_INV, MB>, grid, KI::THREADS, KI::bytes, st, a);
   }
   static void c2r(int grid, cudaStream_t st, const SweepArgs& a) {
     if (a.sig_acc) {
-      if (a.argmax) k_c2r_zp2<N, true, true><<<grid, KZ::THREADS, KZ::bytes, st>>>(a);
-      else k_c2r_zp2<N, false, true><<<grid, KZ::THREADS, KZ::bytes, st>>>(a);
+      if (a.argmax) launch_pdl(&k_c2r_zp2<N, true, true>, grid, KZ::THREADS, KZ::bytes, st, a);
+      else launch_pdl(&k_c2r_zp2<N, false, true>, grid, KZ::THREADS, KZ::bytes, st, a);
     } else {
-      if (a.argmax) k_c2r_zp2<N, true, false><<<grid, KZ::THREADS, KZ::bytes, st>>>(a);
-      else k_c2r_zp2<N, false, false><<<grid, KZ::THREADS, KZ::bytes, st>>>(a);
+      if (a.argmax) launch_pdl(&k_c2r_zp2<N, true, false>, grid, KZ::THREADS, KZ::bytes, st, a);
+      else launch_pdl(&k_c2r_zp2<N, false, false>, grid, KZ::THREADS, KZ::bytes, st, a);
     }
   }
   // grouped: a.argmax != null means every box of the launch records its argmax
   static void c2r_mb(int grid, cudaStream_t st, const SweepArgs& a) {
-    if (a.argmax) k_c2r_zp2<N, true, false, true><<<grid, KZ::THREADS, KZ::bytes, st>>>(a);
-    else k_c2r_zp2<N, false, false, true><<<grid, KZ::THREADS, KZ::bytes, st>>>(a);
+    if (a.argmax) launch_pdl(&k_c2r_zp2<N, true, false, true>, grid, KZM::THREADS, KZM::bytes, st, a);
+    else launch_pdl(&k_c2r_zp2<N, false, false, true>, grid, KZM::THREADS, KZM::bytes, st, a);
   }
 };
 
@@ -237,13 +255,13 @@ template <int N> struct Launchers {
       if ((e = smem(fm, CL::CS)) != cudaSuccess) return e;
       if ((e = smem(im, PL::KI::bytes)) != cudaSuccess) return e;
       if ((e = smem(wm, PL::KW::bytes)) != cudaSuccess) return e;
-      if ((e = smem(z0, PL::KZ::bytes)) != cudaSuccess) return e;
-      if ((e = smem(z1, PL::KZ::bytes)) != cudaSuccess) return e;
+      if ((e = smem(z0, PL::KZM::bytes)) != cudaSuccess) return e;
+      if ((e = smem(z1, PL::KZM::bytes)) != cudaSuccess) return e;
       if ((e = smem(&k_r2c_z<N, true>, LS)) != cudaSuccess) return e;
       if ((e = occ(&ks->occ_mb_tile, fm, CL::THREADS, CL::CS)) != cudaSuccess) return e;
       if ((e = occ(&ks->occ_mb_inv, im, PL::KI::THREADS, PL::KI::bytes)) != cudaSuccess) return e;
       if ((e = occ(&ks->occ_mb_win, wm, PL::KW::THREADS, PL::KW::bytes)) != cudaSuccess) return e;
-      if ((e = occ(&ks->occ_mb_c2r, z1, PL::KZ::THREADS, PL::KZ::bytes)) != cudaSuccess) return e;
+      if ((e = occ(&ks->occ_mb_c2r, z1, PL::KZM::THREADS, PL::KZM::bytes)) != cudaSuccess) return e;
       if ((e = occ(&ks->occ_mb_r2c, &k_r2c_z<N, true>, LL::THREADS, LS)) != cudaSuccess) return e;
     }
     if ((e = smem(CL::faithful_fn(), CL::FS)) != cudaSuccess) return e;
@@ -263,10 +281,11 @@ template <int N> struct Launchers {
   }
   static void r2c_z(const KernelSet&, int grid, cudaStream_t st, const float* d, float dinit, float2* S,
                     float2* Qt, const float2* tw) {
-    k_r2c_z<N><<<grid, LL::THREADS, LS, st>>>(d, dinit, S, Qt, tw, nullptr, 0);
+    launch_pdl(&k_r2c_z<N>, grid, LL::THREADS, LS, st, d, dinit, S, Qt, tw, (const BoxR2c*)nullptr, 0);
   }
   static void r2c_z_mb(const KernelSet&, int grid, cudaStream_t st, const BoxR2c* box, int nbox, const float2* tw) {
-    if constexpr (CL::GROUPED) k_r2c_z<N, true><<<grid, LL::THREADS, LS, st>>>(nullptr, 1.f, nullptr, nullptr, tw, box, nbox);
+    if constexpr (CL::GROUPED) launch_pdl(&k_r2c_z<N, true>, grid, LL::THREADS, LS, st, (const float*)nullptr, 1.f, (float2*)nullptr, (float2*)nullptr,
+                                               tw, box, nbox);
   }
   static void tile_mb(const KernelSet&, int mode, dim3 grid, cudaStream_t st, const TileArgs& a) {
     if constexpr (CL::GROUPED) {
@@ -322,6 +341,7 @@ template <int N> struct Launchers {
     }
     if constexpr (CL::GROUPED) {
       ks.grouped = 1;
+      ks.mb_lines = PL::KZM::NG;
       ks.r2c_z_mb = &r2c_z_mb;
       ks.tile_mb = &tile_mb;
       ks.c2r_z_mb = &c2r_z_mb;

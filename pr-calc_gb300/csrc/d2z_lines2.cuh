@@ -16,24 +16,27 @@
 
 namespace prc {
 
-// PD: padding period, MINB: resident CTAs per SM
+// PD: padding period, MINB: resident CTAs per SM, SP: warps that share a set of
+// lines and split the pairs of a sweep
 template <int N> struct P2Cfg { static constexpr bool on = false; };
-template <> struct P2Cfg<32> { static constexpr bool on = true; static constexpr int PD = 8, MINB = 5; };
-template <> struct P2Cfg<64> { static constexpr bool on = true; static constexpr int PD = 8, MINB = 6; };
-template <> struct P2Cfg<96> { static constexpr bool on = true; static constexpr int PD = 24, MINB = 4; };
-template <> struct P2Cfg<128> { static constexpr bool on = true; static constexpr int PD = 8, MINB = 5; };
-template <> struct P2Cfg<192> { static constexpr bool on = true; static constexpr int PD = 24, MINB = 4; };
-template <> struct P2Cfg<256> { static constexpr bool on = true; static constexpr int PD = 16, MINB = 3; };
-template <> struct P2Cfg<384> { static constexpr bool on = true; static constexpr int PD = 24, MINB = 4; };
-template <> struct P2Cfg<512> { static constexpr bool on = true; static constexpr int PD = 16, MINB = 3; };
-template <> struct P2Cfg<768> { static constexpr bool on = true; static constexpr int PD = 24, MINB = 4; };
-template <> struct P2Cfg<1024> { static constexpr bool on = true; static constexpr int PD = 16, MINB = 3; };
+template <> struct P2Cfg<32> { static constexpr bool on = true; static constexpr int PD = 8, MINB = 5, SP = 4; };
+template <> struct P2Cfg<64> { static constexpr bool on = true; static constexpr int PD = 8, MINB = 5, SP = 4; };
+template <> struct P2Cfg<96> { static constexpr bool on = true; static constexpr int PD = 24, MINB = 4, SP = 4; };
+template <> struct P2Cfg<128> { static constexpr bool on = true; static constexpr int PD = 8, MINB = 5, SP = 4; };
+template <> struct P2Cfg<192> { static constexpr bool on = true; static constexpr int PD = 24, MINB = 4, SP = 1; };
+template <> struct P2Cfg<256> { static constexpr bool on = true; static constexpr int PD = 16, MINB = 3, SP = 1; };
+template <> struct P2Cfg<384> { static constexpr bool on = true; static constexpr int PD = 24, MINB = 4, SP = 1; };
+template <> struct P2Cfg<512> { static constexpr bool on = true; static constexpr int PD = 16, MINB = 3, SP = 1; };
+template <> struct P2Cfg<768> { static constexpr bool on = true; static constexpr int PD = 24, MINB = 4, SP = 1; };
+template <> struct P2Cfg<1024> { static constexpr bool on = true; static constexpr int PD = 16, MINB = 3, SP = 1; };
 
-template <int N> struct PK2 {
+template <int N, bool MB = false> struct PK2 {
   using P = typename PCfg<N>::P;
   static constexpr int H = N / 2, E = P::E, G = H / E, PD = P2Cfg<N>::PD, MINB = P2Cfg<N>::MINB;
-  static constexpr int THREADS = 128, NG = THREADS / G;  // lines per CTA step
-  static_assert(THREADS >= kMaxBatch && NG * G == THREADS, "per-radius sums need a thread per radius");
+  static constexpr int SP = MB ? 1 : P2Cfg<N>::SP;  // (many boxes have lines enough)
+  static constexpr int THREADS = 128, NL = THREADS / G, NG = NL / SP;  // line buffers, lines per CTA step
+  static_assert(THREADS >= kMaxBatch && NG * SP * G == THREADS, "per-radius sums need a thread per radius");
+  static_assert(SP == 1 || (SP == THREADS / 32 && E % SP == 0), "all warps of a CTA or one share lines");
   static_assert(PlanRun<P>::L == H && E % 2 == 0 && G >= 2 && G <= 32 && 32 % G == 0, "paired line shape");
   static constexpr int TW = (PlanRun<P>::TW + 1) & ~1;
   // 16-byte elements of one line's exchange buffer: padded, and G bank groups
@@ -43,7 +46,7 @@ template <int N> struct PK2 {
   // quarter of the N-table, stage twiddles, exchange buffers, every lane's E staged elements,
   // every line's X[H/2]
   static constexpr int QT = N / 4 + 2;  // e^{2 pi i k/N}, k <= N/4 (even, for alignment)
-  static constexpr size_t bytes = (size_t)(QT + TW) * 8 + (size_t)(NG * LS + E * THREADS + NG) * 16;
+  static constexpr size_t bytes = (size_t)(QT + TW) * 8 + (size_t)(NL * LS + E * THREADS + NL) * 16;
 };
 
 // Offsets add except where reads of a 12-point plan (PD = 24) meet a lane's
@@ -69,34 +72,42 @@ __device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(b) : "memory");
 }
 
-// AM, SIG and MB as in k_c2r_zp.  Steps (line group, pair) of a warp run
-// pair-fastest.  A wait that runs out of polls sets *a.err and ends the warp's
-// work; its own copies are waited for (cp.async.wait_all) before it leaves.
+// AM and SIG as in k_c2r_zp, MB as in k_col2.  A warp takes its line groups in
+// turn and of each the pairs sub, sub + SP, ...  With SP > 1 the CTA's warps
+// share the lines of a group: small grids have too few lines to give every
+// scheduler warps, and the warps' running maxima are merged at the end (the
+// larger value wins, of equal ones the smaller radius, as in the serial
+// order).  A wait that runs out of polls sets *a.err and ends the warp's work
+// (it still takes part in the merges); its own copies are waited for
+// (cp.async.wait_all) before it leaves.
 // a.withhold (a test hook) makes the first warp of CTA 0 skip its first copies
 // and their arrival, so that its first wait runs out with nothing in flight.
 template <int N, bool AM, bool SIG, bool MB = false>
-__global__ void __launch_bounds__(PK2<N>::THREADS, PK2<N>::MINB) k_c2r_zp2(const __grid_constant__ SweepArgs a) {
+__global__ void __launch_bounds__(PK2<N, MB>::THREADS, PK2<N, MB>::MINB) k_c2r_zp2(const __grid_constant__ SweepArgs a) {
   static_assert(!(MB && SIG), "no per-radius sums in grouped launches");
-  using KK = PK2<N>;
+  using KK = PK2<N, MB>;
   using P = typename KK::P;
   using L = PairSlot<N>;
   constexpr int H = N / 2, E = KK::E, G = KK::G, NG = KK::NG, EH = E / 2, LS = KK::LS, TH = KK::THREADS;
+  constexpr int SP = KK::SP;
   constexpr long long NN = (long long)N * N;
   static_assert(NN % NG == 0 && (NG % L::XB == 0 || L::XB % NG == 0), "whole line groups");
   extern __shared__ float4 smem4[];
   float2* tw = reinterpret_cast<float2*>(smem4);
   float2* tws = tw + KK::QT;
   ulonglong2* xbuf = reinterpret_cast<ulonglong2*>(tws + KK::TW);
-  ulonglong2* stage = xbuf + NG * LS + threadIdx.x;  // element i of this lane at stage[i * TH]
-  ulonglong2* mid = xbuf + NG * LS + E * TH + threadIdx.x / G;
+  ulonglong2* stage = xbuf + KK::NL * LS + threadIdx.x;  // element i of this lane at stage[i * TH]
+  ulonglong2* mid = xbuf + KK::NL * LS + E * TH + threadIdx.x / G;
   load_tw(tw, a.tw, N / 4 + 1);
   PlanRun<P>::template fill<2>(tws, a.tw);
   __shared__ double red[kMaxBatch];
   __shared__ float s_cb[kMaxBatch];
   if constexpr (!MB) stage_params_all(s_cb, a.cb);
   if (threadIdx.x < kMaxBatch) red[threadIdx.x] = 0.0;
-  const int g = threadIdx.x / G, t = threadIdx.x % G;
-  const GroupSync<G> sync(g);
+  const int lb = threadIdx.x / G, t = threadIdx.x % G;  // line buffer, FFT lane
+  const int sub = SP == 1 ? 0 : threadIdx.x >> 5;       // first pair
+  const int g = SP == 1 ? lb : lb % NG;                 // line of the group
+  const GroupSync<G> sync(lb);
   const int partner = (G - t) & (G - 1);
   constexpr int lgpb = (int)(NN / NG);  // line groups of one box
   const long long lg_all = MB ? (long long)lgpb * a.nbox : lgpb;
@@ -118,6 +129,7 @@ __global__ void __launch_bounds__(PK2<N>::THREADS, PK2<N>::MINB) k_c2r_zp2(const
     mbar_init(bar, 32);
     mbar_init_fence();
   }
+  pdl_wait();
   __syncthreads();
 
   // copies of step (line group lg of this CTA, pair p): lane t's pairs (X[k],
@@ -125,7 +137,7 @@ __global__ void __launch_bounds__(PK2<N>::THREADS, PK2<N>::MINB) k_c2r_zp2(const
   // and X[H/2] besides
   const bool withheld = a.withhold && blockIdx.x == 0 && threadIdx.x < 32;
   auto issue = [&](int lg, int p) {
-    if (lg < nsteps_l && !(withheld && lg == 0 && p == 0)) {
+    if (lg < nsteps_l && !(withheld && lg == 0 && p == sub)) {
       const int bx = box_of(lg);
       int ix, iy;
       line_of(lg, bx, ix, iy);
@@ -148,129 +160,183 @@ __global__ void __launch_bounds__(PK2<N>::THREADS, PK2<N>::MINB) k_c2r_zp2(const
     }
   };
 
-  issue(0, 0);
-  float2 zr[E];
-  uint32_t am[AM ? EH : 1];  // argmax bytes of cells 2p, 2p+1 of elements 2j (low half) and 2j+1
-  int lg = 0, p = 0;         // current step
-  for (int i = 0; lg < nsteps_l; ++i) {
+  auto pairs_of = [&](int lg) { return ((MB ? a.box[box_of(lg)].nb : a.nb) + 1) >> 1; };
+  int lg_next = 0, p_next = sub, np_next = pairs_of(0), i = 0;
+  // moves (lg_next, p_next) on to a step that there is
+  auto seek = [&]() {
+    while (p_next >= np_next && ++lg_next < nsteps_l) {
+      p_next = sub;
+      np_next = pairs_of(lg_next);
+    }
+  };
+  if constexpr (SP > 1) seek();
+  issue(lg_next, p_next);
+  bool dead = false;  // a wait ran out
+  for (int lg = 0; lg < nsteps_l && (SP > 1 || !dead); ++lg) {
     const int bx = box_of(lg);
     const BoxLine* bp = MB ? a.box + bx : nullptr;
-    const int np = ((MB ? bp->nb : a.nb) + 1) >> 1;
-    const int p_next = (p + 1 < np) ? p + 1 : 0;
-    const int lg_next = (p + 1 < np) ? lg : lg + 1;
-    if (p == 0) {
-      if (MB ? bp->first : a.first) {
-#pragma unroll
-        for (int m = 0; m < E; ++m) zr[m] = make_float2(0.f, 0.f);
-        if constexpr (AM) {
-#pragma unroll
-          for (int j = 0; j < EH; ++j) am[j] = 0xFFFFFFFFu;
-        }
-      } else {
-        int ix, iy;
-        line_of(lg, bx, ix, iy);
-        const long long l = (long long)ix * N + iy;
-        const float2* zline = reinterpret_cast<const float2*>((MB ? bp->zreion : a.zreion) + l * N);
-#pragma unroll
-        for (int m = 0; m < E; ++m) zr[m] = zline[t + G * m];
-        if constexpr (AM) {
-          const uint16_t* aline = reinterpret_cast<const uint16_t*>((MB ? bp->argmax : a.argmax) + l * N);
-#pragma unroll
-          for (int j = 0; j < EH; ++j)
-            am[j] = (uint32_t)aline[t + G * (2 * j)] | ((uint32_t)aline[t + G * (2 * j + 1)] << 16);
-        }
-      }
-    }
-    // step i is the barrier's i-th phase
-    const bool late = !mbar_wait(bar, (unsigned)(i & 1), (withheld && i == 0) ? kWithheldPolls : kWaitPolls);
-    if (__any_sync(0xffffffffu, late)) {
-      if ((threadIdx.x & 31) == 0 && a.err) *reinterpret_cast<volatile int*>(a.err) = 1;  // may be mapped host memory
-      break;
-    }
-    Cx2 v[E];
-#pragma unroll
-    for (int m = 0; m < EH; ++m) {
-      const ulonglong2 q = stage[m * TH], qp = stage[(EH + m) * TH];
-      Cx2 x = {q.x, q.y}, xp = {qp.x, qp.y};
-      if (m == 0 && t == 0) x.im = xp.im = 0;
-      const Cx2 xe = {add2(x.re, xp.re), sub2(x.im, xp.im)};
-      const Cx2 xo = ctwid<true>(Cx2{sub2(x.re, xp.re), add2(x.im, xp.im)}, tw[t + G * m]);
-      v[m] = {sub2(xe.re, xo.im), add2(xe.im, xo.re)};
-      // Z[H-k] to the lane that owns it (lane G-t, register E-1-m)
-      const float2 mr = unpack2(add2(xe.re, xo.im)), mi = unpack2(sub2(xo.re, xe.im));
-      v[E - 1 - m].re = pack2(__shfl_sync(0xffffffffu, mr.x, partner, G), __shfl_sync(0xffffffffu, mr.y, partner, G));
-      v[E - 1 - m].im = pack2(__shfl_sync(0xffffffffu, mi.x, partner, G), __shfl_sync(0xffffffffu, mi.y, partner, G));
-    }
-    if (t == 0) {
-      // lane 0 received its own mirrors Z[G*(E-m)] one register low
-#pragma unroll
-      for (int j = E - 1; j > EH; --j) v[j] = v[j - 1];
-      const ulonglong2 q = *mid;
-      const Cx2 x = {q.x, q.y};
-      const Cx2 xe = {add2(x.re, x.re), sub2(x.im, x.im)};
-      const Cx2 xo = ctwid<true>(Cx2{sub2(x.re, x.re), add2(x.im, x.im)}, tw[H / 2]);
-      v[EH] = {sub2(xe.re, xo.im), add2(xe.im, xo.re)};
-    }
-    // the staged elements are in registers (the shuffles have used them), and
-    // the previous exchange of this warp has been read
-    sync();
-    issue(lg_next, p_next);
-    const PairLine<KK::PD> buf{xbuf + g * LS};
-    PlanRun2x<P>::template run<true>(v, buf, t, tws, sync);
-    const f32x2 as = dup2(MB ? bp->as : a.as);
-    const f32x2 cb = MB ? pack2(__ldg(&bp->cb[2 * p]), __ldg(&bp->cb[2 * p + 1])) : pack2(s_cb[2 * p], s_cb[2 * p + 1]);
-    const uint32_t rid = (uint32_t)((MB ? bp->r0 : a.r0) + 2 * p);
-    f32x2 ss = 0;
-#pragma unroll
-    for (int m = 0; m < E; ++m) {
-      const float2 z0 = unpack2(fma2(as, v[m].re, cb)), z1 = unpack2(fma2(as, v[m].im, cb));
-      if constexpr (AM) {
-        const int sh = 16 * (m & 1);
-        auto win = [&](float z, float& best, uint32_t r, int s) {
-          if (z > best) {
-            best = z;
-            am[m >> 1] = (am[m >> 1] & ~(0xFFu << s)) | (r << s);
-          }
-        };
-        win(z0.x, zr[m].x, rid, sh);
-        win(z0.y, zr[m].x, rid + 1, sh);
-        win(z1.x, zr[m].y, rid, sh + 8);
-        win(z1.y, zr[m].y, rid + 1, sh + 8);
-      } else {
-        // fmaxf: as in k_c2r_zp
-        zr[m].x = fmaxf(fmaxf(zr[m].x, z0.x), z0.y);
-        zr[m].y = fmaxf(fmaxf(zr[m].y, z1.x), z1.y);
-      }
-      if constexpr (SIG) ss = fma2(v[m].re, v[m].re, fma2(v[m].im, v[m].im, ss));
-    }
-    if constexpr (SIG) {
-      float2 s = unpack2(ss);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
-        s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
-      }
-      if ((threadIdx.x & 31) == 0) {
-        atomicAdd(&red[2 * p], (double)s.x);
-        atomicAdd(&red[2 * p + 1], (double)s.y);  // (the filler of an odd sweep: never read)
-      }
-    }
-    if (p == np - 1) {
+    const int np = pairs_of(lg);
+    auto line = [&]() {  // this lane group's line in file order
       int ix, iy;
       line_of(lg, bx, ix, iy);
-      const long long l = (long long)ix * N + iy;
-      float2* zout = reinterpret_cast<float2*>((MB ? bp->zreion_out : a.zreion_out) + l * N);
+      return (long long)ix * N + iy;
+    };
+    float2 zr[E];
+    uint32_t am[AM ? EH : 1];  // argmax bytes of cells 2p, 2p+1 of elements 2j (low half) and 2j+1
+    if (MB ? bp->first : a.first) {
 #pragma unroll
-      for (int m = 0; m < E; ++m) zout[t + G * m] = zr[m];
+      for (int m = 0; m < E; ++m) zr[m] = make_float2(0.f, 0.f);
       if constexpr (AM) {
-        uint16_t* aout = reinterpret_cast<uint16_t*>((MB ? bp->argmax_out : a.argmax_out) + l * N);
 #pragma unroll
-        for (int m = 0; m < E; ++m) aout[t + G * m] = (uint16_t)(am[m >> 1] >> (16 * (m & 1)));
+        for (int j = 0; j < EH; ++j) am[j] = 0xFFFFFFFFu;
+      }
+    } else {
+      const long long l = line();
+      const float2* zline = reinterpret_cast<const float2*>((MB ? bp->zreion : a.zreion) + l * N);
+#pragma unroll
+      for (int m = 0; m < E; ++m) zr[m] = zline[t + G * m];
+      if constexpr (AM) {
+        const uint16_t* aline = reinterpret_cast<const uint16_t*>((MB ? bp->argmax : a.argmax) + l * N);
+#pragma unroll
+        for (int j = 0; j < EH; ++j)
+          am[j] = (uint32_t)aline[t + G * (2 * j)] | ((uint32_t)aline[t + G * (2 * j + 1)] << 16);
       }
     }
-    lg = lg_next;
-    p = p_next;
+    for (int p = sub; p < np && (SP == 1 || !dead); p += SP, ++i) {
+      // step i is the barrier's i-th phase
+      const bool late = !mbar_wait(bar, (unsigned)(i & 1), (withheld && i == 0) ? kWithheldPolls : kWaitPolls);
+      if (__any_sync(0xffffffffu, late)) {
+        if ((threadIdx.x & 31) == 0 && a.err) *reinterpret_cast<volatile int*>(a.err) = 1;  // may be mapped host memory
+        dead = true;
+        break;
+      }
+      Cx2 v[E];
+#pragma unroll
+      for (int m = 0; m < EH; ++m) {
+        const ulonglong2 q = stage[m * TH], qp = stage[(EH + m) * TH];
+        Cx2 x = {q.x, q.y}, xp = {qp.x, qp.y};
+        if (m == 0 && t == 0) x.im = xp.im = 0;
+        const Cx2 xe = {add2(x.re, xp.re), sub2(x.im, xp.im)};
+        const Cx2 xo = ctwid<true>(Cx2{sub2(x.re, xp.re), add2(x.im, xp.im)}, tw[t + G * m]);
+        v[m] = {sub2(xe.re, xo.im), add2(xe.im, xo.re)};
+        // Z[H-k] to the lane that owns it (lane G-t, register E-1-m)
+        const float2 mr = unpack2(add2(xe.re, xo.im)), mi = unpack2(sub2(xo.re, xe.im));
+        v[E - 1 - m].re = pack2(__shfl_sync(0xffffffffu, mr.x, partner, G), __shfl_sync(0xffffffffu, mr.y, partner, G));
+        v[E - 1 - m].im = pack2(__shfl_sync(0xffffffffu, mi.x, partner, G), __shfl_sync(0xffffffffu, mi.y, partner, G));
+      }
+      if (t == 0) {
+        // lane 0 received its own mirrors Z[G*(E-m)] one register low
+#pragma unroll
+        for (int j = E - 1; j > EH; --j) v[j] = v[j - 1];
+        const ulonglong2 q = *mid;
+        const Cx2 x = {q.x, q.y};
+        const Cx2 xe = {add2(x.re, x.re), sub2(x.im, x.im)};
+        const Cx2 xo = ctwid<true>(Cx2{sub2(x.re, x.re), add2(x.im, x.im)}, tw[H / 2]);
+        v[EH] = {sub2(xe.re, xo.im), add2(xe.im, xo.re)};
+      }
+      // the staged elements are in registers (the shuffles have used them), and
+      // the previous exchange of this warp has been read
+      sync();
+      if constexpr (SP == 1) {  // every line group has a pair
+        p_next = p + 1 < np ? p + 1 : 0;
+        lg_next = p + 1 < np ? lg : lg + 1;
+      } else {
+        p_next += SP;
+        seek();
+      }
+      issue(lg_next, p_next);
+      const PairLine<KK::PD> buf{xbuf + lb * LS};
+      PlanRun2x<P>::template run<true>(v, buf, t, tws, sync);
+      const f32x2 as = dup2(MB ? bp->as : a.as);
+      const f32x2 cb = MB ? pack2(__ldg(&bp->cb[2 * p]), __ldg(&bp->cb[2 * p + 1])) : pack2(s_cb[2 * p], s_cb[2 * p + 1]);
+      const uint32_t rid = (uint32_t)((MB ? bp->r0 : a.r0) + 2 * p);
+      f32x2 ss = 0;
+#pragma unroll
+      for (int m = 0; m < E; ++m) {
+        const float2 z0 = unpack2(fma2(as, v[m].re, cb)), z1 = unpack2(fma2(as, v[m].im, cb));
+        if constexpr (AM) {
+          const int sh = 16 * (m & 1);
+          auto win = [&](float z, float& best, uint32_t r, int s) {
+            if (z > best) {
+              best = z;
+              am[m >> 1] = (am[m >> 1] & ~(0xFFu << s)) | (r << s);
+            }
+          };
+          win(z0.x, zr[m].x, rid, sh);
+          win(z0.y, zr[m].x, rid + 1, sh);
+          win(z1.x, zr[m].y, rid, sh + 8);
+          win(z1.y, zr[m].y, rid + 1, sh + 8);
+        } else {
+          // fmaxf: as in k_c2r_zp
+          zr[m].x = fmaxf(fmaxf(zr[m].x, z0.x), z0.y);
+          zr[m].y = fmaxf(fmaxf(zr[m].y, z1.x), z1.y);
+        }
+        if constexpr (SIG) ss = fma2(v[m].re, v[m].re, fma2(v[m].im, v[m].im, ss));
+      }
+      if constexpr (SIG) {
+        float2 s = unpack2(ss);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+          s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+        }
+        if ((threadIdx.x & 31) == 0) {
+          atomicAdd(&red[2 * p], (double)s.x);
+          atomicAdd(&red[2 * p + 1], (double)s.y);  // (the filler of an odd sweep: never read)
+        }
+      }
+    }
+    const long long l = line();
+    float2* zout = reinterpret_cast<float2*>((MB ? bp->zreion_out : a.zreion_out) + l * N);
+    uint16_t* aout = AM ? reinterpret_cast<uint16_t*>((MB ? bp->argmax_out : a.argmax_out) + l * N) : nullptr;
+    if constexpr (SP == 1) {
+      if (!dead) {
+#pragma unroll
+        for (int m = 0; m < E; ++m) zout[t + G * m] = zr[m];
+        if constexpr (AM) {
+#pragma unroll
+          for (int m = 0; m < E; ++m) aout[t + G * m] = (uint16_t)(am[m >> 1] >> (16 * (m & 1)));
+        }
+      }
+    } else {
+      // merge the warps' maxima through their exchange buffers: warp w writes
+      // its values, then merges and stores elements m = w*E/SP ...
+      constexpr int LANES = 32, WB = (KK::NL / SP) * LS * 16;  // bytes of a warp's buffers
+      static_assert(E * LANES * 10 <= WB, "room for the maxima");
+      char* const base = reinterpret_cast<char*>(xbuf);
+      auto zb = [&](int w) { return reinterpret_cast<float2*>(base + w * WB) + (threadIdx.x & 31); };
+      auto ab = [&](int w) { return reinterpret_cast<uint16_t*>(base + w * WB + E * LANES * 8) + (threadIdx.x & 31); };
+      __syncwarp();  // the warp's last exchange has been read
+#pragma unroll
+      for (int m = 0; m < E; ++m) {
+        zb(sub)[m * LANES] = zr[m];
+        if constexpr (AM) ab(sub)[m * LANES] = (uint16_t)(am[m >> 1] >> (16 * (m & 1)));
+      }
+      __syncthreads();
+#pragma unroll
+      for (int k = 0; k < E / SP; ++k) {
+        const int m = sub * (E / SP) + k;
+        float2 z = zb(0)[m * LANES];
+        uint32_t w0 = AM ? ab(0)[m * LANES] : 0u;
+        uint32_t x = w0 & 0xFFu, y = w0 >> 8;
+#pragma unroll
+        for (int w = 1; w < SP; ++w) {
+          const float2 o = zb(w)[m * LANES];
+          if constexpr (AM) {
+            const uint32_t q = ab(w)[m * LANES], qx = q & 0xFFu, qy = q >> 8;
+            if (o.x > z.x || (o.x == z.x && qx < x)) x = qx;
+            if (o.y > z.y || (o.y == z.y && qy < y)) y = qy;
+          }
+          z.x = fmaxf(z.x, o.x);
+          z.y = fmaxf(z.y, o.y);
+        }
+        zout[t + G * m] = z;
+        if constexpr (AM) aout[t + G * m] = (uint16_t)(x | (y << 8));
+      }
+      __syncthreads();  // the buffers are free again
+    }
   }
+  pdl_release();
   asm volatile("cp.async.wait_all;\n" ::: "memory");
   if constexpr (SIG) {
     __syncthreads();
