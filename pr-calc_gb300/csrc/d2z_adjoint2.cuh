@@ -1,0 +1,140 @@
+// d2z_adjoint2.cuh — the adjoint's z pass on pairs of radii (k_adj_z of
+// d2z_adjoint.cuh on fft2.cuh): h_R = A dL/dz [argmax == R] along z, its
+// half-complex spectrum into the pair slot, and the sums for dL/dB_R.
+//
+// A warp works alone (two warps a line at 1024): a line's dL/dz and argmax are
+// read once and kept in registers for all pairs of the sweep, and only the
+// transform's exchanges and the mirror X[H-k] go through shared memory.
+#pragma once
+#include "d2z_adjoint.cuh"
+#include "d2z_lines2.cuh"
+
+namespace prc {
+
+template <int N> struct AK2 {
+  using P = typename LCfg<N>::P;  // the plan of k_adj_z
+  static constexpr int H = N / 2, E = P::E, G = H / E, THREADS = 128, NG = THREADS / G;
+  static constexpr int MINB = E == 12 ? 3 : 4;  // CTAs per SM (12 elements a lane: 168 registers)
+  static constexpr int PD = E == 12 ? 24 : 8;
+  static constexpr int pads = H + H / PD;
+  static constexpr int LS = G >= 8 ? pads : pads + ((G - pads % 8) % 8 + 8) % 8;
+  static constexpr int TW = (PlanRun<P>::TW + 1) & ~1;
+  static constexpr size_t bytes = (size_t)(H + TW) * 8 + (size_t)NG * LS * 16;
+  static_assert(G >= 2 && G <= 64 && NG * G == THREADS, "whole lines");
+};
+
+template <int N>
+__global__ void __launch_bounds__(AK2<N>::THREADS, AK2<N>::MINB) k_adj_z2(const __grid_constant__ AdjArgs a) {
+  using KK = AK2<N>;
+  using P = typename KK::P;
+  using L = PairSlot<N>;
+  using Buf = PairLine<KK::PD>;
+  constexpr int H = N / 2, E = KK::E, G = KK::G, NG = KK::NG;
+  constexpr long long NN = (long long)N * N;
+  static_assert(NN % NG == 0, "whole line groups");
+  extern __shared__ float4 smem4[];
+  float2* tw = reinterpret_cast<float2*>(smem4);  // e^{2 pi i k/N}, k < H
+  float2* tws = tw + H;
+  ulonglong2* xbuf = reinterpret_cast<ulonglong2*>(tws + KK::TW);
+  load_tw(tw, a.tw, H);
+  PlanRun<P>::template fill<2>(tws, a.tw);
+  __shared__ double red[kMaxBatch];
+  if (threadIdx.x < kMaxBatch) red[threadIdx.x] = 0.0;
+  pdl_wait();
+  __syncthreads();
+  const int g = threadIdx.x / G, t = threadIdx.x % G;
+  const Buf buf{xbuf + g * KK::LS};
+  const GroupSync<G> sync(g);
+  const bool want_db = a.dB != nullptr;
+  const int np = (a.nb + 1) >> 1;
+  // A unit is the W consecutive lines (iy) of a warp, which its sums for
+  // dL/dB_R run over; units take the planes of a block first, so that the
+  // pieces written next to one another are written at the same time.
+  constexpr int W = G < 32 ? 32 / G : 1, UPC = NG / W;
+  for (int s = blockIdx.x; s < (int)(NN / NG); s += gridDim.x) {
+    const int u0 = s * UPC + g / W, xi = u0 % L::XB, q0 = u0 / L::XB;
+    const int ix = q0 / (N / W) * L::XB + xi, iy = q0 % (N / W) * W + g % W;
+    const int l = ix * N + iy;
+    const float2* gl = reinterpret_cast<const float2*>(a.g + (long long)l * N);
+    const uchar2* al = reinterpret_cast<const uchar2*>(a.am + (long long)l * N);
+    float2 gv[E];
+    uchar2 u[E];
+#pragma unroll
+    for (int m = 0; m < E; ++m) {
+      gv[m] = gl[t + G * m];
+      u[m] = al[t + G * m];
+    }
+    for (int p = 0; p < np; ++p) {
+      // (no argmax byte is 256: the second half of an odd sweep's last pair)
+      const int ra = a.r0 + 2 * p, rb = 2 * p + 1 < a.nb ? ra + 1 : 256;
+      Cx2 v[E];
+      f32x2 part = 0;
+      {
+        float2 h0[E], h1[E];  // (radius a, radius b) of cells 2p and 2p + 1
+#pragma unroll
+        for (int m = 0; m < E; ++m) {
+          h0[m] = make_float2(u[m].x == ra ? gv[m].x : 0.f, u[m].x == rb ? gv[m].x : 0.f);
+          h1[m] = make_float2(u[m].y == ra ? gv[m].y : 0.f, u[m].y == rb ? gv[m].y : 0.f);
+          part = add2(part, add2(pack2(h0[m].x, h0[m].y), pack2(h1[m].x, h1[m].y)));
+        }
+        adj_layer<E, FirstRadix<P>::v>(v, a.A, h0, h1);
+      }
+      if (want_db) {
+        float2 q = unpack2(part);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          q.x += __shfl_xor_sync(0xffffffffu, q.x, o);
+          q.y += __shfl_xor_sync(0xffffffffu, q.y, o);
+        }
+        if ((threadIdx.x & 31) == 0) {
+          atomicAdd(&red[2 * p], (double)q.x);
+          if (2 * p + 1 < a.nb) atomicAdd(&red[2 * p + 1], (double)q.y);
+        }
+      }
+      // Z = DFT_H of (even + i odd cells); X[k] = Ze[k] + e^{-2 pi i k/N} Zo[k]
+      PlanRun2x<P>::template run<false, true>(v, buf, t, tws, sync);
+      sync();  // the last exchange has been read
+      if constexpr (G % KK::PD != 0) {
+#pragma unroll
+        for (int m = 0; m < E; ++m) buf.put_pos(t + G * m, v[m]);
+      } else {
+        const int h = Buf::off(t);
+#pragma unroll
+        for (int m = 0; m < E; ++m) buf.put(h, G * m, v[m]);
+      }
+      sync();
+      ulonglong2* const slot = reinterpret_cast<ulonglong2*>(a.slots) + (long long)p * a.slot_stride;
+      static_assert(G % L::T == 0 || L::T % G == 0, "a lane's positions split");
+      ulonglong2* const dst = slot + L::at(ix, iy, t);  // positions t + G*m: along(G*m) on
+      // mirrors H - t - G*m: (G - t) + (H - G*(m+1)), lane 0's first: itself
+      const int hm = Buf::off(t ? G - t : G);
+      const f32x2 half = dup2(0.5f), mhalf = dup2(-0.5f);
+#pragma unroll
+      for (int m = 0; m < E; ++m) {
+        const int k = t + G * m;
+        Cx2 q;
+        if constexpr (G % KK::PD != 0) q = buf.get_pos(k ? H - k : 0);
+        else if (m == 0) q = buf.get_pos(t ? H - t : 0);
+        else q = buf.get(hm, H - G * (m + 1));
+        const Cx2 z = v[m];
+        const Cx2 ze = {mul2(add2(z.re, q.re), half), mul2(sub2(z.im, q.im), half)};
+        const Cx2 zo = {mul2(add2(z.im, q.im), half), mul2(sub2(z.re, q.re), mhalf)};
+        const float2 w = tw[k];
+        const f32x2 wx = dup2(w.x), wy = dup2(w.y);
+        const Cx2 x = {add2(ze.re, fma2(wx, zo.re, mul2(wy, zo.im))),
+                       add2(ze.im, fma2(wx, zo.im, neg2(mul2(wy, zo.re))))};
+        dst[L::along(G * m)] = make_ulonglong2(x.re, x.im);
+        if (m == 0 && t == 0)  // X[H] = Ze[0] - Zo[0], into the transposed scratch plane
+          slot[NN * (H + 1) + (long long)iy * N + ix] = make_ulonglong2(sub2(ze.re, zo.re), 0ull);
+      }
+      sync();  // the mirrors have been read
+    }
+  }
+  pdl_release();
+  if (want_db) {
+    __syncthreads();
+    if (threadIdx.x < a.nb) atomicAdd(&a.dB[a.r0 + threadIdx.x], (double)a.A * red[threadIdx.x]);
+  }
+}
+
+}  // namespace prc

@@ -411,7 +411,7 @@ void pair_rows(const KernelSet& ks, TileSeg* s) {
 }
 
 // one column pass over the main array and the Nyquist plane
-// (pair: TM_WIN or TM_INV on pair slots; gy then counts pairs)
+// (pair: on pair slots; gy then counts pairs)
 void run_tile(prc_d2z_ctx* c, int mode, TileSeg s0, TileSeg s1, int gy, int nb = 1, int r0 = 0, int first = 0,
               bool pair = false) {
   TileArgs a;
@@ -419,11 +419,12 @@ void run_tile(prc_d2z_ctx* c, int mode, TileSeg s0, TileSeg s1, int gy, int nb =
   const bool faithful = mode == TM_WIN && (c->flags & PRC_FLAG_FAITHFUL_WINDOW);
   const int wv = faithful ? 0 : c->win_var;  // the faithful window runs on variant 0's tiles
   if (pair || mode == TM_WIN || mode == TM_ACC) {  // these passes may use narrower tiles
-    const int tw = pair ? (mode == TM_WIN ? c->ksl.pair_tile_w_win : c->ksl.pair_tile_w)
+    const bool xpass = mode == TM_WIN || mode == TM_ACC;
+    const int tw = pair ? (xpass ? c->ksl.pair_tile_w_win : c->ksl.pair_tile_w)
                         : mode == TM_WIN ? c->ksl.tile_w_winv[wv] : c->ksl.tile_w_acc;
     s0.tpo = (s0.nyq ? c->N : c->H) / tw;
     s1.tpo = (s1.nyq ? c->N : c->H) / tw;
-    if (pair && mode == TM_INV) pair_rows(c->ksl, &s0);
+    if (pair && !xpass) pair_rows(c->ksl, &s0);
   }
   a.seg[0] = s0;
   a.seg[1] = s1;
@@ -444,7 +445,9 @@ void run_tile(prc_d2z_ctx* c, int mode, TileSeg s0, TileSeg s1, int gy, int nb =
     if (pair && nb % 2) a.kr[nb] = a.kr[nb - 1];  // the last pair's second half: any radius (its barrier never wins)
   }
   const int tiles = s0.n_outer * s0.tpo + s1.n_outer * s1.tpo;
-  const int occ = pair ? (mode == TM_WIN ? c->ksl.occ_pair_win : c->ksl.occ_pair_inv)
+  const int occ = pair ? (mode == TM_WIN   ? c->ksl.occ_pair_win
+                          : mode == TM_INV ? c->ksl.occ_pair_inv
+                          : mode == TM_FWD ? c->ksl.occ_pair_fwd : c->ksl.occ_pair_acc)
                 : (mode == TM_ACC) ? c->ksl.occ_tile_acc
                 : faithful         ? c->ksl.occ_win_faithful
                 : (mode == TM_WIN) ? c->ksl.occ_winv[wv] : c->ksl.occ_tile;
@@ -1338,8 +1341,10 @@ int prc_d2z_backward(prc_d2z_ctx* c, const float* dL_dz, const uint8_t* argmax, 
   PRC_CU(cudaEventRecord(c->ev[0], c->st), "event");
   float2* U = c->slots;
   float2* acc = c->spec;
-  for (int r0 = 0; r0 < c->nr; r0 += c->B) {
-    const int nb = (c->nr - r0 < c->B) ? c->nr - r0 : c->B;
+  const int B = sweep_len(c);
+  for (int r0 = 0; r0 < c->nr; r0 += B) {
+    const int nb = (c->nr - r0 < B) ? c->nr - r0 : B;
+    const bool pair = paired(c) && nb > 1;
     AdjArgs aa;
     memset(&aa, 0, sizeof(aa));
     aa.g = d_g;
@@ -1353,13 +1358,18 @@ int prc_d2z_backward(prc_d2z_ctx* c, const float* dL_dz, const uint8_t* argmax, 
     aa.r0 = r0;
     {
       Prof pf(c, PRC_KIND_ADJ_Z);
-      c->ks->adj_z(c->ksl, grid_for(N * N, c->ksl.line_groups, c->ksl.occ_adj_z, c->sms), c->st, aa);
+      if (pair)
+        c->ks->pair_adj_z(c->ksl, grid_for(N * N, c->ksl.pair_adj_lines, c->ksl.occ_pair_adj, c->sms), c->st, aa);
+      else
+        c->ks->adj_z(c->ksl, grid_for(N * N, c->ksl.line_groups, c->ksl.occ_adj_z, c->sms), c->st, aa);
     }
     c->launches++;
+    float2* UQ = U + NN * H * (pair ? 2 : 1);         // Nyquist plane, and the scratch plane after it,
+    float2* UT = U + NN * (H + 1) * (pair ? 2 : 1);   // of the first pair or radius
     // forward y pass of each slot; Nyquist scratch Qt_b -> Q_b[ix][ky]
-    run_tile(c, TM_FWD, mseg(c, U, U, false), qseg(c, U + NN * (H + 1), U + NN * H, true), nb);
+    run_tile(c, TM_FWD, mseg(c, U, U, false), qseg(c, UT, UQ, true), pair ? (nb + 1) / 2 : nb, 1, 0, 0, pair);
     // forward x pass of each slot, acc += W_b * (.)
-    run_tile(c, TM_ACC, mseg(c, U, acc, true), qseg(c, U + NN * H, acc + NN * H, false), 1, nb, r0, r0 == 0);
+    run_tile(c, TM_ACC, mseg(c, U, acc, true), qseg(c, UQ, acc + NN * H, false), 1, nb, r0, r0 == 0, pair);
   }
   PRC_CU(cudaEventRecord(c->ev[1], c->st), "event");
   // inverse of the accumulated spectrum into slot 0, then the z C2R

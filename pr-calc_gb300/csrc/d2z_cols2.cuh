@@ -64,16 +64,17 @@ template <int T, int PD> struct PairCol {
 
 template <int N, int MODE> struct CK2 {
   using P = typename CCfg<N>::P;
-  static constexpr int H = N / 2, T = MODE == TM_WIN ? C2Cfg<N>::TWIN : C2Cfg<N>::T;
+  static constexpr bool XP = MODE == TM_WIN || MODE == TM_ACC;  // an x pass: tiles of the slot's pieces
+  static constexpr int H = N / 2, T = XP ? C2Cfg<N>::TWIN : C2Cfg<N>::T;
   static constexpr int E = P::E, G = N / E, THREADS = T * G, EH = E / 2;
-  static constexpr int MINB = MODE == TM_WIN ? C2Cfg<N>::MINBWIN : C2Cfg<N>::MINB;
+  static constexpr int MINB = XP ? C2Cfg<N>::MINBWIN : C2Cfg<N>::MINB;
   static_assert(T == 16 || (T == 8 && G >= 4) || (T == 4 && G >= 8), "lane layouts");
   static_assert(THREADS % 32 == 0 && H % T == 0, "whole warps, whole tiles");
   static constexpr int TW = (PlanRun<P>::TW + 1) & ~1;
   static constexpr int PD = FirstRadix<P>::v == 12 ? 4 : 16;
   using Buf = PairCol<T, PD>;
   static constexpr int ROWS = T == 4 ? N + N / PD : N;
-  // Inverse y pass: the tile by cp.async (16 bytes, past the L1 cache) instead
+  // y passes: the tile by cp.async (16 bytes, past the L1 cache) instead
   // of loads into registers.  What such loads have in flight needs room in the
   // L1; at 256^3 a carve-out that another stream's kernel has enlarged slows
   // the pass from 0.635 to 0.94 ms for 32 radii, and at 1024^3 two CTAs' shared
@@ -81,9 +82,9 @@ template <int N, int MODE> struct CK2 {
   // The copies take one more trip through shared memory: 0.642 against 0.635
   // ms at 256, 0.381 against 0.356 at 192^3 x 41, 1.404 against 1.364 at 384 x
   // 16, so those sizes and the smaller ones load into registers.
-  static constexpr bool ASYNC = MODE == TM_INV && N >= 256 && N != 384;
-  // stage twiddles, exchange buffer, (window pass) the spectrum tile
-  static constexpr size_t bytes = (size_t)TW * 8 + (size_t)ROWS * T * 16 + (MODE == TM_WIN ? (size_t)N * T * 8 : 0);
+  static constexpr bool ASYNC = (MODE == TM_INV || MODE == TM_FWD) && N >= 256 && N != 384;
+  // stage twiddles, exchange buffer, (x passes) the spectrum tile or the sums
+  static constexpr size_t bytes = (size_t)TW * 8 + (size_t)ROWS * T * 16 + (XP ? (size_t)N * T * 8 : 0);
 };
 
 template <int THREADS> struct CtaSync2 {
@@ -141,8 +142,10 @@ __device__ __forceinline__ f32x2 tophat_big2(float kq, float kra, float krb) {
   return mul2(mul2(dup2(3.0f), fma2(neg2(x), c, s)), mul2(mul2(ix, ix), ix));
 }
 
-// MODE: TM_INV (blockIdx.y: the pair) or TM_WIN (the spectrum tile stays in
-// shared memory, each thread's own elements, for all pairs of the sweep).
+// MODE: TM_INV, TM_FWD (blockIdx.y: the pair), TM_WIN (the spectrum tile stays
+// in shared memory, each thread's own elements, for all pairs of the sweep) or
+// TM_ACC (per pair: forward transform, W times it added to the tile's sums,
+// which stay in shared memory likewise; one read-modify-write of the output).
 // MB: grouped launch, as in k_col; a.nvb counts boxes per pair there.
 template <int N, int MODE, bool MB = false>
 __global__ void __launch_bounds__(CK2<N, MODE>::THREADS, CK2<N, MODE>::MINB) k_col2(const __grid_constant__ TileArgs a) {
@@ -151,19 +154,21 @@ __global__ void __launch_bounds__(CK2<N, MODE>::THREADS, CK2<N, MODE>::MINB) k_c
   using L = PairSlot<N>;
   // the window's products are fused into the first stage's additions
   constexpr bool PRE = MODE == TM_WIN;
+  constexpr bool INV = MODE == TM_INV || MODE == TM_WIN, XP = KK::XP;
   constexpr int H = N / 2, E = KK::E, G = KK::G, T = KK::T, EH = KK::EH, TH = KK::THREADS;
-  static_assert(MODE == TM_INV || MODE == TM_WIN, "pair passes");
+  static_assert(!MB || INV, "no grouped adjoint passes");
   extern __shared__ float4 smem4[];
   float2* tws = reinterpret_cast<float2*>(smem4);
   ulonglong2* xbuf = reinterpret_cast<ulonglong2*>(tws + KK::TW);
   float2* raw = reinterpret_cast<float2*>(xbuf + KK::ROWS * T) + threadIdx.x;  // element m at raw[m * TH]
   __shared__ float s_kr[kMaxBatch];
-  if constexpr (MODE == TM_WIN && !MB) stage_params_all(s_kr, a.kr);
+  if constexpr (XP && !MB) stage_params_all(s_kr, a.kr);
   PlanRun<P>::template fill<1>(tws, a.tw);
   pdl_wait();
   __syncthreads();
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, c = lane & (T - 1);
-  using F = ColFft<N, P>;
+  // (TM_ACC: the final rows pair up with the mirrors of the first, t + G*m)
+  using F = ColFft<N, typename std::conditional<MODE == TM_ACC, Plan<P::E>, P>::type>;
   // FFT lane t of the first stage.  A warp holds lanes and their mirrors G - t
   // (lane ^ 16; t = 0 pairs with G/2), for the window.
   int t;
@@ -189,7 +194,7 @@ __global__ void __launch_bounds__(CK2<N, MODE>::THREADS, CK2<N, MODE>::MINB) k_c
   using Buf = typename KK::Buf;
   const Buf buf{xbuf + c};
   const CtaSync2<TH> sync;
-  const long long yoff = MODE == TM_INV ? (long long)blockIdx.y * a.slot_stride : 0;
+  const long long yoff = XP ? 0 : (long long)blockIdx.y * a.slot_stride;
   const int tiles0 = a.seg[0].n_outer * a.seg[0].tpo;
   const int tpb = tiles0 + a.seg[1].n_outer * a.seg[1].tpo;
   const int tiles = !MB ? tpb : tpb * (MODE == TM_INV ? a.nvb[blockIdx.y] : a.nbox);
@@ -226,11 +231,11 @@ __global__ void __launch_bounds__(CK2<N, MODE>::THREADS, CK2<N, MODE>::MINB) k_c
   auto seg_rs = [&](const Where& w) { return w.sn ? a.seg[1].row_stride : a.seg[0].row_stride; };
   auto transform = [&](Cx2 (&v)[E]) {
     if constexpr (!F::TAIL) {
-      PlanRun2x<P>::template run<true, PRE>(v, buf, t, tws, sync);
+      PlanRun2x<P>::template run<INV, PRE>(v, buf, t, tws, sync);
     } else {
       constexpr int R2 = N / 256, K = 16 / R2, U = 32 / T / R2;
       const int own = Buf::off(16 * t);
-      Dft2x<16, true, PRE>::run(v);
+      Dft2x<16, INV, PRE>::run(v);
 #pragma unroll
       for (int r = 0; r < 16; ++r) buf.put(own, r, v[r]);
       sync();
@@ -240,8 +245,8 @@ __global__ void __launch_bounds__(CK2<N, MODE>::THREADS, CK2<N, MODE>::MINB) k_c
       sync();  // every lane has read: the rows may be written again
       const int u = j & 15;
 #pragma unroll
-      for (int r = 1; r < 16; ++r) v[r] = ctwid<true>(v[r], tws[(r - 1) * 16 + u]);
-      Dft2x<16, true>::run(v);
+      for (int r = 1; r < 16; ++r) v[r] = ctwid<INV>(v[r], tws[(r - 1) * 16 + u]);
+      Dft2x<16, INV>::run(v);
 #pragma unroll
       for (int r = 0; r < 16; ++r) buf.put(own, r, v[r]);
       __syncwarp();
@@ -257,8 +262,8 @@ __global__ void __launch_bounds__(CK2<N, MODE>::THREADS, CK2<N, MODE>::MINB) k_c
         for (int q = 0; q < R2; ++q) a[q] = buf.get(src[q], r);
         const int k = K * 16 * (j >> 4) + 16 * r + u;
 #pragma unroll
-        for (int q = 1; q < R2; ++q) a[q] = ctwid<true>(a[q], tws[240 + (q - 1) * 256 + k]);
-        Dft2x<R2, true>::run(a);
+        for (int q = 1; q < R2; ++q) a[q] = ctwid<INV>(a[q], tws[240 + (q - 1) * 256 + k]);
+        Dft2x<R2, INV>::run(a);
 #pragma unroll
         for (int q = 0; q < R2; ++q) v[r + K * q] = a[q];
       }
@@ -295,7 +300,57 @@ __global__ void __launch_bounds__(CK2<N, MODE>::THREADS, CK2<N, MODE>::MINB) k_c
     }
   };
 
-  if constexpr (MODE == TM_INV) {
+  // |k| of rows t + G*m, m <= E/2, of this thread's column (-1: k = 0);
+  // returns the warp's smallest
+  auto kmag = [&](const Where& w, float (&kq)[EH + 1]) {
+    const int col = w.tc * T + c;
+    const int syz = (w.sn ? a.seg[1].nyq : a.seg[0].nyq) ? fsq(col, N) + H * H : fsq(w.outer, N) + col * col;
+#pragma unroll
+    for (int m = 0; m <= EH; ++m) {
+      const int m2 = fsq(t + G * m, N) + syz;
+      kq[m] = (m2 == 0) ? -1.f : sqrtf((float)m2);
+    }
+    float kmin = kq[0];
+#pragma unroll
+    for (int m = 1; m <= EH; ++m) kmin = fminf(kmin, kq[m]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) kmin = fminf(kmin, __shfl_xor_sync(0xffffffffu, kmin, o));
+    return kmin;
+  };
+  // W(|k| R) of all E rows for the two radii
+  auto windows = [&](const float (&kq)[EH + 1], float kmin, float kra, float krb, float2 (&wm)[E]) {
+    f32x2 wv[EH + 1];
+#pragma unroll
+    for (int m = 0; m <= EH; ++m) wv[m] = tophat_big2(kq[m], kra, krb);
+    if (kmin * fminf(kra, krb) < 1.0f) {
+      // some lane of the warp needs the series (or W(0) = 0)
+#pragma unroll
+      for (int m = 0; m <= EH; ++m) {
+        const float xa = kq[m] * kra, xb = kq[m] * krb;
+        float2 ww = unpack2(wv[m]);
+        if (xa < 1.0f) ww.x = kq[m] < 0.f ? 0.f : tophat_small(xa);
+        if (xb < 1.0f) ww.y = kq[m] < 0.f ? 0.f : tophat_small(xb);
+        wv[m] = pack2(ww.x, ww.y);
+      }
+    }
+    // rows m > E/2 mirror rows of the partner lane (lane ^ 16, FFT lane
+    // G - t, register E-1-m), or of this lane (t = 0: E-m; t = G/2:
+    // E-1-m; both in the first warp)
+#pragma unroll
+    for (int m = 0; m <= EH; ++m) wm[m] = unpack2(wv[m]);
+#pragma unroll
+    for (int m = EH + 1; m < E; ++m) {
+      const float2 s = wm[E - 1 - m];
+      float2 o = make_float2(__shfl_xor_sync(0xffffffffu, s.x, 16), __shfl_xor_sync(0xffffffffu, s.y, 16));
+      if (wp == 0) {
+        if (t == 0) o = wm[E - m];
+        if (t == G / 2) o = s;
+      }
+      wm[m] = o;
+    }
+  };
+
+  if constexpr (MODE == TM_INV || MODE == TM_FWD) {
     auto src = [&](const Where& w) {
       return reinterpret_cast<const ulonglong2*>(seg_in(w)) + yoff + w.off + (long long)t * seg_rs(w) + c;
     };
@@ -341,6 +396,70 @@ __global__ void __launch_bounds__(CK2<N, MODE>::THREADS, CK2<N, MODE>::MINB) k_c
         gstore(w, seg_out(w) + yoff, v);
       }
     }
+  } else if constexpr (MODE == TM_ACC) {
+    // The sums of a tile (raw) and its exchange buffer; a pair's tile is copied
+    // into the exchange buffer by cp.async like the y passes' tiles, the next
+    // one when the last exchange of this one has been read.
+    const int own = Buf::off(t);
+    auto load = [&](const Where& w, int p) {
+      const ulonglong2* base = reinterpret_cast<const ulonglong2*>(seg_in(w)) + (long long)p * a.slot_stride + c;
+      const int rs = seg_rs(w);
+      if constexpr (G % L::XB == 0) {
+        const ulonglong2* q = base + (w.sn ? w.off + (long long)t * rs : L::at(t, w.outer, w.tc * T));
+        const long long step = w.sn ? (long long)G * rs : (long long)G * N * H;
+#pragma unroll
+        for (int m = 0; m < E; ++m) cp_async16(buf.b + own + Buf::off(G * m), q + m * step);
+      } else {
+#pragma unroll
+        for (int m = 0; m < E; ++m)
+          cp_async16(buf.b + own + Buf::off(G * m),
+                     base + (w.sn ? w.off + (long long)(t + G * m) * rs : L::at(t + G * m, w.outer, w.tc * T)));
+      }
+    };
+    const int np = (a.nb + 1) >> 1;
+    int ti = blockIdx.x;
+    if (ti < tiles) load(where(ti), 0);
+    for (; ti < tiles; ti += gridDim.x) {
+      const Where w = where(ti);
+      float kq[EH + 1];
+      const float kmin = kmag(w, kq);
+#pragma unroll
+      for (int m = 0; m < E; ++m) raw[m * TH] = make_float2(0.f, 0.f);
+      for (int p = 0; p < np; ++p) {
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+        Cx2 v[E];
+#pragma unroll
+        for (int m = 0; m < E; ++m) v[m] = buf.get(own, G * m);
+        sync();  // every thread has its elements: the buffer is free for the exchanges
+        transform(v);
+        sync();  // the last exchange has been read
+        if (p + 1 < np) load(w, p + 1);
+        else if (ti + (int)gridDim.x < tiles) load(where(ti + gridDim.x), 0);
+        float2 wm[E];
+        windows(kq, kmin, s_kr[2 * p], s_kr[2 * p + 1], wm);
+        const bool two = 2 * p + 1 < a.nb;
+#pragma unroll
+        for (int m = 0; m < E; ++m) {
+          const float2 re = unpack2(v[m].re), im = unpack2(v[m].im);
+          float2 s = raw[m * TH];
+          s.x = fmaf(wm[m].x, re.x, s.x);
+          s.y = fmaf(wm[m].x, im.x, s.y);
+          if (two) {
+            s.x = fmaf(wm[m].y, re.y, s.x);
+            s.y = fmaf(wm[m].y, im.y, s.y);
+          }
+          raw[m * TH] = s;
+        }
+      }
+      const int rs = seg_rs(w);
+      float2* q = (w.sn ? a.seg[1].out : a.seg[0].out) + w.off + (long long)t * rs + c;
+      const long long step = (long long)G * rs;
+#pragma unroll
+      for (int m = 0; m < E; ++m) {
+        const float2 o = a.first ? make_float2(0.f, 0.f) : q[m * step], s = raw[m * TH];
+        q[m * step] = make_float2(o.x + s.x, o.y + s.y);
+      }
+    }
   } else {
     auto load_raw = [&](int ti) {
       const Where w = where(ti);
@@ -355,22 +474,8 @@ __global__ void __launch_bounds__(CK2<N, MODE>::THREADS, CK2<N, MODE>::MINB) k_c
     cp_async_commit();
     for (; ti < tiles; ti += gridDim.x) {
       const Where w = where(ti);
-      // |k| of rows t + G*m, m <= E/2 (-1: k = 0), and the warp's smallest
       float kq[EH + 1];
-      {
-        const int col = w.tc * T + c;
-        const int syz = (w.sn ? a.seg[1].nyq : a.seg[0].nyq) ? fsq(col, N) + H * H : fsq(w.outer, N) + col * col;
-#pragma unroll
-        for (int m = 0; m <= EH; ++m) {
-          const int m2 = fsq(t + G * m, N) + syz;
-          kq[m] = (m2 == 0) ? -1.f : sqrtf((float)m2);
-        }
-      }
-      float kmin = kq[0];
-#pragma unroll
-      for (int m = 1; m <= EH; ++m) kmin = fminf(kmin, kq[m]);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) kmin = fminf(kmin, __shfl_xor_sync(0xffffffffu, kmin, o));
+      const float kmin = kmag(w, kq);
       cp_async_wait<0>();
       int p0 = 0, p1;
       if constexpr (MB) p1 = (__ldg(&a.box[w.bx].nb) + 1) >> 1;
@@ -386,36 +491,8 @@ __global__ void __launch_bounds__(CK2<N, MODE>::THREADS, CK2<N, MODE>::MINB) k_c
           kra = s_kr[2 * p];
           krb = s_kr[2 * p + 1];
         }
-        f32x2 wv[EH + 1];
-#pragma unroll
-        for (int m = 0; m <= EH; ++m) wv[m] = tophat_big2(kq[m], kra, krb);
-        if (kmin * fminf(kra, krb) < 1.0f) {
-          // some lane of the warp needs the series (or W(0) = 0)
-#pragma unroll
-          for (int m = 0; m <= EH; ++m) {
-            const float xa = kq[m] * kra, xb = kq[m] * krb;
-            float2 ww = unpack2(wv[m]);
-            if (xa < 1.0f) ww.x = kq[m] < 0.f ? 0.f : tophat_small(xa);
-            if (xb < 1.0f) ww.y = kq[m] < 0.f ? 0.f : tophat_small(xb);
-            wv[m] = pack2(ww.x, ww.y);
-          }
-        }
-        // rows m > E/2 mirror rows of the partner lane (lane ^ 16, FFT lane
-        // G - t, register E-1-m), or of this lane (t = 0: E-m; t = G/2:
-        // E-1-m; both in the first warp)
         float2 wm[E];
-#pragma unroll
-        for (int m = 0; m <= EH; ++m) wm[m] = unpack2(wv[m]);
-#pragma unroll
-        for (int m = EH + 1; m < E; ++m) {
-          const float2 s = wm[E - 1 - m];
-          float2 o = make_float2(__shfl_xor_sync(0xffffffffu, s.x, 16), __shfl_xor_sync(0xffffffffu, s.y, 16));
-          if (wp == 0) {
-            if (t == 0) o = wm[E - m];
-            if (t == G / 2) o = s;
-          }
-          wm[m] = o;
-        }
+        windows(kq, kmin, kra, krb, wm);
         Cx2 v[E];
         scaled_layer<E, FirstRadix<P>::v>(v, [&](int m) { return raw[m * TH]; }, [&](int m) { return wm[m]; });
         reuse();

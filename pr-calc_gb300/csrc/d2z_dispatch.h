@@ -38,8 +38,10 @@ struct KernelSet {
   // per block of a pair slot, tile widths, lines per CTA step, resident CTAs
   int pair;
   int pair_xb, pair_tile_w, pair_tile_w_win, pair_lines;
-  int occ_pair_inv, occ_pair_win, occ_pair_c2r;
-  void (*pair_tile)(const KernelSet&, int mode, dim3 grid, cudaStream_t, const TileArgs&);  // TM_INV, TM_WIN
+  int pair_adj_lines;  // lines per CTA step of the adjoint's z pass
+  int occ_pair_inv, occ_pair_win, occ_pair_c2r, occ_pair_fwd, occ_pair_acc, occ_pair_adj;
+  void (*pair_tile)(const KernelSet&, int mode, dim3 grid, cudaStream_t, const TileArgs&);
+  void (*pair_adj_z)(const KernelSet&, int grid, cudaStream_t, const AdjArgs&);
   void (*pair_c2r)(const KernelSet&, int grid, cudaStream_t, const SweepArgs&);
   // grouped launches (several boxes of this size per launch), when compiled
   // for this size (grouped = 1): forward z pass, forward column passes, and

@@ -1,6 +1,6 @@
 // d2z_launch.cuh — host launchers for one grid size; included by inst_*.cu.
 #pragma once
-#include "d2z_adjoint.cuh"
+#include "d2z_adjoint2.cuh"
 #include "d2z_cols.cuh"
 #include "d2z_dispatch.h"
 #include "d2z_kernels.cuh"
@@ -164,7 +164,8 @@ template <int N> struct C2rLaunch<N, true> {
 };
 
 // The sweep's passes on pairs of radii (grids with both a column and a z-line
-// plan): window + inverse x, inverse y, inverse z; MB: grouped launches.
+// plan): window + inverse x, inverse y, inverse z (MB: grouped launches), and
+// the adjoint's z, forward y and accumulating x passes.
 template <int N, bool ON = C2Cfg<N>::on> struct PairLaunch {
   static constexpr bool on = false;
 };
@@ -175,6 +176,19 @@ template <int N> struct PairLaunch<N, true> {
   using KZ = PK2<N>;
   using KZM = PK2<N, true>;
   template <bool MB> static void* win_fn() { return reinterpret_cast<void*>(&k_col2<N, TM_WIN, MB>); }
+  using KF = CK2<N, TM_FWD>;
+  using KA = CK2<N, TM_ACC>;
+  using KS = AK2<N>;
+  static void* fwd_fn() { return reinterpret_cast<void*>(&k_col2<N, TM_FWD>); }
+  static void* acc_fn() { return reinterpret_cast<void*>(&k_col2<N, TM_ACC>); }
+  static void* adj_fn() { return reinterpret_cast<void*>(&k_adj_z2<N>); }
+  static void tile_adj(int mode, dim3 grid, cudaStream_t st, const TileArgs& a) {
+    if (mode == TM_FWD) launch_pdl(&k_col2<N, TM_FWD>, grid, KF::THREADS, KF::bytes, st, a);
+    else launch_pdl(&k_col2<N, TM_ACC>, grid, KA::THREADS, KA::bytes, st, a);
+  }
+  static void adj_z(int grid, cudaStream_t st, const AdjArgs& a) {
+    launch_pdl(&k_adj_z2<N>, grid, KS::THREADS, KS::bytes, st, a);
+  }
   template <bool MB> static void* inv_fn() { return reinterpret_cast<void*>(&k_col2<N, TM_INV, MB>); }
   template <bool AM, bool SIG, bool MB> static void* z_fn() { return reinterpret_cast<void*>(&k_c2r_zp2<N, AM, SIG, MB>); }
   template <bool MB> static void tile(int mode, dim3 grid, cudaStream_t st, const TileArgs& a) {
@@ -242,6 +256,12 @@ template <int N> struct Launchers {
       if ((e = smem(v, PL::KI::bytes)) != cudaSuccess) return e;
       for (void* f : z)
         if ((e = smem(f, PL::KZ::bytes)) != cudaSuccess) return e;
+      if ((e = smem(PL::fwd_fn(), PL::KF::bytes)) != cudaSuccess) return e;
+      if ((e = smem(PL::acc_fn(), PL::KA::bytes)) != cudaSuccess) return e;
+      if ((e = smem(PL::adj_fn(), PL::KS::bytes)) != cudaSuccess) return e;
+      if ((e = occ(&ks->occ_pair_fwd, PL::fwd_fn(), PL::KF::THREADS, PL::KF::bytes)) != cudaSuccess) return e;
+      if ((e = occ(&ks->occ_pair_acc, PL::acc_fn(), PL::KA::THREADS, PL::KA::bytes)) != cudaSuccess) return e;
+      if ((e = occ(&ks->occ_pair_adj, PL::adj_fn(), PL::KS::THREADS, PL::KS::bytes)) != cudaSuccess) return e;
       if ((e = occ(&ks->occ_pair_win, w, PL::KW::THREADS, PL::KW::bytes)) != cudaSuccess) return e;
       if ((e = occ(&ks->occ_pair_inv, v, PL::KI::THREADS, PL::KI::bytes)) != cudaSuccess) return e;
       if ((e = occ(&ks->occ_pair_c2r, z[1], PL::KZ::THREADS, PL::KZ::bytes)) != cudaSuccess) return e;
@@ -297,7 +317,13 @@ template <int N> struct Launchers {
     if constexpr (CL::GROUPED) PL::c2r_mb(grid, st, a);
   }
   static void pair_tile(const KernelSet&, int mode, dim3 grid, cudaStream_t st, const TileArgs& a) {
-    if constexpr (PL::on) PL::template tile<false>(mode, grid, st, a);
+    if constexpr (PL::on) {
+      if (mode == TM_FWD || mode == TM_ACC) PL::tile_adj(mode, grid, st, a);
+      else PL::template tile<false>(mode, grid, st, a);
+    }
+  }
+  static void pair_adj_z(const KernelSet&, int grid, cudaStream_t st, const AdjArgs& a) {
+    if constexpr (PL::on) PL::adj_z(grid, st, a);
   }
   static void pair_c2r(const KernelSet&, int grid, cudaStream_t st, const SweepArgs& a) {
     if constexpr (PL::on) PL::c2r(grid, st, a);
@@ -336,6 +362,8 @@ template <int N> struct Launchers {
       ks.pair_tile_w = PL::KI::T;
       ks.pair_tile_w_win = PL::KW::T;
       ks.pair_lines = PL::KZ::NG;
+      ks.pair_adj_lines = PL::KS::NG;
+      ks.pair_adj_z = &pair_adj_z;
       ks.pair_tile = &pair_tile;
       ks.pair_c2r = &pair_c2r;
     }

@@ -63,6 +63,7 @@ template <int PD> struct PairLine {
     const ulonglong2 q = b[off(p)];
     return {q.x, q.y};
   }
+  __device__ __forceinline__ void put_pos(int p, Cx2 v) const { b[off(p)] = make_ulonglong2(v.re, v.im); }
   __device__ __forceinline__ void put(int h, int cp, Cx2 v) const { b[h + off(cp)] = make_ulonglong2(v.re, v.im); }
 };
 

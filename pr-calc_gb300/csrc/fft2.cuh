@@ -242,6 +242,36 @@ template <int E, int R0, class X, class W> __device__ __forceinline__ void scale
   }
 }
 
+// The same for the adjoint's sources A * (h0 + i h1), h0 and h1 pairs of reals.
+template <int E, int R0> __device__ __forceinline__ void adj_layer(Cx2* v, float A, const float2* h0, const float2* h1) {
+  const f32x2 aa = dup2(A);
+  auto pk = [](float2 h) { return pack2(h.x, h.y); };
+  // (scalar products: packed ones would be fused into a packed addition)
+  auto sc = [&](float2 h) { return pack2(__fmul_rn(A, h.x), __fmul_rn(A, h.y)); };
+  auto scale = [&](int m) { return Cx2{sc(h0[m]), sc(h1[m])}; };
+  auto fused = [&](int m, Cx2 c) { return Cx2{fma2(aa, pk(h0[m]), c.re), fma2(aa, pk(h1[m]), c.im)}; };
+  auto minus = [](Cx2 c) { return Cx2{neg2(c.re), neg2(c.im)}; };
+  if constexpr (R0 == 12) {
+    const f32x2 mh = dup2(-0.5f);
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+      const int i0 = (3 * n) % 12, i1 = (4 + 3 * n) % 12, i2 = (8 + 3 * n) % 12;
+      const Cx2 z = scale(i0), p = scale(i1);
+      const Cx2 t1 = fused(i2, p);
+      v[i2] = minus(fused(i2, minus(p)));
+      v[i1] = {fma2(mh, t1.re, z.re), fma2(mh, t1.im, z.im)};
+      v[i0] = cadd(z, t1);
+    }
+  } else {
+#pragma unroll
+    for (int m = 0; m < E / 2; ++m) {
+      const Cx2 q = scale(m + E / 2);
+      v[m] = fused(m, q);
+      v[m + E / 2] = fused(m, minus(q));
+    }
+  }
+}
+
 // ---------------------------------------------------------------- Stockham
 // As Stages in fft.cuh.  Buf addresses are sums: off(p) is the offset of
 // position p, and off(a + b) = off(a) + off(b) for the splits used here (a

@@ -41,3 +41,29 @@ def test_pairs_match_single_radius(N, nr, batch):
         del zr
     assert torch.equal(z, best)
     assert torch.equal(am, win)
+
+
+# the adjoint of a context with the faithful float window runs the
+# single-radius kernels (with the same accurate window as any other): the same
+# sums in the same order, so the same bits (dL/dB_R up to the order of its
+# double-precision additions)
+@pytest.mark.parametrize("N,nr,batch", [(32, 5, 0), (64, 9, 4), (96, 3, 0), (128, 8, 6), (192, 4, 2), (256, 5, 0),
+                                        (384, 3, 0), (512, 3, 2), (768, 2, 0), (1024, 2, 0)])
+def test_adjoint_pairs_match_single_radius(N, nr, batch):
+    import torch
+    box = 1.5 * N
+    cl = prc_d2z.CLParameters(Rmax=min(0.4 * box, 60.0), zeta=30.0, M_min=1.47e9)
+    t = prc_d2z.compute_tables(prc_d2z.Parameters(N=N, Nscales=nr, BoxSize=box), cl)
+    gen = torch.Generator(device="cuda").manual_seed(7 * N + nr)
+    g = torch.randn((N, N, N), device="cuda", generator=gen)
+    am = torch.randint(0, nr + 1, (N, N, N), device="cuda", generator=gen, dtype=torch.uint8)
+    am[am == nr] = prc_d2z.PRC_ARGMAX_NONE
+    out = []
+    for faithful in (False, True):
+        with prc_d2z.Delta2Zreion(N, float(np.float32(box) / np.float32(0.68)), t.radii_mpc, t.barrier_b, t.barrier_a,
+                                  t.DInit, radius_batch=batch, faithful_window=faithful) as ctx:
+            out.append(ctx.backward(g, am))
+    (d, db), (d1, db1) = out
+    assert torch.equal(d, d1)
+    # sums of about N^3/nr random terms of size A: compared on that scale
+    assert np.max(np.abs(db - db1)) <= 1e-12 * t.barrier_a * N ** 1.5
