@@ -242,10 +242,14 @@ __global__ void __launch_bounds__(CK2<N, MODE>::THREADS, CK2<N, MODE>::MINB) k_c
       const int hr = Buf::off(j);
 #pragma unroll
       for (int m = 0; m < 16; ++m) v[m] = buf.get(hr, G * m);
-      sync();  // every lane has read: the rows may be written again
+      if constexpr (R2 > 2) sync();  // every lane has read: the rows may be written again
       const int u = j & 15;
 #pragma unroll
       for (int r = 1; r < 16; ++r) v[r] = ctwid<INV>(v[r], tws[(r - 1) * 16 + u]);
+      if constexpr (R2 == 2) {
+        last_two_stages<INV>(v, j, tws);
+        return;
+      }
       Dft2x<16, INV>::run(v);
 #pragma unroll
       for (int r = 0; r < 16; ++r) buf.put(own, r, v[r]);
@@ -269,10 +273,10 @@ __global__ void __launch_bounds__(CK2<N, MODE>::THREADS, CK2<N, MODE>::MINB) k_c
       }
     }
   };
-  // the previous transform's last exchange has been read by its readers: the
-  // CTA, or (TAIL) this warp alone
+  // the previous transform's last exchange through memory has been read by its
+  // readers: the CTA, or (R2 = 4) this warp alone
   auto reuse = [&]() {
-    if constexpr (F::TAIL) __syncwarp();
+    if constexpr (F::TAIL && N > 512) __syncwarp();
     else sync();
   };
   auto gstore = [&](const Where& w, ulonglong2* dst, const Cx2 (&v)[E]) {

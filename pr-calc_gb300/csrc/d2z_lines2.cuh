@@ -49,6 +49,37 @@ template <int N, bool MB = false> struct PK2 {
   static constexpr size_t bytes = (size_t)(QT + TW) * 8 + (size_t)(NL * LS + E * THREADS + NL) * 16;
 };
 
+// The transform of a line and the positions it leaves in a lane: register m
+// holds position pos(t) + step(m).  A <16, 16, 2> plan on 32 lanes (1024) ends
+// without its second exchange (last_two_stages), but for the per-radius sums
+// (SIG), which add up the cells of a lane in a fixed order.
+template <class P, bool SIG> struct LineFft {
+  static constexpr int L = PlanRun<P>::L, G = L / P::E;
+  static __device__ __forceinline__ int pos(int t) { return t; }
+  static __device__ __forceinline__ constexpr int step(int m) { return G * m; }
+  template <class Buf, class Sync>
+  static __device__ __forceinline__ void run(Cx2 (&v)[P::E], const Buf& buf, int t, const float2* tws, const Sync& sync) {
+    PlanRun2x<P>::template run<true>(v, buf, t, tws, sync);
+  }
+};
+template <> struct LineFft<Plan<16, 16, 16, 2>, false> {
+  static __device__ __forceinline__ int pos(int t) { return (t & 15) + 128 * (t >> 4); }
+  static __device__ __forceinline__ constexpr int step(int m) { return 16 * (m % 8) + 256 * (m / 8); }
+  template <class Buf, class Sync>
+  static __device__ __forceinline__ void run(Cx2 (&v)[16], const Buf& buf, int t, const float2* tws, const Sync& sync) {
+    Dft2x<16, true>::run(v);
+    const int hw = Buf::off(16 * t), hr = Buf::off(t);
+#pragma unroll
+    for (int r = 0; r < 16; ++r) buf.put(hw, r, v[r]);
+    sync();
+#pragma unroll
+    for (int m = 0; m < 16; ++m) v[m] = buf.get(hr, 32 * m);
+#pragma unroll
+    for (int r = 1; r < 16; ++r) v[r] = ctwid<true>(v[r], tws[(r - 1) * 16 + (t & 15)]);
+    last_two_stages<true>(v, t, tws);
+  }
+};
+
 // Offsets add except where reads of a 12-point plan (PD = 24) meet a lane's
 // position t: there each is formed by itself (Stages2x: get_pos).
 template <int PD> struct PairLine {
@@ -89,6 +120,7 @@ __global__ void __launch_bounds__(PK2<N, MB>::THREADS, PK2<N, MB>::MINB) k_c2r_z
   using KK = PK2<N, MB>;
   using P = typename KK::P;
   using L = PairSlot<N>;
+  using F = LineFft<P, SIG>;
   constexpr int H = N / 2, E = KK::E, G = KK::G, NG = KK::NG, EH = E / 2, LS = KK::LS, TH = KK::THREADS;
   constexpr int SP = KK::SP;
   constexpr long long NN = (long long)N * N;
@@ -110,6 +142,7 @@ __global__ void __launch_bounds__(PK2<N, MB>::THREADS, PK2<N, MB>::MINB) k_c2r_z
   const int g = SP == 1 ? lb : lb % NG;                 // line of the group
   const GroupSync<G> sync(lb);
   const int partner = (G - t) & (G - 1);
+  const int t0 = F::pos(t);  // first cell pair of the lane after the transform
   constexpr int lgpb = (int)(NN / NG);  // line groups of one box
   const long long lg_all = MB ? (long long)lgpb * a.nbox : lgpb;
   const int nsteps_l = (int)((lg_all - blockIdx.x + gridDim.x - 1) / gridDim.x);
@@ -195,12 +228,12 @@ __global__ void __launch_bounds__(PK2<N, MB>::THREADS, PK2<N, MB>::MINB) k_c2r_z
       const long long l = line();
       const float2* zline = reinterpret_cast<const float2*>((MB ? bp->zreion : a.zreion) + l * N);
 #pragma unroll
-      for (int m = 0; m < E; ++m) zr[m] = zline[t + G * m];
+      for (int m = 0; m < E; ++m) zr[m] = zline[t0 + F::step(m)];
       if constexpr (AM) {
         const uint16_t* aline = reinterpret_cast<const uint16_t*>((MB ? bp->argmax : a.argmax) + l * N);
 #pragma unroll
         for (int j = 0; j < EH; ++j)
-          am[j] = (uint32_t)aline[t + G * (2 * j)] | ((uint32_t)aline[t + G * (2 * j + 1)] << 16);
+          am[j] = (uint32_t)aline[t0 + F::step(2 * j)] | ((uint32_t)aline[t0 + F::step(2 * j + 1)] << 16);
       }
     }
     for (int p = sub; p < np && (SP == 1 || !dead); p += SP, ++i) {
@@ -247,7 +280,7 @@ __global__ void __launch_bounds__(PK2<N, MB>::THREADS, PK2<N, MB>::MINB) k_c2r_z
       }
       issue(lg_next, p_next);
       const PairLine<KK::PD> buf{xbuf + lb * LS};
-      PlanRun2x<P>::template run<true>(v, buf, t, tws, sync);
+      F::run(v, buf, t, tws, sync);
       const f32x2 as = dup2(MB ? bp->as : a.as);
       const f32x2 cb = MB ? pack2(__ldg(&bp->cb[2 * p]), __ldg(&bp->cb[2 * p + 1])) : pack2(s_cb[2 * p], s_cb[2 * p + 1]);
       const uint32_t rid = (uint32_t)((MB ? bp->r0 : a.r0) + 2 * p);
@@ -293,10 +326,10 @@ __global__ void __launch_bounds__(PK2<N, MB>::THREADS, PK2<N, MB>::MINB) k_c2r_z
     if constexpr (SP == 1) {
       if (!dead) {
 #pragma unroll
-        for (int m = 0; m < E; ++m) zout[t + G * m] = zr[m];
+        for (int m = 0; m < E; ++m) zout[t0 + F::step(m)] = zr[m];
         if constexpr (AM) {
 #pragma unroll
-          for (int m = 0; m < E; ++m) aout[t + G * m] = (uint16_t)(am[m >> 1] >> (16 * (m & 1)));
+          for (int m = 0; m < E; ++m) aout[t0 + F::step(m)] = (uint16_t)(am[m >> 1] >> (16 * (m & 1)));
         }
       }
     } else {
@@ -331,8 +364,8 @@ __global__ void __launch_bounds__(PK2<N, MB>::THREADS, PK2<N, MB>::MINB) k_c2r_z
           z.x = fmaxf(z.x, o.x);
           z.y = fmaxf(z.y, o.y);
         }
-        zout[t + G * m] = z;
-        if constexpr (AM) aout[t + G * m] = (uint16_t)(x | (y << 8));
+        zout[t0 + F::step(m)] = z;
+        if constexpr (AM) aout[t0 + F::step(m)] = (uint16_t)(x | (y << 8));
       }
       __syncthreads();  // the buffers are free again
     }

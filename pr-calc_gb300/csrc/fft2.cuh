@@ -207,6 +207,75 @@ template <bool INV, bool PRE> struct Dft2x<16, INV, PRE> {
   }
 };
 
+// The 16-point DFT whose last layer's sums and differences change places where
+// s = -1 (s = +1: Dft2x<16>): a[k] = e[k] + s t[k], a[k + 8] = e[k] - s t[k].
+// The products by s are exact, so the values keep their bits.
+template <bool INV> __device__ __forceinline__ void dft16_signed(Cx2* a, float s) {
+  const f32x2 p = dup2(s), m = dup2(-s), c = dup2(s * PRC_SQRT1_2), mc = dup2(-s * PRC_SQRT1_2);
+  Cx2 e[8], o[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    e[k] = a[2 * k];
+    o[k] = a[2 * k + 1];
+  }
+  Dft2x<8, INV>::run(e);
+  Dft2x<8, INV>::run(o);
+  auto pm = [&](int k, Cx2 t) {
+    a[k] = {fma2(t.re, p, e[k].re), fma2(t.im, p, e[k].im)};
+    a[k + 8] = {fma2(t.re, m, e[k].re), fma2(t.im, m, e[k].im)};
+  };
+  // e +- s w8 o, e +- s w8^3 o: comb_w8_1 and comb_w8_3 with c for sqrt(1/2)
+  auto w81 = [&](int k) {
+    const f32x2 d = sub2(o[k].re, o[k].im), q = add2(o[k].re, o[k].im);
+    a[k] = INV ? Cx2{fma2(d, c, e[k].re), fma2(q, c, e[k].im)} : Cx2{fma2(q, c, e[k].re), fma2(d, mc, e[k].im)};
+    a[k + 8] = INV ? Cx2{fma2(d, mc, e[k].re), fma2(q, mc, e[k].im)} : Cx2{fma2(q, mc, e[k].re), fma2(d, c, e[k].im)};
+  };
+  auto w83 = [&](int k) {
+    const f32x2 d = sub2(o[k].re, o[k].im), q = add2(o[k].re, o[k].im);
+    a[k] = INV ? Cx2{fma2(q, mc, e[k].re), fma2(d, c, e[k].im)} : Cx2{fma2(d, mc, e[k].re), fma2(q, mc, e[k].im)};
+    a[k + 8] = INV ? Cx2{fma2(q, c, e[k].re), fma2(d, mc, e[k].im)} : Cx2{fma2(d, c, e[k].re), fma2(q, c, e[k].im)};
+  };
+  pm(0, o[0]);
+  pm(1, ctwid<INV>(o[1], make_float2(PRC_COS_PI8, PRC_SIN_PI8)));
+  w81(2);
+  pm(3, ctwid<INV>(o[3], make_float2(PRC_SIN_PI8, PRC_COS_PI8)));
+  // s i o[4] and its negative
+  const f32x2 ip = INV ? p : m, im = INV ? m : p;
+  a[4] = {fma2(o[4].im, im, e[4].re), fma2(o[4].re, ip, e[4].im)};
+  a[12] = {fma2(o[4].im, ip, e[4].re), fma2(o[4].re, im, e[4].im)};
+  pm(5, ctwid<INV>(o[5], make_float2(-PRC_SIN_PI8, PRC_COS_PI8)));
+  w83(6);
+  pm(7, ctwid<INV>(o[7], make_float2(-PRC_COS_PI8, PRC_SIN_PI8)));
+}
+
+// The second and third stage of a <16, 16, 2> plan of length 512 whose lanes j
+// and j ^ 16 are lanes of one warp (lane ^ 16).  v: the second stage's inputs
+// j + 32*m with their twiddles applied.  The last butterflies join positions k
+// and k + 256, which the second stage leaves in lanes u and u + 16: each keeps
+// eight of its values and gives the other eight to its partner by shuffles (no
+// exchange through shared memory: 5.07 -> 4.32 ms where the exchange inside
+// the warp through memory took 4.64, the window pass of 32 radii at 512^3).
+// With the sums and differences of lane u + 16 changed places, those given are
+// v[8..15] in both lanes.  Out: v[r + 8*q] is position u + 128*(j / 16) + 16*r
+// + 256*q.
+template <bool INV> __device__ __forceinline__ void last_two_stages(Cx2 (&v)[16], int j, const float2* tws) {
+  const int u = j & 15, h = j >> 4;
+  dft16_signed<INV>(v, h ? -1.f : 1.f);
+  auto swap = [](f32x2 x) {
+    const float2 f = unpack2(x);
+    return pack2(__shfl_xor_sync(0xffffffffu, f.x, 16), __shfl_xor_sync(0xffffffffu, f.y, 16));
+  };
+#pragma unroll
+  for (int r = 0; r < 8; ++r) {
+    const Cx2 got = {swap(v[r + 8].re), swap(v[r + 8].im)}, kept = v[r];
+    Cx2 a[2] = {h ? got : kept, h ? kept : got};
+    a[1] = ctwid<INV>(a[1], tws[240 + 128 * h + 16 * r + u]);
+    Dft2x<2, INV>::run(a);
+    v[r] = a[0];
+    v[r + 8] = a[1];
+  }
+}
+
 // The first layer of the first stage (radix R0, E elements a lane) on real
 // multiples x[m] * w[m] of complex numbers x[m].  The compiler fuses these
 // products into the additions in the one-field kernel; the same ones are fused
