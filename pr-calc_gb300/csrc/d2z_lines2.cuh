@@ -290,16 +290,16 @@ __global__ void __launch_bounds__(PK2<N, MB>::THREADS, PK2<N, MB>::MINB) k_c2r_z
         const float2 z0 = unpack2(fma2(as, v[m].re, cb)), z1 = unpack2(fma2(as, v[m].im, cb));
         if constexpr (AM) {
           const int sh = 16 * (m & 1);
-          auto win = [&](float z, float& best, uint32_t r, int s) {
-            if (z > best) {
-              best = z;
-              am[m >> 1] = (am[m >> 1] & ~(0xFFu << s)) | (r << s);
-            }
+          // the pair's larger value (the first radius's of equal ones; fmaxf
+          // drops a NaN), then the strict comparison with the running maximum
+          auto win = [&](float2 z, float& best, int s) {
+            const float zm = fmaxf(z.x, z.y);
+            const uint32_t who = (z.x == zm ? rid : rid + 1) << s;
+            if (zm > best) am[m >> 1] = (am[m >> 1] & ~(0xFFu << s)) | who;
+            best = fmaxf(best, zm);
           };
-          win(z0.x, zr[m].x, rid, sh);
-          win(z0.y, zr[m].x, rid + 1, sh);
-          win(z1.x, zr[m].y, rid, sh + 8);
-          win(z1.y, zr[m].y, rid + 1, sh + 8);
+          win(z0, zr[m].x, sh);
+          win(z1, zr[m].y, sh + 8);
         } else {
           // fmaxf: as in k_c2r_zp
           zr[m].x = fmaxf(fmaxf(zr[m].x, z0.x), z0.y);
