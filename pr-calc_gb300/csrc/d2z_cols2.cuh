@@ -499,13 +499,14 @@ __global__ void __launch_bounds__(CK2<N, MODE>::THREADS, CK2<N, MODE>::MINB) k_c
         windows(kq, kmin, kra, krb, wm);
         Cx2 v[E];
         scaled_layer<E, FirstRadix<P>::v>(v, [&](int m) { return raw[m * TH]; }, [&](int m) { return wm[m]; });
-        reuse();
-        transform(v);
         if (p == p1 - 1) {
-          // this thread has read its spectrum elements for the last time
+          // this thread has read its spectrum elements for the last time: the
+          // next tile's come in under the transform and the stores
           if (ti + (int)gridDim.x < tiles) load_raw(ti + gridDim.x);
           cp_async_commit();
         }
+        reuse();
+        transform(v);
         gstore(w, out + (long long)p * a.slot_stride, v);
       }
     }
