@@ -359,6 +359,24 @@ int sweep_len(const prc_d2z_ctx* c) {
   return c->B + 1 <= c->slots_b ? c->B + 1 : c->B - 1;
 }
 
+// Whether a sweep of nb radii runs in pairs.  The last pair of an odd sweep is
+// filled up, and a pair of radii costs nearly two, so from 256^3 on few and odd
+// radii stay with the single-radius kernels.  The lines are where one whole
+// step took the same time either way (pairs against single radii: 256^3 x 5
+// 435 / 396 us, x 11 705 / 704; 384^3 x 5 1654 / 1603, x 7 2064 / 2089; 512^3 x 4
+// 2573 / 2528, x 6 3355 / 3394, x 7 4169 / 3831, x 15 7.40 / 7.25 ms; 1024^3 x 3
+// 26.3 / 22.6); smaller grids win with any number.  The adjoint gains more from
+// pairs (256^3 x 3 354 / 345 us, x 5 455 / 471; 512^3 x 5 3613 / 3524, x 7 4519 /
+// 4619).
+bool in_pairs(const prc_d2z_ctx* c, int nb, bool adjoint) {
+  if (!paired(c) || nb < 2) return false;
+  const int N = c->N;
+  if (N < 256) return true;
+  if (adjoint) return nb % 2 == 0 || nb >= (N < 512 ? 5 : 7);
+  if (N == 512) return nb >= (nb % 2 ? 21 : 6);
+  return nb % 2 == 0 || nb >= (N == 256 ? 11 : 7);
+}
+
 // Radius slots for a radius batch of B into *out: with one more for an odd
 // batch of a size with pair kernels, if that can be had.
 int alloc_slots(const prc_d2z_ctx* c, int B, float2** out, int* n) {
@@ -511,7 +529,7 @@ void enqueue_sweeps(prc_d2z_ctx* c, float* d_z, uint8_t* d_am, double* sig, floa
   const int B = sweep_len(c);
   for (int r0 = 0; r0 < c->nr; r0 += B) {
     const int nb = (c->nr - r0 < B) ? c->nr - r0 : B;
-    const bool pair = paired(c) && nb > 1;
+    const bool pair = in_pairs(c, nb, false);
     SweepArgs sa;
     memset(&sa, 0, sizeof(sa));
     sa.slots = c->slots;
@@ -626,10 +644,12 @@ void batch_enqueue(prc_d2z_batch* b, const float* const* delta, float* const* zr
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // A box joins a grouped launch when its size has grouped kernels and it asks
-// for nothing they leave out: the faithful window and a single radius (or
-// slot) run per box.  (A tuned window variant is not used there.)
+// for nothing they leave out: the faithful window, a single radius (or slot)
+// and the few odd radii at 256^3 that in_pairs leaves to the single-radius
+// kernels run per box.  (A tuned window variant is not used there.)
 bool groupable(const prc_d2z_ctx* c) {
-  return c->ksl.grouped && !(c->flags & PRC_FLAG_FAITHFUL_WINDOW) && c->nr > 1 && c->slots_b > 1;
+  return c->ksl.grouped && !(c->flags & PRC_FLAG_FAITHFUL_WINDOW) && c->nr > 1 && c->slots_b > 1 &&
+         !(c->N >= 256 && c->nr % 2 && c->nr < 11);
 }
 // radii per sweep of a grouped box (its window variant does not matter)
 int grouped_len(const prc_d2z_ctx* c) {
@@ -1344,7 +1364,7 @@ int prc_d2z_backward(prc_d2z_ctx* c, const float* dL_dz, const uint8_t* argmax, 
   const int B = sweep_len(c);
   for (int r0 = 0; r0 < c->nr; r0 += B) {
     const int nb = (c->nr - r0 < B) ? c->nr - r0 : B;
-    const bool pair = paired(c) && nb > 1;
+    const bool pair = in_pairs(c, nb, true);
     AdjArgs aa;
     memset(&aa, 0, sizeof(aa));
     aa.g = d_g;

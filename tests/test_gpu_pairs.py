@@ -14,9 +14,11 @@ pytestmark = pytest.mark.gpu
 
 
 # every size with pair kernels; odd and even counts, several sweeps, a last
-# sweep of one radius, an odd radius batch
+# sweep of one radius, an odd radius batch, counts on both sides of the lines
+# below which larger grids keep the single-radius kernels
 @pytest.mark.parametrize("N,nr,batch", [(32, 5, 0), (32, 9, 4), (64, 7, 3), (96, 6, 0), (128, 3, 2), (192, 5, 4),
-                                        (256, 4, 3), (384, 3, 0), (512, 3, 0), (768, 2, 0), (1024, 3, 2)])
+                                        (256, 4, 3), (256, 11, 0), (384, 3, 0), (384, 7, 0), (512, 3, 0),
+                                        (512, 6, 0), (512, 21, 0), (768, 2, 0), (1024, 3, 2)])
 def test_pairs_match_single_radius(N, nr, batch):
     import torch
     box = 1.5 * N
