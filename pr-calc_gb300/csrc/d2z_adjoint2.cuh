@@ -4,7 +4,10 @@
 //
 // A warp works alone (two warps a line at 1024): a line's dL/dz and argmax are
 // read once and kept in registers for all pairs of the sweep, and only the
-// transform's exchanges and the mirror X[H-k] go through shared memory.
+// transform's exchanges and the upper half of Z go through shared memory: the
+// lane that holds Z[k], k < H/2, fetches Z[H-k] and forms X[k] and X[H-k] from
+// the two (5.12 -> 4.63 ms for 32 radii at 512^3, 1.20 -> 1.09 for 64 at 256^3,
+// against every lane fetching a mirror for each of its values).
 #pragma once
 #include "d2z_adjoint.cuh"
 #include "d2z_lines2.cuh"
@@ -31,7 +34,10 @@ __global__ void __launch_bounds__(AK2<N>::THREADS, AK2<N>::MINB) k_adj_z2(const 
   using Buf = PairLine<KK::PD>;
   constexpr int H = N / 2, E = KK::E, G = KK::G, NG = KK::NG;
   constexpr long long NN = (long long)N * N;
-  static_assert(NN % NG == 0, "whole line groups");
+  // a lane's positions t + G*m split into a part of the lane and a constant,
+  // in the exchange buffer and in the slot
+  constexpr bool SPLIT = G % KK::PD == 0 && G % L::T == 0;
+  static_assert(NN % NG == 0 && (G % L::T == 0 || L::T % G == 0), "whole line groups");
   extern __shared__ float4 smem4[];
   float2* tw = reinterpret_cast<float2*>(smem4);  // e^{2 pi i k/N}, k < H
   float2* tws = tw + H;
@@ -94,38 +100,54 @@ __global__ void __launch_bounds__(AK2<N>::THREADS, AK2<N>::MINB) k_adj_z2(const 
       // Z = DFT_H of (even + i odd cells); X[k] = Ze[k] + e^{-2 pi i k/N} Zo[k]
       PlanRun2x<P>::template run<false, true>(v, buf, t, tws, sync);
       sync();  // the last exchange has been read
-      if constexpr (G % KK::PD != 0) {
-#pragma unroll
-        for (int m = 0; m < E; ++m) buf.put_pos(t + G * m, v[m]);
-      } else {
+      if constexpr (SPLIT) {
         const int h = Buf::off(t);
 #pragma unroll
-        for (int m = 0; m < E; ++m) buf.put(h, G * m, v[m]);
+        for (int m = E / 2; m < E; ++m) buf.put(h, G * m, v[m]);
+      } else {
+#pragma unroll
+        for (int m = E / 2; m < E; ++m) buf.put_pos(t + G * m, v[m]);
       }
       sync();
       ulonglong2* const slot = reinterpret_cast<ulonglong2*>(a.slots) + (long long)p * a.slot_stride;
-      static_assert(G % L::T == 0 || L::T % G == 0, "a lane's positions split");
-      ulonglong2* const dst = slot + L::at(ix, iy, t);  // positions t + G*m: along(G*m) on
-      // mirrors H - t - G*m: (G - t) + (H - G*(m+1)), lane 0's first: itself
+      ulonglong2* const line = slot + L::at(ix, iy, 0);
+      // positions k = t + G*m from lo on, their mirrors H - k = (t ? G - t : G)
+      // + (H - G*(m+1)) from hi on
+      ulonglong2* const lo = line + L::along(t);
+      ulonglong2* const hi = line + L::along(t ? G - t : G);
       const int hm = Buf::off(t ? G - t : G);
       const f32x2 half = dup2(0.5f), mhalf = dup2(-0.5f);
-#pragma unroll
-      for (int m = 0; m < E; ++m) {
-        const int k = t + G * m;
-        Cx2 q;
-        if constexpr (G % KK::PD != 0) q = buf.get_pos(k ? H - k : 0);
-        else if (m == 0) q = buf.get_pos(t ? H - t : 0);
-        else q = buf.get(hm, H - G * (m + 1));
-        const Cx2 z = v[m];
-        const Cx2 ze = {mul2(add2(z.re, q.re), half), mul2(sub2(z.im, q.im), half)};
-        const Cx2 zo = {mul2(add2(z.im, q.im), half), mul2(sub2(z.re, q.re), mhalf)};
+      auto out = [&](Cx2 ze, Cx2 zo, int k) {
         const float2 w = tw[k];
         const f32x2 wx = dup2(w.x), wy = dup2(w.y);
-        const Cx2 x = {add2(ze.re, fma2(wx, zo.re, mul2(wy, zo.im))),
-                       add2(ze.im, fma2(wx, zo.im, neg2(mul2(wy, zo.re))))};
-        dst[L::along(G * m)] = make_ulonglong2(x.re, x.im);
-        if (m == 0 && t == 0)  // X[H] = Ze[0] - Zo[0], into the transposed scratch plane
+        return make_ulonglong2(add2(ze.re, fma2(wx, zo.re, mul2(wy, zo.im))),
+                               add2(ze.im, fma2(wx, zo.im, neg2(mul2(wy, zo.re)))));
+      };
+#pragma unroll
+      for (int m = 0; m < E / 2; ++m) {
+        const int k = t + G * m;
+        const Cx2 z = v[m];
+        Cx2 q;
+        if constexpr (!SPLIT) q = k ? buf.get_pos(H - k) : z;
+        else if (m == 0) q = t ? buf.get_pos(H - t) : z;
+        else q = buf.get(hm, H - G * (m + 1));
+        const f32x2 er = mul2(add2(z.re, q.re), half), orr = mul2(add2(z.im, q.im), half);
+        const Cx2 ze = {er, mul2(sub2(z.im, q.im), half)}, zo = {orr, mul2(sub2(z.re, q.re), mhalf)};
+        lo[L::along(G * m)] = out(ze, zo, k);
+        if (m || t) {
+          const Cx2 me = {er, mul2(sub2(q.im, z.im), half)}, mo = {orr, mul2(sub2(q.re, z.re), mhalf)};
+          const ulonglong2 x = out(me, mo, H - k);
+          if constexpr (SPLIT) hi[L::along(H - G * (m + 1))] = x;
+          else line[L::along(H - k)] = x;
+        } else {
+          // X[H] = Ze[0] - Zo[0], into the transposed scratch plane, and H/2,
+          // its own mirror
           slot[NN * (H + 1) + (long long)iy * N + ix] = make_ulonglong2(sub2(ze.re, zo.re), 0ull);
+          const Cx2 c = v[E / 2];
+          const Cx2 ce = {mul2(add2(c.re, c.re), half), mul2(sub2(c.im, c.im), half)};
+          const Cx2 co = {mul2(add2(c.im, c.im), half), mul2(sub2(c.re, c.re), mhalf)};
+          line[L::along(H / 2)] = out(ce, co, H / 2);
+        }
       }
       sync();  // the mirrors have been read
     }

@@ -21,6 +21,11 @@
 // inverse transform, store to the radius slot; the next tile's load is issued
 // during the last radius), TM_ACC (per radius: forward transform of the slot
 // tile, accumulate W_b times it; one read-modify-write of the output).
+//
+// The sweeps of most radius batches run on pairs of radii instead
+// (d2z_cols2.cuh); these kernels serve the forward transform, the last passes
+// of the adjoint, short and some odd sweeps, the faithful window and tuned
+// window variants (in_pairs, d2z_capi.cu).
 #pragma once
 #include <type_traits>
 

@@ -21,6 +21,9 @@
 // Then, per radius of the sweep, the barrier crossing of delta2zreion_d2z.C
 // :206-216 (z = A/N^3 x + (A B_b - 1)) and the running max of :105-146 with
 // strict >, in registers; one zreion / argmax read-modify-write per sweep.
+//
+// Sweeps on pairs of radii run k_c2r_zp2 (d2z_lines2.cuh); this one serves the
+// sweeps of single radii, and the measurements below are of such sweeps.
 #pragma once
 #include "d2z_kernels.cuh"
 
