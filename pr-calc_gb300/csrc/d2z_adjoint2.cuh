@@ -52,6 +52,11 @@ __global__ void __launch_bounds__(AK2<N>::THREADS, AK2<N>::MINB) k_adj_z2(const 
   const Buf buf{xbuf + g * KK::LS};
   const GroupSync<G> sync(g);
   const bool want_db = a.dB != nullptr;
+  // sums for dL/dB_R: lane i of the lower half those of radius a of the pairs i
+  // and i + 16, lane i of the upper half radius b's
+  const int lane = threadIdx.x & 31, up = lane >> 4;
+  double acc0 = 0.0, acc1 = 0.0;
+  static_assert(kMaxBatch <= 64, "two pairs a lane");
   const int np = (a.nb + 1) >> 1;
   // A unit is the W consecutive lines (iy) of a warp, which its sums for
   // dL/dB_R run over; units take the planes of a block first, so that the
@@ -86,16 +91,11 @@ __global__ void __launch_bounds__(AK2<N>::THREADS, AK2<N>::MINB) k_adj_z2(const 
         adj_layer<E, FirstRadix<P>::v>(v, a.A, h0, h1);
       }
       if (want_db) {
-        float2 q = unpack2(part);
+        const float2 q = unpack2(part);
+        float sum = (up ? q.y : q.x) + __shfl_xor_sync(0xffffffffu, up ? q.x : q.y, 16);
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          q.x += __shfl_xor_sync(0xffffffffu, q.x, o);
-          q.y += __shfl_xor_sync(0xffffffffu, q.y, o);
-        }
-        if ((threadIdx.x & 31) == 0) {
-          atomicAdd(&red[2 * p], (double)q.x);
-          if (2 * p + 1 < a.nb) atomicAdd(&red[2 * p + 1], (double)q.y);
-        }
+        for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if ((lane & 15) == (p & 15)) (p < 16 ? acc0 : acc1) += (double)sum;
       }
       // Z = DFT_H of (even + i odd cells); X[k] = Ze[k] + e^{-2 pi i k/N} Zo[k]
       PlanRun2x<P>::template run<false, true>(v, buf, t, tws, sync);
@@ -154,6 +154,9 @@ __global__ void __launch_bounds__(AK2<N>::THREADS, AK2<N>::MINB) k_adj_z2(const 
   }
   pdl_release();
   if (want_db) {
+    const int r = 2 * (lane & 15) + up;
+    if (r < a.nb) atomicAdd(&red[r], acc0);
+    if (r + 32 < a.nb) atomicAdd(&red[r + 32], acc1);
     __syncthreads();
     if (threadIdx.x < a.nb) atomicAdd(&a.dB[a.r0 + threadIdx.x], (double)a.A * red[threadIdx.x]);
   }
