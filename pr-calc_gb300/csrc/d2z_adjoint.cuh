@@ -31,11 +31,20 @@ struct AdjArgs {
   float scale;           // k_c2r_plain scale
 };
 
+// Line plan of the adjoint's z pass.  From 256^3 on sixteen elements a lane: one
+// exchange through shared memory less than the forward pass's eight (32 radii at
+// 512^3 4.44 -> 3.64 ms, 64 at 256^3 1.05 -> 0.92).
+template <int N> struct ACfg { using P = typename LCfg<N>::P; };
+template <> struct ACfg<256> { using P = Plan<16, 16, 8>; };
+template <> struct ACfg<512> { using P = Plan<16, 16, 16>; };
+template <> struct ACfg<1024> { using P = Plan<16, 16, 16, 2>; };
+template <int N> using ALK = LK<N, typename ACfg<N>::P>;
+
 // h_R along z -> half spectrum: main into slot b, X[H] into the slot's
 // transposed Nyquist scratch (offset NN*(H+1)).
 template <int N>
-__global__ void __launch_bounds__(LK<N>::THREADS, LK<N>::MINB) k_adj_z(AdjArgs a) {
-  using KK = LK<N>;
+__global__ void __launch_bounds__(ALK<N>::THREADS, ALK<N>::MINB) k_adj_z(AdjArgs a) {
+  using KK = ALK<N>;
   constexpr int H = N / 2, E = KK::E, G = KK::G, NG = KK::NG;
   constexpr long long NN = (long long)N * N;
   extern __shared__ float4 smem4[];
@@ -77,7 +86,7 @@ __global__ void __launch_bounds__(LK<N>::THREADS, LK<N>::MINB) k_adj_z(AdjArgs a
         for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
         if ((threadIdx.x & 31) == 0) atomicAdd(&red[b], (double)part);
       }
-      const float xh = line_r2c<N>(v, gbuf, t, tw, tws, sync);
+      const float xh = line_r2c<N, KK>(v, gbuf, t, tw, tws, sync);
       if (valid) {
         float2* slot = a.slots + (long long)b * a.slot_stride;
         float2* dst = slot + (long long)l * H;

@@ -2,7 +2,7 @@
 // d2z_adjoint.cuh on fft2.cuh): h_R = A dL/dz [argmax == R] along z, its
 // half-complex spectrum into the pair slot, and the sums for dL/dB_R.
 //
-// A warp works alone (two warps a line at 1024): a line's dL/dz and argmax are
+// A warp works alone: a line's dL/dz and argmax are
 // read once and kept in registers for all pairs of the sweep, and only the
 // transform's exchanges and the upper half of Z go through shared memory: the
 // lane that holds Z[k], k < H/2, fetches Z[H-k] and forms X[k] and X[H-k] from
@@ -15,10 +15,10 @@
 namespace prc {
 
 template <int N> struct AK2 {
-  using P = typename LCfg<N>::P;  // the plan of k_adj_z
+  using P = typename ACfg<N>::P;
   static constexpr int H = N / 2, E = P::E, G = H / E, THREADS = 128, NG = THREADS / G;
-  static constexpr int MINB = E == 12 ? 3 : 4;  // CTAs per SM (12 elements a lane: 168 registers)
-  static constexpr int PD = E == 12 ? 24 : 8;
+  static constexpr int MINB = E >= 12 ? 3 : 4;  // CTAs per SM (12 or 16 elements a lane: 168 registers)
+  static constexpr int PD = E == 12 ? 24 : E;
   static constexpr int pads = H + H / PD;
   static constexpr int LS = G >= 8 ? pads : pads + ((G - pads % 8) % 8 + 8) % 8;
   static constexpr int TW = (PlanRun<P>::TW + 1) & ~1;
@@ -36,7 +36,7 @@ __global__ void __launch_bounds__(AK2<N>::THREADS, AK2<N>::MINB) k_adj_z2(const 
   constexpr long long NN = (long long)N * N;
   // a lane's positions t + G*m split into a part of the lane and a constant,
   // in the exchange buffer and in the slot
-  constexpr bool SPLIT = G % KK::PD == 0 && G % L::T == 0;
+  constexpr bool SPLIT = G % KK::PD == 0, SPLITS = G % L::T == 0;
   static_assert(NN % NG == 0 && (G % L::T == 0 || L::T % G == 0), "whole line groups");
   extern __shared__ float4 smem4[];
   float2* tw = reinterpret_cast<float2*>(smem4);  // e^{2 pi i k/N}, k < H
@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(AK2<N>::THREADS, AK2<N>::MINB) k_adj_z2(const 
       // Z = DFT_H of (even + i odd cells); X[k] = Ze[k] + e^{-2 pi i k/N} Zo[k]
       PlanRun2x<P>::template run<false, true>(v, buf, t, tws, sync);
       sync();  // the last exchange has been read
-      if constexpr (SPLIT) {
+      if constexpr (G % KK::PD == 0 || KK::PD % G == 0) {
         const int h = Buf::off(t);
 #pragma unroll
         for (int m = E / 2; m < E; ++m) buf.put(h, G * m, v[m]);
@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(AK2<N>::THREADS, AK2<N>::MINB) k_adj_z2(const 
         if (m || t) {
           const Cx2 me = {er, mul2(sub2(q.im, z.im), half)}, mo = {orr, mul2(sub2(q.re, z.re), mhalf)};
           const ulonglong2 x = out(me, mo, H - k);
-          if constexpr (SPLIT) hi[L::along(H - G * (m + 1))] = x;
+          if constexpr (SPLITS) hi[L::along(H - G * (m + 1))] = x;
           else line[L::along(H - k)] = x;
         } else {
           // X[H] = Ze[0] - Zo[0], into the transposed scratch plane, and H/2,

@@ -65,9 +65,9 @@ template <> struct TCfg<256> { using P = Plan<16, 16, 16>; static constexpr int 
 template <> struct TCfg<512> { using P = Plan<16, 8, 8, 8>; static constexpr int T = 8, SA = 1, SB = 3; };
 template <> struct TCfg<1024> { using P = Plan<16, 16, 16, 4>; static constexpr int T = 4, SA = 1, SB = 2; };
 
-template <int N> struct LK {
+template <int N, class PL = typename LCfg<N>::P> struct LK {
   static constexpr int H = N / 2;
-  using P = typename LCfg<N>::P;
+  using P = PL;
   static constexpr int E = P::E;
   static constexpr int G = H / E;
   static_assert(PlanRun<P>::L == H, "line plan length");
@@ -662,11 +662,11 @@ __global__ void __launch_bounds__(TK<N>::THREADS, MODE == TM_ACC ? TK<N>::MINB_A
 // Forward real-to-half-complex along a line.  In: v[m] = (x[2p], x[2p+1]) at
 // p = t + G*m.  Out: v[m] = X[k] at k = t + G*m (k < H); returns X[H] (real) in
 // lane t == 0.  Z = DFT_H(x_even + i x_odd); X[k] = Ze[k] + e^{-2 pi i k/N} Zo[k].
-template <int N, class Sync>
-__device__ __forceinline__ float line_r2c(float2 (&v)[LK<N>::E], float2* gbuf, int t, const float2* tw,
+template <int N, class KK = LK<N>, class Sync>
+__device__ __forceinline__ float line_r2c(float2 (&v)[KK::E], float2* gbuf, int t, const float2* tw,
                                           const float2* tws, const Sync& sync) {
-  constexpr int H = N / 2, E = LK<N>::E, G = LK<N>::G;
-  using P = typename LK<N>::P;
+  constexpr int H = N / 2, E = KK::E, G = KK::G;
+  using P = typename KK::P;
   const LineBuf<H> buf{gbuf};
   PlanRun<P>::template run<false>(v, buf, t, tws, sync);
   const int h = buf.thread(t);

@@ -217,6 +217,7 @@ template <int N> struct Launchers {
   using CR = C2rLaunch<N>;
   using LL = LK<N>;
   static constexpr size_t LS = (size_t)LL::smem_f2 * sizeof(float2);
+  static constexpr size_t AS = (size_t)ALK<N>::smem_f2 * sizeof(float2);
 
   template <class F> static cudaError_t smem(F fn, size_t bytes) {
     return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
@@ -289,14 +290,14 @@ template <int N> struct Launchers {
     if ((e = smem(&k_r2c_z<N>, LS)) != cudaSuccess) return e;
     for (int i = 0; i < CR::NFN; ++i)
       if ((e = smem(CR::fn(i), CR::BYTES)) != cudaSuccess) return e;
-    if ((e = smem(&k_adj_z<N>, LS)) != cudaSuccess) return e;
+    if ((e = smem(&k_adj_z<N>, AS)) != cudaSuccess) return e;
     if ((e = smem(&k_c2r_plain<N>, LS)) != cudaSuccess) return e;
     if ((e = occ(&ks->occ_tile, ti, CL::THREADS, CL::bytes(TM_INV))) != cudaSuccess) return e;
     if ((e = occ(&ks->occ_tile_acc, ta, CL::threads(TM_ACC), CL::bytes(TM_ACC))) != cudaSuccess) return e;
     if ((e = occ(&ks->occ_r2c, &k_r2c_z<N>, LL::THREADS, LS)) != cudaSuccess) return e;
     if ((e = occ(&ks->occ_c2r, CR::fn(0), CR::THREADS, CR::BYTES)) != cudaSuccess) return e;
     if ((e = occ(&ks->occ_c2r_plain, &k_c2r_plain<N>, LL::THREADS, LS)) != cudaSuccess) return e;
-    if ((e = occ(&ks->occ_adj_z, &k_adj_z<N>, LL::THREADS, LS)) != cudaSuccess) return e;
+    if ((e = occ(&ks->occ_adj_z, &k_adj_z<N>, ALK<N>::THREADS, AS)) != cudaSuccess) return e;
     return cudaSuccess;
   }
   static void r2c_z(const KernelSet&, int grid, cudaStream_t st, const float* d, float dinit, float2* S,
@@ -333,7 +334,7 @@ template <int N> struct Launchers {
   }
   static void c2r_z(const KernelSet&, int grid, cudaStream_t st, const SweepArgs& a) { CR::launch(grid, st, a); }
   static void adj_z(const KernelSet&, int grid, cudaStream_t st, const AdjArgs& a) {
-    k_adj_z<N><<<grid, LL::THREADS, LS, st>>>(a);
+    k_adj_z<N><<<grid, ALK<N>::THREADS, AS, st>>>(a);
   }
   static void c2r_plain(const KernelSet&, int grid, cudaStream_t st, const AdjArgs& a) {
     k_c2r_plain<N><<<grid, LL::THREADS, LS, st>>>(a);
