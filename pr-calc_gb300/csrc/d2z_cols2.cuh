@@ -167,8 +167,11 @@ __global__ void __launch_bounds__(CK2<N, MODE>::THREADS, CK2<N, MODE>::MINB) k_c
   pdl_wait();
   __syncthreads();
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, c = lane & (T - 1);
-  // (TM_ACC: the final rows pair up with the mirrors of the first, t + G*m)
-  using F = ColFft<N, typename std::conditional<MODE == TM_ACC, Plan<P::E>, P>::type>;
+  // (TM_ACC needs the mirrors of its final rows in the same warp: rows t + G*m,
+  // or at 512 those of the lanes u below, which leave out an exchange: 4.68 ->
+  // 4.33 ms for 32 radii)
+  using F = ColFft<N, typename std::conditional<MODE == TM_ACC && N != 512, Plan<P::E>, P>::type>;
+  constexpr bool ACC_TAIL = MODE == TM_ACC && F::TAIL;
   // FFT lane t of the first stage.  A warp holds lanes and their mirrors G - t
   // (lane ^ 16; t = 0 pairs with G/2), for the window.
   int t;
@@ -188,7 +191,15 @@ __global__ void __launch_bounds__(CK2<N, MODE>::THREADS, CK2<N, MODE>::MINB) k_c
   if constexpr (F::TAIL) {
     constexpr int R2 = N / 256, U = 32 / T / R2;  // values of u a warp
     const int s = lane / T;
-    j = (s / U) * 16 + wp * U + s % U;
+    int u = wp * U + s % U;
+    if constexpr (ACC_TAIL) {
+      // u and 16 - u in one warp: 2 wp, 2 wp + 1 and their mirrors (0 and 8
+      // are their own)
+      static_assert(U == 4, "two values of u and their mirrors");
+      const int i = s % U;
+      u = i < 2 ? 2 * wp + i : (wp == 0 && i == 2 ? 8 : 18 - 2 * wp - i);
+    }
+    j = (s / U) * 16 + u;
   }
   const int row0 = F::TAIL ? (j & 15) + (j >> 4) * (256 / (F::TAIL ? N / 256 : 1)) : t;  // first of the lane's final rows
   using Buf = typename KK::Buf;
@@ -304,14 +315,14 @@ __global__ void __launch_bounds__(CK2<N, MODE>::THREADS, CK2<N, MODE>::MINB) k_c
     }
   };
 
-  // |k| of rows t + G*m, m <= E/2, of this thread's column (-1: k = 0);
-  // returns the warp's smallest
+  // |k| of rows t + G*m (TM_ACC: of the final rows), m <= E/2, of this thread's
+  // column (-1: k = 0); returns the warp's smallest
   auto kmag = [&](const Where& w, float (&kq)[EH + 1]) {
     const int col = w.tc * T + c;
     const int syz = (w.sn ? a.seg[1].nyq : a.seg[0].nyq) ? fsq(col, N) + H * H : fsq(w.outer, N) + col * col;
 #pragma unroll
     for (int m = 0; m <= EH; ++m) {
-      const int m2 = fsq(t + G * m, N) + syz;
+      const int m2 = fsq(MODE == TM_ACC ? row0 + F::rows(m) : t + G * m, N) + syz;
       kq[m] = (m2 == 0) ? -1.f : sqrtf((float)m2);
     }
     float kmin = kq[0];
@@ -342,6 +353,17 @@ __global__ void __launch_bounds__(CK2<N, MODE>::THREADS, CK2<N, MODE>::MINB) k_c
     // E-1-m; both in the first warp)
 #pragma unroll
     for (int m = 0; m <= EH; ++m) wm[m] = unpack2(wv[m]);
+    if constexpr (ACC_TAIL) {
+      // row u + 128 h + 16 r + 256 q mirrors that of 16 - u, 1 - h and register
+      // E-1-m; u = 0: of 0, 1 - h and E-m (but for r = 0, evaluated here)
+      const int u = j & 15, from = lane ^ (u % 8 ? 24 : 16);
+#pragma unroll
+      for (int m = EH + 1; m < E; ++m) {
+        const float2 s = u ? wm[E - 1 - m] : wm[E - m];
+        wm[m] = make_float2(__shfl_sync(0xffffffffu, s.x, from), __shfl_sync(0xffffffffu, s.y, from));
+      }
+      return;
+    }
 #pragma unroll
     for (int m = EH + 1; m < E; ++m) {
       const float2 s = wm[E - 1 - m];
@@ -456,12 +478,12 @@ __global__ void __launch_bounds__(CK2<N, MODE>::THREADS, CK2<N, MODE>::MINB) k_c
         }
       }
       const int rs = seg_rs(w);
-      float2* q = (w.sn ? a.seg[1].out : a.seg[0].out) + w.off + (long long)t * rs + c;
-      const long long step = (long long)G * rs;
+      float2* q = (w.sn ? a.seg[1].out : a.seg[0].out) + w.off + (long long)row0 * rs + c;
 #pragma unroll
       for (int m = 0; m < E; ++m) {
-        const float2 o = a.first ? make_float2(0.f, 0.f) : q[m * step], s = raw[m * TH];
-        q[m * step] = make_float2(o.x + s.x, o.y + s.y);
+        float2* const qm = q + (long long)F::rows(m) * rs;
+        const float2 o = a.first ? make_float2(0.f, 0.f) : *qm, s = raw[m * TH];
+        *qm = make_float2(o.x + s.x, o.y + s.y);
       }
     }
   } else {
