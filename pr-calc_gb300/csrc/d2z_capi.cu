@@ -366,13 +366,13 @@ int sweep_len(const prc_d2z_ctx* c) {
 // 435 / 396 us, x 11 705 / 704; 384^3 x 5 1654 / 1603, x 7 2064 / 2089; 512^3 x 4
 // 2573 / 2528, x 6 3355 / 3394, x 7 4169 / 3831, x 15 7.40 / 7.25 ms; 1024^3 x 3
 // 26.3 / 22.6); smaller grids win with any number.  The adjoint gains more from
-// pairs (256^3 x 3 354 / 345 us, x 5 455 / 471; 512^3 x 5 3613 / 3524, x 7 4519 /
-// 4619).
+// pairs (256^3 x 3 343 / 338 us, 384^3 x 3 1271 / 1209, 512^3 x 3 2502 / 2276,
+// x 5 3258 / 3271, 1024^3 x 3 24.7 / 24.3 ms, x 5 31.8 / 35.1).
 bool in_pairs(const prc_d2z_ctx* c, int nb, bool adjoint) {
   if (!paired(c) || nb < 2) return false;
   const int N = c->N;
   if (N < 256) return true;
-  if (adjoint) return nb % 2 == 0 || nb >= (N < 512 ? 5 : 7);
+  if (adjoint) return nb % 2 == 0 || nb >= 5;
   if (N == 512) return nb >= (nb % 2 ? 21 : 6);
   return nb % 2 == 0 || nb >= (N == 256 ? 11 : 7);
 }

@@ -50,7 +50,7 @@ def test_pairs_match_single_radius(N, nr, batch):
 # sums in the same order, so the same bits (dL/dB_R up to the order of its
 # double-precision additions)
 @pytest.mark.parametrize("N,nr,batch", [(32, 5, 0), (64, 9, 4), (96, 3, 0), (128, 8, 6), (192, 4, 2), (256, 5, 0),
-                                        (384, 3, 0), (512, 3, 2), (768, 2, 0), (1024, 2, 0)])
+                                        (384, 3, 0), (512, 3, 2), (512, 5, 0), (768, 2, 0), (1024, 2, 0)])
 def test_adjoint_pairs_match_single_radius(N, nr, batch):
     import torch
     box = 1.5 * N
