@@ -345,8 +345,8 @@ def run_ours(args, rank, world, local_rank):
     del scratch
     ctx.forward_many([hd, hd], hz)
     # three streams of K boxes, the median reported: the pipelined rate
-    # varies from run to run on a shared machine (28.3 to 34.0 ms a box for
-    # the same build, the device-resident step taking 28.2-28.4 ms); clocks
+    # varies from run to run on a shared machine (by up to a fifth for one
+    # build, the device-resident step's by 1%); clocks
     # and power are sampled over the three
     e2e_reps = []
     with Clocks(local_rank) as clk_e2e:
