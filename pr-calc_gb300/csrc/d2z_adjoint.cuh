@@ -33,7 +33,12 @@ struct AdjArgs {
 
 // Line plan of the adjoint's z pass.  From 256^3 on sixteen elements a lane: one
 // exchange through shared memory less than the forward pass's eight (32 radii at
-// 512^3 4.44 -> 3.64 ms, 64 at 256^3 1.05 -> 0.92).
+// 512^3 4.44 -> 3.57 ms, 64 at 256^3 1.05 -> 0.94).
+//
+// The sums for dL/dB_R run in float over 32 lanes of eight cells and in double
+// from there; with sixteen elements a lane they are still those: the even and
+// the odd elements are the cells of two such lanes, t and t + G, and the sums
+// of different warps' lanes are added in double.
 template <int N> struct ACfg { using P = typename LCfg<N>::P; };
 template <> struct ACfg<256> { using P = Plan<16, 16, 8>; };
 template <> struct ACfg<512> { using P = Plan<16, 16, 16>; };
@@ -70,7 +75,7 @@ __global__ void __launch_bounds__(ALK<N>::THREADS, ALK<N>::MINB) k_adj_z(AdjArgs
     for (int b = 0; b < a.nb; ++b) {
       const uint8_t rid = (uint8_t)(a.r0 + b);
       float2 v[E];
-      float part = 0.f;
+      float part = 0.f, odd = 0.f;  // (odd: of sixteen elements a lane)
 #pragma unroll
       for (int m = 0; m < E; ++m) {
         const int p = t + G * m;
@@ -78,13 +83,28 @@ __global__ void __launch_bounds__(ALK<N>::THREADS, ALK<N>::MINB) k_adj_z(AdjArgs
         uchar2 u = valid ? al[p] : make_uchar2(255, 255);
         const float h0 = (u.x == rid) ? gv.x : 0.f;
         const float h1 = (u.y == rid) ? gv.y : 0.f;
-        part += h0 + h1;
+        if (E == 16 && m % 2) odd += h0 + h1;
+        else part += h0 + h1;
         v[m] = make_float2(a.A * h0, a.A * h1);
       }
       if (want_db) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-        if ((threadIdx.x & 31) == 0) atomicAdd(&red[b], (double)part);
+        auto tree = [](float x, int from) {
+          for (int o = from; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+          return x;
+        };
+        if constexpr (E != 16 || G == 32) {
+          part = tree(part, 16);
+          if constexpr (E == 16) odd = tree(odd, 16);
+          if ((threadIdx.x & 31) == 0) atomicAdd(&red[b], (double)part + (double)odd);
+        } else {
+          static_assert(G == 8 || G == 16, "two or four lines a warp");
+          if constexpr (G == 8) {  // two lines to a sum
+            part += __shfl_xor_sync(0xffffffffu, part, 8);
+            odd += __shfl_xor_sync(0xffffffffu, odd, 8);
+          }
+          part = tree(part + odd, G / 2);
+          if (threadIdx.x % 16 == 0) atomicAdd(&red[b], (double)part);
+        }
       }
       const float xh = line_r2c<N, KK>(v, gbuf, t, tw, tws, sync);
       if (valid) {

@@ -52,9 +52,11 @@ __global__ void __launch_bounds__(AK2<N>::THREADS, AK2<N>::MINB) k_adj_z2(const 
   const Buf buf{xbuf + g * KK::LS};
   const GroupSync<G> sync(g);
   const bool want_db = a.dB != nullptr;
-  // sums for dL/dB_R: lane i of the lower half those of radius a of the pairs i
-  // and i + 16, lane i of the upper half radius b's
-  const int lane = threadIdx.x & 31, up = lane >> 4;
+  // sums for dL/dB_R (ACfg): 16 lanes i (own) keep those of radius a of the pairs
+  // i and i + 16, the other 16 (up) radius b's
+  constexpr bool HALF = E != 16 || G == 32;
+  const int lane = threadIdx.x & 31, up = HALF ? lane >> 4 : (lane >> 3) & 1;
+  const int own = HALF ? lane & 15 : (lane & 7) | (lane >> 4) * 8;
   double acc0 = 0.0, acc1 = 0.0;
   static_assert(kMaxBatch <= 64, "two pairs a lane");
   const int np = (a.nb + 1) >> 1;
@@ -75,27 +77,57 @@ __global__ void __launch_bounds__(AK2<N>::THREADS, AK2<N>::MINB) k_adj_z2(const 
       gv[m] = gl[t + G * m];
       u[m] = al[t + G * m];
     }
+    float mine = 0.f, mine2 = 0.f;
     for (int p = 0; p < np; ++p) {
       // (no argmax byte is 256: the second half of an odd sweep's last pair)
       const int ra = a.r0 + 2 * p, rb = 2 * p + 1 < a.nb ? ra + 1 : 256;
       Cx2 v[E];
-      f32x2 part = 0;
+      f32x2 part = 0, odd = 0;
       {
         float2 h0[E], h1[E];  // (radius a, radius b) of cells 2p and 2p + 1
 #pragma unroll
         for (int m = 0; m < E; ++m) {
           h0[m] = make_float2(u[m].x == ra ? gv[m].x : 0.f, u[m].x == rb ? gv[m].x : 0.f);
           h1[m] = make_float2(u[m].y == ra ? gv[m].y : 0.f, u[m].y == rb ? gv[m].y : 0.f);
-          part = add2(part, add2(pack2(h0[m].x, h0[m].y), pack2(h1[m].x, h1[m].y)));
+          f32x2& sum = E == 16 && m % 2 ? odd : part;
+          sum = add2(sum, add2(pack2(h0[m].x, h0[m].y), pack2(h1[m].x, h1[m].y)));
         }
         adj_layer<E, FirstRadix<P>::v>(v, a.A, h0, h1);
       }
       if (want_db) {
-        const float2 q = unpack2(part);
-        float sum = (up ? q.y : q.x) + __shfl_xor_sync(0xffffffffu, up ? q.x : q.y, 16);
+        // each lane keeps one radius's sum and gives the other away
+        auto split = [&](f32x2 x, int o) {
+          const float2 q = unpack2(x);
+          return (up ? q.y : q.x) + __shfl_xor_sync(0xffffffffu, up ? q.x : q.y, o);
+        };
+        float sum;
+        if constexpr (E != 16) {
+          sum = split(part, 16);
+          sum += __shfl_xor_sync(0xffffffffu, sum, 8);
+        } else if constexpr (G == 32) {  // (8 lanes keep the even elements', 8 the odd ones')
+          const float e = split(part, 16), f = split(odd, 16);
+          sum = (lane & 8 ? f : e) + __shfl_xor_sync(0xffffffffu, lane & 8 ? e : f, 8);
+        } else if constexpr (G == 16) {
+          sum = split(add2(part, odd), 8);
+        } else {
+          static_assert(G == 8, "four lines a warp");
+          sum = split(part, 8) + split(odd, 8);
+        }
 #pragma unroll
-        for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        if ((lane & 15) == (p & 15)) (p < 16 ? acc0 : acc1) += (double)sum;
+        for (int o = 4; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if constexpr (E != 16) {
+          if (own == (p & 15)) (p < 16 ? acc0 : acc1) += (double)sum;
+        } else {
+          const float sum2 = __shfl_xor_sync(0xffffffffu, sum, HALF ? 8 : 16);
+          if (own == (p & 15)) {
+            mine = sum;
+            mine2 = sum2;
+          }
+          if ((p & 15) == 15 || p == np - 1) {  // in double, for 16 pairs at once
+            (p < 16 ? acc0 : acc1) += (double)mine + (double)mine2;
+            mine = mine2 = 0.f;
+          }
+        }
       }
       // Z = DFT_H of (even + i odd cells); X[k] = Ze[k] + e^{-2 pi i k/N} Zo[k]
       PlanRun2x<P>::template run<false, true>(v, buf, t, tws, sync);
@@ -154,7 +186,7 @@ __global__ void __launch_bounds__(AK2<N>::THREADS, AK2<N>::MINB) k_adj_z2(const 
   }
   pdl_release();
   if (want_db) {
-    const int r = 2 * (lane & 15) + up;
+    const int r = 2 * own + up;
     if (r < a.nb) atomicAdd(&red[r], acc0);
     if (r + 32 < a.nb) atomicAdd(&red[r + 32], acc1);
     __syncthreads();
