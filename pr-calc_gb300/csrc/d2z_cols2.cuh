@@ -17,17 +17,23 @@
 namespace prc {
 
 // Tile width and resident CTAs per SM of the pair passes (plans as in CCfg).
+// Twelve elements a lane leave room for a third y CTA of 256 threads (85
+// registers): 384^3 x 24 1.98 -> 1.83 ms, 768^3 x 16 12.6 -> 11.6; a fifth window CTA
+// of 128 at 192 (x 41 0.305 -> 0.294 ms).  (Ten at 128 would gain 0.001 ms there
+// and lose 0.02 in TM_ACC.)  At 1024 shared memory holds two y CTAs whatever MINB
+// says; 85 registers took 18.1 ms for 12 radii, 128 18.5.  With sixteen elements
+// elsewhere the same only spills (512^3 x 32: y 5.44 -> 5.51, window 4.12 -> 4.27).
 template <int N> struct C2Cfg { static constexpr bool on = false; };
 template <> struct C2Cfg<32> { static constexpr bool on = true; static constexpr int T = 16, MINB = 16, TWIN = 16, MINBWIN = 16, XB = 8; };
 template <> struct C2Cfg<64> { static constexpr bool on = true; static constexpr int T = 8, MINB = 16, TWIN = 8, MINBWIN = 16, XB = 8; };
 template <> struct C2Cfg<96> { static constexpr bool on = true; static constexpr int T = 8, MINB = 8, TWIN = 8, MINBWIN = 8, XB = 8; };
 template <> struct C2Cfg<128> { static constexpr bool on = true; static constexpr int T = 8, MINB = 8, TWIN = 8, MINBWIN = 8, XB = 8; };
-template <> struct C2Cfg<192> { static constexpr bool on = true; static constexpr int T = 8, MINB = 4, TWIN = 8, MINBWIN = 4, XB = 8; };
+template <> struct C2Cfg<192> { static constexpr bool on = true; static constexpr int T = 8, MINB = 5, TWIN = 8, MINBWIN = 5, XB = 8; };
 template <> struct C2Cfg<256> { static constexpr bool on = true; static constexpr int T = 8, MINB = 4, TWIN = 8, MINBWIN = 4, XB = 8; };
-template <> struct C2Cfg<384> { static constexpr bool on = true; static constexpr int T = 8, MINB = 2, TWIN = 4, MINBWIN = 4, XB = 8; };
+template <> struct C2Cfg<384> { static constexpr bool on = true; static constexpr int T = 8, MINB = 3, TWIN = 4, MINBWIN = 4, XB = 8; };
 template <> struct C2Cfg<512> { static constexpr bool on = true; static constexpr int T = 8, MINB = 2, TWIN = 4, MINBWIN = 4, XB = 4; };
-template <> struct C2Cfg<768> { static constexpr bool on = true; static constexpr int T = 4, MINB = 2, TWIN = 4, MINBWIN = 2, XB = 4; };
-template <> struct C2Cfg<1024> { static constexpr bool on = true; static constexpr int T = 4, MINB = 2, TWIN = 8, MINBWIN = 1, XB = 4; };
+template <> struct C2Cfg<768> { static constexpr bool on = true; static constexpr int T = 4, MINB = 3, TWIN = 4, MINBWIN = 2, XB = 4; };
+template <> struct C2Cfg<1024> { static constexpr bool on = true; static constexpr int T = 4, MINB = 3, TWIN = 8, MINBWIN = 1, XB = 4; };
 
 // Layout of a pair slot's main array: blocks of XB planes ix, in a block the
 // order (iy, kz / T, ix % XB, kz % T) with T the window pass's tile width, so
