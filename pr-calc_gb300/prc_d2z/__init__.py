@@ -233,6 +233,14 @@ def _dev_ptr(x, dtype_name: str, n: int):
     return ctypes.c_void_p(x.data_ptr())
 
 
+def _dev_in(x, dtype_name: str, n: int, keep: list):
+    """Device pointer of an input's elements in order.  reshape copies a tensor
+    whose elements do not lie in order; `keep` holds the copy until the call has
+    returned (freed earlier, its memory goes to the next allocation)."""
+    keep.append(x.reshape(-1))
+    return _dev_ptr(keep[-1], dtype_name, n)
+
+
 def _host_ptr(x, dtype, n: int):
     if not isinstance(x, np.ndarray) or x.dtype != dtype or x.size != n or not x.flags.c_contiguous:
         raise ValueError(f"expected a contiguous numpy array of {n} {np.dtype(dtype).name}")
@@ -306,7 +314,8 @@ class Delta2Zreion:
         sig_p = ctypes.c_void_p(sig.ctypes.data) if sig is not None else None
         if _is_torch(delta_lin):
             import torch
-            dp = _dev_ptr(delta_lin.reshape(-1), "float32", n3)
+            keep = []
+            dp = _dev_in(delta_lin, "float32", n3, keep)
             if zreion is None:
                 zreion = torch.empty(delta_lin.shape, dtype=torch.float32, device=delta_lin.device)
             if want_argmax and argmax is None:
@@ -346,8 +355,9 @@ class Delta2Zreion:
         L = load()
         if _is_torch(delta_lin):
             import torch
+            keep = []
             out = torch.empty(delta_lin.shape, dtype=torch.float32, device=delta_lin.device)
-            check(L.prc_d2z_smooth(self._ctx, _dev_ptr(delta_lin.reshape(-1), "float32", self.n3), 1, int(radius),
+            check(L.prc_d2z_smooth(self._ctx, _dev_in(delta_lin, "float32", self.n3, keep), 1, int(radius),
                                    _dev_ptr(out.reshape(-1), "float32", self.n3), 1))
             return out
         d = np.ascontiguousarray(delta_lin, np.float32)
@@ -410,8 +420,9 @@ class Delta2Zreion:
         counts = np.zeros(PRC_NHISTORY, np.uint32)
         hist = np.zeros(PRC_NHISTORY, np.float32)
         hz = np.zeros(PRC_NHISTORY, np.float32)
+        keep = []
         if _is_torch(zreion):
-            zp, on_dev = _dev_ptr(zreion.reshape(-1), "float32", self.n3), 1
+            zp, on_dev = _dev_in(zreion, "float32", self.n3, keep), 1
         else:
             z = np.ascontiguousarray(zreion, np.float32)
             zp, on_dev = _host_ptr(z, np.float32, self.n3), 0
@@ -460,8 +471,9 @@ class Delta2Zreion:
         dBp = ctypes.c_void_p(dB.ctypes.data) if dB is not None else None
         if _is_torch(dL_dz):
             import torch
-            gp = _dev_ptr(dL_dz.reshape(-1), "float32", self.n3)
-            ap = _dev_ptr(argmax.reshape(-1), "uint8", self.n3)
+            keep = []
+            gp = _dev_in(dL_dz, "float32", self.n3, keep)
+            ap = _dev_in(argmax, "uint8", self.n3, keep)
             if dL_ddelta is None:
                 dL_ddelta = torch.empty(dL_dz.shape, dtype=torch.float32, device=dL_dz.device)
             op = _dev_ptr(dL_ddelta.reshape(-1), "float32", self.n3)
@@ -519,7 +531,8 @@ class Batch:
         m = self.MODES[mode] if mode is not None else (_lib.PRC_BATCH_GRAPH if use_graph else _lib.PRC_BATCH_LOOP)
         L = load()
         n = self.n
-        dp = (ctypes.c_void_p * n)(*[_dev_ptr(d.reshape(-1), "float32", self.N[i] ** 3).value
+        keep = []
+        dp = (ctypes.c_void_p * n)(*[_dev_in(d, "float32", self.N[i] ** 3, keep).value
                                     for i, d in enumerate(deltas)])
         zp = (ctypes.c_void_p * n)(*[_dev_ptr(z.reshape(-1), "float32", self.N[i] ** 3).value
                                     for i, z in enumerate(zreions)])
