@@ -241,6 +241,26 @@ def _dev_in(x, dtype_name: str, n: int, keep: list):
     return _dev_ptr(keep[-1], dtype_name, n)
 
 
+class _Out:
+    """Output tensors of a call.  One whose elements do not lie in order is
+    written through a copy (which holds its elements, for calls that work in
+    place); done(), after the call, puts the results into the tensors."""
+
+    def __init__(self):
+        self.copies = []
+
+    def ptr(self, x, dtype_name: str, n: int):
+        flat = x.reshape(-1)
+        p = _dev_ptr(flat, dtype_name, n)
+        if not x.is_contiguous():
+            self.copies.append((x, flat))
+        return p
+
+    def done(self):
+        for x, flat in self.copies:
+            x.detach().copy_(flat.detach().view(x.shape))
+
+
 def _host_ptr(x, dtype, n: int):
     if not isinstance(x, np.ndarray) or x.dtype != dtype or x.size != n or not x.flags.c_contiguous:
         raise ValueError(f"expected a contiguous numpy array of {n} {np.dtype(dtype).name}")
@@ -320,9 +340,11 @@ class Delta2Zreion:
                 zreion = torch.empty(delta_lin.shape, dtype=torch.float32, device=delta_lin.device)
             if want_argmax and argmax is None:
                 argmax = torch.empty(delta_lin.shape, dtype=torch.uint8, device=delta_lin.device)
-            zp = _dev_ptr(zreion.reshape(-1), "float32", n3)
-            ap = _dev_ptr(argmax.reshape(-1), "uint8", n3) if argmax is not None else None
+            out = _Out()
+            zp = out.ptr(zreion, "float32", n3)
+            ap = out.ptr(argmax, "uint8", n3) if argmax is not None else None
             check(L.prc_d2z_forward(self._ctx, dp, 1, zp, ap, 1, sig_p))
+            out.done()
         else:
             d = np.ascontiguousarray(delta_lin, np.float32)
             dp = _host_ptr(d, np.float32, n3)
@@ -373,8 +395,10 @@ class Delta2Zreion:
         a = np.ascontiguousarray(amp, np.float32)
         L = load()
         if out is not None and _is_torch(out):
+            o = _Out()
             check(L.prc_d2z_gaussian_field(self._ctx, int(seed) & 0xFFFFFFFF, a.ctypes.data, len(a),
-                                           _dev_ptr(out.reshape(-1), "float32", self.n3), 1))
+                                           o.ptr(out, "float32", self.n3), 1))
+            o.done()
             return out
         res = np.empty((self.N,) * 3, np.float32) if out is None else out
         check(L.prc_d2z_gaussian_field(self._ctx, int(seed) & 0xFFFFFFFF, a.ctypes.data, len(a),
@@ -448,7 +472,9 @@ class Delta2Zreion:
         """CorrectHistory's per-cell map, in place (host array or CUDA tensor)."""
         zv = np.ascontiguousarray(zvz, np.float32)
         if _is_torch(zreion):
-            check(load().prc_d2z_correct(self._ctx, zv.ctypes.data, _dev_ptr(zreion.reshape(-1), "float32", self.n3), 1))
+            out = _Out()
+            check(load().prc_d2z_correct(self._ctx, zv.ctypes.data, out.ptr(zreion, "float32", self.n3), 1))
+            out.done()
         else:
             check(load().prc_d2z_correct(self._ctx, zv.ctypes.data, _host_ptr(zreion, np.float32, self.n3), 0))
         return zreion
@@ -476,8 +502,10 @@ class Delta2Zreion:
             ap = _dev_in(argmax, "uint8", self.n3, keep)
             if dL_ddelta is None:
                 dL_ddelta = torch.empty(dL_dz.shape, dtype=torch.float32, device=dL_dz.device)
-            op = _dev_ptr(dL_ddelta.reshape(-1), "float32", self.n3)
+            out = _Out()
+            op = out.ptr(dL_ddelta, "float32", self.n3)
             check(L.prc_d2z_backward(self._ctx, gp, ap, 1, op, 1, dBp))
+            out.done()
         else:
             g = np.ascontiguousarray(dL_dz, np.float32)
             a = np.ascontiguousarray(argmax, np.uint8)
@@ -534,13 +562,13 @@ class Batch:
         keep = []
         dp = (ctypes.c_void_p * n)(*[_dev_in(d, "float32", self.N[i] ** 3, keep).value
                                     for i, d in enumerate(deltas)])
-        zp = (ctypes.c_void_p * n)(*[_dev_ptr(z.reshape(-1), "float32", self.N[i] ** 3).value
-                                    for i, z in enumerate(zreions)])
+        out = _Out()
+        zp = (ctypes.c_void_p * n)(*[out.ptr(z, "float32", self.N[i] ** 3).value for i, z in enumerate(zreions)])
         ap = None
         if argmaxes is not None:
-            ap = (ctypes.c_void_p * n)(*[_dev_ptr(a.reshape(-1), "uint8", self.N[i] ** 3).value
-                                        for i, a in enumerate(argmaxes)])
+            ap = (ctypes.c_void_p * n)(*[out.ptr(a, "uint8", self.N[i] ** 3).value for i, a in enumerate(argmaxes)])
         check(L.prc_d2z_batch_forward(self._b, dp, zp, ap, m))
+        out.done()
         return zreions
 
     def launches(self) -> int:

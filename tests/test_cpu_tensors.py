@@ -40,6 +40,20 @@ class _Library:
     def __init__(self):
         self.seen = []
 
+    def prc_d2z_forward(self, ctx, d, in_dev, z, am, out_dev, sig):
+        _write(z, np.arange(N ** 3))
+        if am is not None:
+            _write(am, np.arange(N ** 3) % 7, np.uint8)
+        return 0
+
+    def prc_d2z_correct(self, ctx, zvz, z, on_dev):
+        _write(z, _read(z) + 1)
+        return 0
+
+    def prc_d2z_gaussian_field(self, ctx, seed, amp, n, z, on_dev):
+        _write(z, np.arange(N ** 3) + 5)
+        return 0
+
     def prc_d2z_backward(self, ctx, g, am, in_dev, out, out_dev, db):
         self.seen += [_read(g), _read(am, np.uint8)]
         _write(out, 4)
@@ -47,6 +61,8 @@ class _Library:
 
     def prc_d2z_batch_forward(self, b, dp, zp, ap, mode):
         self.seen += [_read(p) for p in dp]
+        for i, p in enumerate(zp):
+            _write(p, np.arange(N ** 3) + i)
         return 0
 
 
@@ -86,3 +102,39 @@ def test_copies_of_unordered_inputs_live_until_the_call(lib):
     _engine().backward(g, am, dL_ddelta=_dev(torch.zeros(N, N, N)))
     assert np.array_equal(lib.seen[0], g.numpy().ravel())
     assert np.array_equal(lib.seen[1], am.numpy().ravel())
+
+
+def test_unordered_outputs_get_the_results(lib):
+    """A transposed output tensor holds the result afterwards (reshape gives the
+    library a copy of it), in its own element order."""
+    count = np.arange(N ** 3, dtype=np.float32).reshape(N, N, N)
+    flat = lambda: _dev(torch.zeros(N, N, N))  # noqa: E731
+    e = _engine()
+    z, am = _transposed(1), _transposed(2, torch.uint8)
+    r = e.forward(flat(), zreion=z, argmax=am)
+    assert r[0] is z and np.array_equal(z.numpy(), count)
+    assert np.array_equal(am.numpy(), count % 7)
+    z = _transposed(3)
+    before = z.numpy().copy()
+    e.correct(z, np.zeros(4, np.float32))
+    assert np.array_equal(z.numpy(), before + 1)
+    z = _transposed(4)
+    e.gaussian_field(1, np.zeros(4, np.float32), out=z)
+    assert np.array_equal(z.numpy(), count + 5)
+    z = _transposed(5)
+    e.backward(flat(), _dev(torch.zeros(N, N, N, dtype=torch.uint8)), dL_ddelta=z)
+    assert np.array_equal(z.numpy(), np.full_like(count, 4))
+    zs = [_transposed(6), flat(), _transposed(7)]
+    _batch(3).forward([flat() for _ in zs], zs, mode="loop")
+    for i, z in enumerate(zs):
+        assert np.array_equal(z.numpy(), count + i)
+
+
+def test_what_was_refused_stays_refused(lib):
+    """Strided vectors, wrong types and counts, tensors in host memory."""
+    e, ok = _engine(), _dev(torch.zeros(N, N, N))
+    for bad in (_dev(torch.zeros(2 * N ** 3))[::2], _dev(torch.zeros(N ** 3, dtype=torch.float64)),
+                _dev(torch.zeros(N, N, N - 1)), torch.zeros(N, N, N)):
+        for a, b in ((bad, ok), (ok, bad)):
+            with pytest.raises(ValueError):
+                e.forward(a, zreion=b, want_argmax=False)
