@@ -263,6 +263,8 @@ int prc_d2z_last_launches(prc_d2z_ctx* ctx, int* n);
  * Many independent boxes (realisations), possibly of different grid sizes,
  * one workspace per box.  delta, zreion (and argmax, nullable) are arrays of
  * n_boxes device pointers; every mode gives the same results bit for bit.
+ * The batch runs on streams of its own, which wait for no other stream: the
+ * inputs are complete before the call (prc_d2z.Batch waits for torch's stream).
  * Modes of prc_d2z_batch_forward:
  *   PRC_BATCH_LOOP     each box's launches, boxes spread over n_streams streams;
  *   PRC_BATCH_GRAPH    the same launches captured once into a CUDA graph and

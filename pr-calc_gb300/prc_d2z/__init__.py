@@ -233,6 +233,16 @@ def _dev_ptr(x, dtype_name: str, n: int):
     return ctypes.c_void_p(x.data_ptr())
 
 
+def _after_torch(x, stream: int) -> None:
+    """The library's kernels run on `stream`, torch's (which fill x, or copied
+    it) on torch's current stream: another stream's work is waited for here.
+    (The calls return with their own work finished.)"""
+    import torch
+    s = torch.cuda.current_stream(x.device)
+    if s.cuda_stream != stream:
+        s.synchronize()
+
+
 def _dev_in(x, dtype_name: str, n: int, keep: list):
     """Device pointer of an input's elements in order.  reshape copies a tensor
     whose elements do not lie in order; `keep` holds the copy until the call has
@@ -292,7 +302,8 @@ class Delta2Zreion:
         d.radius_batch = int(radius_batch)
         d.flags = ((PRC_FLAG_ARGMAX if argmax else 0) | (PRC_FLAG_SIGMA_GRID if sigma_grid else 0)
                    | (_lib.PRC_FLAG_FAITHFUL_WINDOW if faithful_window else 0))
-        d.stream = ctypes.c_void_p(int(stream)) if stream is not None else None
+        self._stream = int(stream) if stream is not None else 0
+        d.stream = ctypes.c_void_p(self._stream)
         self._ctx = ctypes.c_void_p()
         check(L.prc_d2z_create(ctypes.byref(d), ctypes.byref(self._ctx)))
 
@@ -343,6 +354,7 @@ class Delta2Zreion:
             out = _Out()
             zp = out.ptr(zreion, "float32", n3)
             ap = out.ptr(argmax, "uint8", n3) if argmax is not None else None
+            _after_torch(delta_lin, self._stream)
             check(L.prc_d2z_forward(self._ctx, dp, 1, zp, ap, 1, sig_p))
             out.done()
         else:
@@ -379,7 +391,9 @@ class Delta2Zreion:
             import torch
             keep = []
             out = torch.empty(delta_lin.shape, dtype=torch.float32, device=delta_lin.device)
-            check(L.prc_d2z_smooth(self._ctx, _dev_in(delta_lin, "float32", self.n3, keep), 1, int(radius),
+            dp = _dev_in(delta_lin, "float32", self.n3, keep)
+            _after_torch(delta_lin, self._stream)
+            check(L.prc_d2z_smooth(self._ctx, dp, 1, int(radius),
                                    _dev_ptr(out.reshape(-1), "float32", self.n3), 1))
             return out
         d = np.ascontiguousarray(delta_lin, np.float32)
@@ -396,8 +410,9 @@ class Delta2Zreion:
         L = load()
         if out is not None and _is_torch(out):
             o = _Out()
-            check(L.prc_d2z_gaussian_field(self._ctx, int(seed) & 0xFFFFFFFF, a.ctypes.data, len(a),
-                                           o.ptr(out, "float32", self.n3), 1))
+            op = o.ptr(out, "float32", self.n3)
+            _after_torch(out, self._stream)
+            check(L.prc_d2z_gaussian_field(self._ctx, int(seed) & 0xFFFFFFFF, a.ctypes.data, len(a), op, 1))
             o.done()
             return out
         res = np.empty((self.N,) * 3, np.float32) if out is None else out
@@ -447,6 +462,7 @@ class Delta2Zreion:
         keep = []
         if _is_torch(zreion):
             zp, on_dev = _dev_in(zreion, "float32", self.n3, keep), 1
+            _after_torch(zreion, self._stream)
         else:
             z = np.ascontiguousarray(zreion, np.float32)
             zp, on_dev = _host_ptr(z, np.float32, self.n3), 0
@@ -473,7 +489,9 @@ class Delta2Zreion:
         zv = np.ascontiguousarray(zvz, np.float32)
         if _is_torch(zreion):
             out = _Out()
-            check(load().prc_d2z_correct(self._ctx, zv.ctypes.data, out.ptr(zreion, "float32", self.n3), 1))
+            zp = out.ptr(zreion, "float32", self.n3)
+            _after_torch(zreion, self._stream)
+            check(load().prc_d2z_correct(self._ctx, zv.ctypes.data, zp, 1))
             out.done()
         else:
             check(load().prc_d2z_correct(self._ctx, zv.ctypes.data, _host_ptr(zreion, np.float32, self.n3), 0))
@@ -504,6 +522,7 @@ class Delta2Zreion:
                 dL_ddelta = torch.empty(dL_dz.shape, dtype=torch.float32, device=dL_dz.device)
             out = _Out()
             op = out.ptr(dL_ddelta, "float32", self.n3)
+            _after_torch(dL_dz, self._stream)
             check(L.prc_d2z_backward(self._ctx, gp, ap, 1, op, 1, dBp))
             out.done()
         else:
@@ -567,6 +586,8 @@ class Batch:
         ap = None
         if argmaxes is not None:
             ap = (ctypes.c_void_p * n)(*[out.ptr(a, "uint8", self.N[i] ** 3).value for i, a in enumerate(argmaxes)])
+        if n:
+            _after_torch(deltas[0], -1)  # (the batch runs on streams of its own)
         check(L.prc_d2z_batch_forward(self._b, dp, zp, ap, m))
         out.done()
         return zreions

@@ -34,11 +34,27 @@ def _write(p, value, dtype=np.float32):
     np.frombuffer((ctypes.c_char * (N ** 3 * np.dtype(dtype).itemsize)).from_address(p), dtype)[:] = value
 
 
+class _Stream:
+    """Stands for torch's current stream."""
+
+    def __init__(self, handle):
+        self.cuda_stream, self.waits = handle, 0
+
+    def synchronize(self):
+        self.waits += 1
+
+
 class _Library:
     """Records what the pointers hold at the time of the call."""
 
     def __init__(self):
         self.seen = []
+
+    def prc_d2z_history(self, ctx, z, on_dev, counts, h, hz):
+        return 0
+
+    def prc_d2z_smooth(self, ctx, d, in_dev, radius, out, out_dev):
+        return 0
 
     def prc_d2z_forward(self, ctx, d, in_dev, z, am, out_dev, sig):
         _write(z, np.arange(N ** 3))
@@ -70,12 +86,14 @@ class _Library:
 def lib(monkeypatch):
     L = _Library()
     monkeypatch.setattr(prc_d2z, "load", lambda: L)
+    L.stream = _Stream(0)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: L.stream)
     return L
 
 
-def _engine():
+def _engine(stream=0):
     e = object.__new__(prc_d2z.Delta2Zreion)
-    e.n3, e.n_radii, e._ctx = N ** 3, 3, None
+    e.N, e.n3, e.n_radii, e._ctx, e._stream = N, N ** 3, 3, None, stream
     return e
 
 
@@ -138,3 +156,26 @@ def test_what_was_refused_stays_refused(lib):
         for a, b in ((bad, ok), (ok, bad)):
             with pytest.raises(ValueError):
                 e.forward(a, zreion=b, want_argmax=False)
+
+
+@pytest.mark.parametrize("torch_stream,ctx_stream,waits", [(0, 0, 0), (7, 7, 0), (7, 0, 1), (0, 7, 1)])
+def test_work_of_another_torch_stream_is_waited_for(lib, monkeypatch, torch_stream, ctx_stream, waits):
+    """Tensors filled on a stream that the context does not use are complete
+    before the library reads them; on the same stream nothing is waited for."""
+    lib.stream = _Stream(torch_stream)
+    e, x = _engine(ctx_stream), _dev(torch.zeros(N, N, N))
+    am, tab = _dev(torch.zeros(N, N, N, dtype=torch.uint8)), np.zeros(4, np.float32)
+    monkeypatch.setattr(torch, "empty", lambda *a, **k: x)
+    calls = [lambda: e.forward(x, zreion=x, argmax=am), lambda: e.backward(x, am, dL_ddelta=x),
+             lambda: e.smooth(x, 0), lambda: e.history(x), lambda: e.correct(x, tab),
+             lambda: e.gaussian_field(1, tab, out=x)]
+    for k, call in enumerate(calls):
+        call()
+        assert lib.stream.waits == (k + 1) * waits, k
+
+
+def test_a_batch_waits_for_torch(lib):
+    """A batch's streams are its own: torch's work is always waited for."""
+    x = _dev(torch.zeros(N, N, N))
+    _batch(2).forward([x, x], [_dev(torch.zeros(N, N, N)) for _ in range(2)], mode="loop")
+    assert lib.stream.waits == 1
