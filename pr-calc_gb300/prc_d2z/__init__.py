@@ -223,14 +223,16 @@ def _is_torch(x) -> bool:
     return type(x).__module__.startswith("torch")
 
 
-def _dev_ptr(x, dtype_name: str, n: int):
+# A small box's whole step takes some tens of microseconds, so the checks of a
+# tensor look at the tensor itself: no view of it, no text of its type.
+def _dev_ptr(x, dtype, n: int) -> int:
     if not x.is_cuda:
         raise ValueError("torch tensors passed to prc_d2z must live on a CUDA device")
     if not x.is_contiguous():
         raise ValueError("tensor must be contiguous")
-    if str(x.dtype) != f"torch.{dtype_name}" or x.numel() != n:
-        raise ValueError(f"expected {n} elements of {dtype_name}, got {x.numel()} of {x.dtype}")
-    return ctypes.c_void_p(x.data_ptr())
+    if x.dtype != dtype or x.numel() != n:
+        raise ValueError(f"expected {n} elements of {dtype}, got {x.numel()} of {x.dtype}")
+    return x.data_ptr()
 
 
 def _after_torch(x, stream: int) -> None:
@@ -238,37 +240,37 @@ def _after_torch(x, stream: int) -> None:
     it) on torch's current stream: another stream's work is waited for here.
     (The calls return with their own work finished.)"""
     import torch
-    s = torch.cuda.current_stream(x.device)
-    if s.cuda_stream != stream:
-        s.synchronize()
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)  # (without the Stream object, where there is one)
+    if raw is None or raw(x.get_device()) != stream:
+        s = torch.cuda.current_stream(x.device)
+        if s.cuda_stream != stream:
+            s.synchronize()
 
 
-def _dev_in(x, dtype_name: str, n: int, keep: list):
+def _dev_in(x, dtype, n: int, copies: list) -> int:
     """Device pointer of an input's elements in order.  reshape copies a tensor
-    whose elements do not lie in order; `keep` holds the copy until the call has
-    returned (freed earlier, its memory goes to the next allocation)."""
-    keep.append(x.reshape(-1))
-    return _dev_ptr(keep[-1], dtype_name, n)
+    whose elements do not lie in order; `copies` holds the copy until the call
+    has returned (freed earlier, its memory goes to the next allocation)."""
+    if not x.is_contiguous():
+        x = x.reshape(-1)
+        copies.append(x)
+    return _dev_ptr(x, dtype, n)
 
 
-class _Out:
-    """Output tensors of a call.  One whose elements do not lie in order is
-    written through a copy (which holds its elements, for calls that work in
-    place); done(), after the call, puts the results into the tensors."""
+def _dev_out(x, dtype, n: int, outs: list) -> int:
+    """The same of an output.  One whose elements do not lie in order is written
+    through a copy (which holds its elements, for calls that work in place);
+    _put_back(outs), after the call, puts the results into the tensors."""
+    if x.is_contiguous():
+        return _dev_ptr(x, dtype, n)
+    flat = x.reshape(-1)
+    outs.append((x, flat))
+    return _dev_ptr(flat, dtype, n)
 
-    def __init__(self):
-        self.copies = []
 
-    def ptr(self, x, dtype_name: str, n: int):
-        flat = x.reshape(-1)
-        p = _dev_ptr(flat, dtype_name, n)
-        if not x.is_contiguous():
-            self.copies.append((x, flat))
-        return p
-
-    def done(self):
-        for x, flat in self.copies:
-            x.detach().copy_(flat.detach().view(x.shape))
+def _put_back(outs: list) -> None:
+    for x, flat in outs:
+        x.detach().copy_(flat.detach().view(x.shape))
 
 
 def _host_ptr(x, dtype, n: int):
@@ -345,18 +347,18 @@ class Delta2Zreion:
         sig_p = ctypes.c_void_p(sig.ctypes.data) if sig is not None else None
         if _is_torch(delta_lin):
             import torch
-            keep = []
-            dp = _dev_in(delta_lin, "float32", n3, keep)
+            copies = []
+            dp = _dev_in(delta_lin, torch.float32, n3, copies)
             if zreion is None:
                 zreion = torch.empty(delta_lin.shape, dtype=torch.float32, device=delta_lin.device)
             if want_argmax and argmax is None:
                 argmax = torch.empty(delta_lin.shape, dtype=torch.uint8, device=delta_lin.device)
-            out = _Out()
-            zp = out.ptr(zreion, "float32", n3)
-            ap = out.ptr(argmax, "uint8", n3) if argmax is not None else None
+            outs = []
+            zp = _dev_out(zreion, torch.float32, n3, outs)
+            ap = _dev_out(argmax, torch.uint8, n3, outs) if argmax is not None else None
             _after_torch(delta_lin, self._stream)
             check(L.prc_d2z_forward(self._ctx, dp, 1, zp, ap, 1, sig_p))
-            out.done()
+            _put_back(outs)
         else:
             d = np.ascontiguousarray(delta_lin, np.float32)
             dp = _host_ptr(d, np.float32, n3)
@@ -389,12 +391,12 @@ class Delta2Zreion:
         L = load()
         if _is_torch(delta_lin):
             import torch
-            keep = []
+            copies = []
             out = torch.empty(delta_lin.shape, dtype=torch.float32, device=delta_lin.device)
-            dp = _dev_in(delta_lin, "float32", self.n3, keep)
+            dp = _dev_in(delta_lin, torch.float32, self.n3, copies)
             _after_torch(delta_lin, self._stream)
             check(L.prc_d2z_smooth(self._ctx, dp, 1, int(radius),
-                                   _dev_ptr(out.reshape(-1), "float32", self.n3), 1))
+                                   _dev_ptr(out, torch.float32, self.n3), 1))
             return out
         d = np.ascontiguousarray(delta_lin, np.float32)
         out = np.empty(d.shape, np.float32)
@@ -409,11 +411,12 @@ class Delta2Zreion:
         a = np.ascontiguousarray(amp, np.float32)
         L = load()
         if out is not None and _is_torch(out):
-            o = _Out()
-            op = o.ptr(out, "float32", self.n3)
+            import torch
+            outs = []
+            op = _dev_out(out, torch.float32, self.n3, outs)
             _after_torch(out, self._stream)
             check(L.prc_d2z_gaussian_field(self._ctx, int(seed) & 0xFFFFFFFF, a.ctypes.data, len(a), op, 1))
-            o.done()
+            _put_back(outs)
             return out
         res = np.empty((self.N,) * 3, np.float32) if out is None else out
         check(L.prc_d2z_gaussian_field(self._ctx, int(seed) & 0xFFFFFFFF, a.ctypes.data, len(a),
@@ -459,9 +462,10 @@ class Delta2Zreion:
         counts = np.zeros(PRC_NHISTORY, np.uint32)
         hist = np.zeros(PRC_NHISTORY, np.float32)
         hz = np.zeros(PRC_NHISTORY, np.float32)
-        keep = []
+        copies = []
         if _is_torch(zreion):
-            zp, on_dev = _dev_in(zreion, "float32", self.n3, keep), 1
+            import torch
+            zp, on_dev = _dev_in(zreion, torch.float32, self.n3, copies), 1
             _after_torch(zreion, self._stream)
         else:
             z = np.ascontiguousarray(zreion, np.float32)
@@ -488,11 +492,12 @@ class Delta2Zreion:
         """CorrectHistory's per-cell map, in place (host array or CUDA tensor)."""
         zv = np.ascontiguousarray(zvz, np.float32)
         if _is_torch(zreion):
-            out = _Out()
-            zp = out.ptr(zreion, "float32", self.n3)
+            import torch
+            outs = []
+            zp = _dev_out(zreion, torch.float32, self.n3, outs)
             _after_torch(zreion, self._stream)
             check(load().prc_d2z_correct(self._ctx, zv.ctypes.data, zp, 1))
-            out.done()
+            _put_back(outs)
         else:
             check(load().prc_d2z_correct(self._ctx, zv.ctypes.data, _host_ptr(zreion, np.float32, self.n3), 0))
         return zreion
@@ -515,16 +520,16 @@ class Delta2Zreion:
         dBp = ctypes.c_void_p(dB.ctypes.data) if dB is not None else None
         if _is_torch(dL_dz):
             import torch
-            keep = []
-            gp = _dev_in(dL_dz, "float32", self.n3, keep)
-            ap = _dev_in(argmax, "uint8", self.n3, keep)
+            copies = []
+            gp = _dev_in(dL_dz, torch.float32, self.n3, copies)
+            ap = _dev_in(argmax, torch.uint8, self.n3, copies)
             if dL_ddelta is None:
                 dL_ddelta = torch.empty(dL_dz.shape, dtype=torch.float32, device=dL_dz.device)
-            out = _Out()
-            op = out.ptr(dL_ddelta, "float32", self.n3)
+            outs = []
+            op = _dev_out(dL_ddelta, torch.float32, self.n3, outs)
             _after_torch(dL_dz, self._stream)
             check(L.prc_d2z_backward(self._ctx, gp, ap, 1, op, 1, dBp))
-            out.done()
+            _put_back(outs)
         else:
             g = np.ascontiguousarray(dL_dz, np.float32)
             a = np.ascontiguousarray(argmax, np.uint8)
@@ -575,21 +580,22 @@ class Batch:
     def forward(self, deltas, zreions, argmaxes=None, use_graph: bool = True, mode: str | None = None):
         """deltas/zreions (/argmaxes): lists of contiguous CUDA tensors.  mode:
         "loop", "graph" or "grouped" (default: "graph" if use_graph else "loop")."""
+        import torch
         m = self.MODES[mode] if mode is not None else (_lib.PRC_BATCH_GRAPH if use_graph else _lib.PRC_BATCH_LOOP)
         L = load()
         n = self.n
-        keep = []
-        dp = (ctypes.c_void_p * n)(*[_dev_in(d, "float32", self.N[i] ** 3, keep).value
+        copies = []
+        dp = (ctypes.c_void_p * n)(*[_dev_in(d, torch.float32, self.N[i] ** 3, copies)
                                     for i, d in enumerate(deltas)])
-        out = _Out()
-        zp = (ctypes.c_void_p * n)(*[out.ptr(z, "float32", self.N[i] ** 3).value for i, z in enumerate(zreions)])
+        outs = []
+        zp = (ctypes.c_void_p * n)(*[_dev_out(z, torch.float32, self.N[i] ** 3, outs) for i, z in enumerate(zreions)])
         ap = None
         if argmaxes is not None:
-            ap = (ctypes.c_void_p * n)(*[out.ptr(a, "uint8", self.N[i] ** 3).value for i, a in enumerate(argmaxes)])
+            ap = (ctypes.c_void_p * n)(*[_dev_out(a, torch.uint8, self.N[i] ** 3, outs) for i, a in enumerate(argmaxes)])
         if n:
             _after_torch(deltas[0], -1)  # (the batch runs on streams of its own)
         check(L.prc_d2z_batch_forward(self._b, dp, zp, ap, m))
-        out.done()
+        _put_back(outs)
         return zreions
 
     def launches(self) -> int:

@@ -88,6 +88,7 @@ def lib(monkeypatch):
     monkeypatch.setattr(prc_d2z, "load", lambda: L)
     L.stream = _Stream(0)
     monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: L.stream)
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda device: L.stream.cuda_stream, raising=False)
     return L
 
 
