@@ -108,10 +108,18 @@ typedef struct {
   const double* barrier_b;        /* n_radii barrier offsets B_r (NaN: radius never wins) */
   double        barrier_a;        /* A in z = A*(delta_R + B_r) - 1             */
   double        growth_init;      /* D(zInit); delta_lin is divided by it (main_d2z.C:59) */
-  int           radius_batch;     /* radii per sweep, <= 64; 0 = what 1 GB of slots holds, at least 16 (8 for N >= 1024) */
+  int           radius_batch;     /* radii per sweep, <= 64; 0 = default (below)         */
   int           flags;            /* PRC_FLAG_*                                 */
   void*         stream;           /* cudaStream_t; NULL = default stream        */
 } prc_d2z_desc;
+
+/* Device memory of a context: radius_batch slots of N^2 (N/2 + 2) * 8 bytes, the
+ * spectrum (one slot more) and small tables.  The default radius batch is 16 (8
+ * for N >= 1024), or more, up to what 1 GB of slots holds, while a reserve lasts:
+ * all contexts and batches of the process together hold at most 6 GB a device
+ * beyond the slots named here (an odd batch's extra slot comes out of it too).
+ * A batch's boxes all get their share of it or none does.  zreion does not depend on the
+ * radius batch; sigma_grid and the adjoint do in their rounding. */
 
 /* Tuning knobs (no counterpart in the reference, whose FFTW plans are
  * chosen by FFTW).  prc_d2z_win_variants: how many window-pass variants (tile

@@ -15,6 +15,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <functional>
 #include <vector>
 
 #include "../../include/prc_d2z.h"
@@ -202,6 +203,7 @@ struct prc_d2z_ctx {
   int N = 0, H = 0, nr = 0, B = 0, flags = 0, dev = 0, sms = 0;
   int win_var = 0;   // window-pass variant (prc_d2z_tune)
   int slots_b = 0;   // radius slots allocated (one more than B for an odd B of paired sweeps)
+  long long spare = 0;  // bytes of them taken from the reserve (SlotPlan)
   int waves = 1;     // CTA waves of the window and z passes (batches: kBatchWaves)
   long long NN = 0, slot_f2 = 0;
   double box = 0, A = 0, dinit = 1;
@@ -319,33 +321,6 @@ template <class T> int dalloc(T** p, size_t count, const char* what) {
   return PRC_OK;
 }
 
-void free_all(prc_d2z_ctx* c) {
-  cudaFree(c->spec);
-  cudaFree(c->slots);
-  cudaFree(c->tw);
-  cudaFree(c->zre);
-  cudaFree(c->am);
-  cudaFree(c->sig);
-  cudaFree(c->dB);
-  cudaFree(c->counts);
-  cudaFree(c->gstage);
-  cudaFree(c->amstage);
-  cudaFree(c->grf_amp);
-  if (c->err_h) cudaFreeHost(c->err_h);
-  for (auto& e : c->ev)
-    if (e) cudaEventDestroy(e);
-  for (int k = 0; k < 2; ++k) {
-    cudaFree(c->m_delta[k]);
-    cudaFree(c->m_z[k]);
-    cudaFree(c->m_am[k]);
-    if (c->m_copy[k]) cudaStreamDestroy(c->m_copy[k]);
-    for (cudaEvent_t e : {c->m_in[k], c->m_read[k], c->m_done[k], c->m_out[k]})
-      if (e) cudaEventDestroy(e);
-  }
-  for (auto& e : c->pev) cudaEventDestroy(e);
-  c->pev.clear();
-}
-
 // Radii per sweep.  Sweeps on pairs of radii (fft2.cuh) take an even number:
 // an odd radius batch is rounded up, or down when the extra slot could not be
 // allocated.  The pair kernels are left for the single-radius ones by the
@@ -377,16 +352,99 @@ bool in_pairs(const prc_d2z_ctx* c, int nb, bool adjoint) {
   return nb % 2 == 0 || nb >= (N == 256 ? 11 : 7);
 }
 
-// Radius slots for a radius batch of B into *out: with one more for an odd
-// batch of a size with pair kernels, if that can be had.
-int alloc_slots(const prc_d2z_ctx* c, int B, float2** out, int* n) {
-  if (c->ksl.pair && c->nr > 1 && B % 2 == 1) {
-    *n = B + 1;
-    if (cudaMalloc((void**)out, (size_t)c->slot_f2 * *n * sizeof(float2)) == cudaSuccess) return PRC_OK;
-    cudaGetLastError();
+// Radius slots beyond those that a context cannot do without (the radius batch
+// it was given, or the smallest default) come out of a reserve of kReserveBytes a
+// device that all contexts of the process share: however many contexts and
+// batches there are, they hold at most that much more together.  6 GB is 2% of
+// the device: ten default contexts of 192^3 x 64 at full width, or one slot of
+// 1024^3.
+constexpr long long kReserveBytes = 6ll << 30;
+constexpr int kReserveDevices = 64;
+std::atomic<long long> g_reserve[kReserveDevices];  // bytes taken
+
+bool reserve_take(int dev, long long bytes) {
+  if (bytes <= 0) return true;
+  if (dev < 0 || dev >= kReserveDevices) return false;
+  long long held = g_reserve[dev].load();
+  do {
+    if (held + bytes > kReserveBytes) return false;
+  } while (!g_reserve[dev].compare_exchange_weak(held, held + bytes));
+  return true;
+}
+void reserve_give(int dev, long long bytes) {
+  if (bytes > 0) g_reserve[dev].fetch_sub(bytes);
+}
+
+// What a context takes beyond its need: nothing, the odd batch's slot, or that
+// and the full default width.
+enum Spare { kLean = 0, kOdd = 1, kFull = 2 };
+
+struct SlotPlan {
+  int B;            // radii per sweep
+  int n;            // slots
+  long long spare;  // bytes of them out of the reserve
+};
+
+// Default radii per sweep: as many as 1 GB of slots holds, at least 16 (8 at
+// 1024^3, where one slot is 4.3 GB).  More radii per sweep are fewer launches
+// and fewer re-reads of the spectrum and of zreion: 64^3 x 64 radii in one
+// sweep instead of four, 122 -> 92 us; 192^3 x 41 1127 -> 1087.  Without reserve
+// the default is those 16 (8).
+SlotPlan slot_plan(const KernelSet& ks, int nr, int radius_batch, Spare level) {
+  const long long bytes = (long long)ks.N * ks.N * (ks.N / 2 + 2) * sizeof(float2);
+  const int b_min = ks.N >= 1024 ? 8 : 16;
+  const int need = std::min(radius_batch ? radius_batch : b_min, nr);
+  SlotPlan p;
+  p.B = need;
+  if (!radius_batch && level == kFull)
+    p.B = std::min(nr, std::max(b_min, (int)std::min<long long>(kMaxBatch, (1ll << 30) / bytes)));
+  p.n = p.B;
+  if (level >= kOdd && ks.pair && nr > 1 && p.B % 2 == 1) p.n = p.B + 1;
+  p.spare = (p.n - need) * bytes;
+  return p;
+}
+
+// The plan's slots into *out.  PRC_ERR_ALLOC without a message: try a smaller
+// plan (there is no reserve, or no memory, for this one).
+int alloc_slots(const prc_d2z_ctx* c, const SlotPlan& p, float2** out) {
+  *out = nullptr;
+  if (!reserve_take(c->dev, p.spare)) return PRC_ERR_ALLOC;
+  const size_t count = (size_t)c->slot_f2 * p.n;
+  if (p.spare == 0) return dalloc(out, count, "radius slots");
+  if (cudaMalloc((void**)out, count * sizeof(float2)) == cudaSuccess) return PRC_OK;
+  *out = nullptr;
+  cudaGetLastError();
+  reserve_give(c->dev, p.spare);
+  return PRC_ERR_ALLOC;
+}
+
+void free_all(prc_d2z_ctx* c) {
+  cudaFree(c->spec);
+  cudaFree(c->slots);
+  reserve_give(c->dev, c->spare);
+  c->spare = 0;
+  cudaFree(c->tw);
+  cudaFree(c->zre);
+  cudaFree(c->am);
+  cudaFree(c->sig);
+  cudaFree(c->dB);
+  cudaFree(c->counts);
+  cudaFree(c->gstage);
+  cudaFree(c->amstage);
+  cudaFree(c->grf_amp);
+  if (c->err_h) cudaFreeHost(c->err_h);
+  for (auto& e : c->ev)
+    if (e) cudaEventDestroy(e);
+  for (int k = 0; k < 2; ++k) {
+    cudaFree(c->m_delta[k]);
+    cudaFree(c->m_z[k]);
+    cudaFree(c->m_am[k]);
+    if (c->m_copy[k]) cudaStreamDestroy(c->m_copy[k]);
+    for (cudaEvent_t e : {c->m_in[k], c->m_read[k], c->m_done[k], c->m_out[k]})
+      if (e) cudaEventDestroy(e);
   }
-  *n = B;
-  return dalloc(out, (size_t)c->slot_f2 * B, "radius slots");
+  for (auto& e : c->pev) cudaEventDestroy(e);
+  c->pev.clear();
 }
 
 // main-array segment of a column pass along x (rows ix) or y (rows iy)
@@ -884,7 +942,9 @@ int prc_d2z_test_withhold_copy(int calls) {
   return PRC_OK;
 }
 
-int prc_d2z_create(const prc_d2z_desc* d, prc_d2z_ctx** out) {
+namespace {
+// prc_d2z_create at one level of slots.
+int create_at(const prc_d2z_desc* d, Spare level, prc_d2z_ctx** out) {
   if (!d || !out) return prc_fail(PRC_ERR_INVALID, "prc_d2z_create: null argument");
   *out = nullptr;
   const KernelSet* ks = kernel_set(d->N);
@@ -913,16 +973,6 @@ int prc_d2z_create(const prc_d2z_desc* d, prc_d2z_ctx** out) {
   c->st = (cudaStream_t)d->stream;
   c->ks = ks;
   c->ksl = *ks;
-  // Default radii per sweep: as many as 1 GB of slots holds, at least 16 (8 at
-  // 1024^3, where one slot is 4.3 GB).  More radii per sweep are fewer launches
-  // and fewer re-reads of the spectrum and of zreion: 64^3 x 64 radii in one
-  // sweep instead of four, 122 -> 92 us; 192^3 x 41 1127 -> 1087.
-  const int b_min = d->N >= 1024 ? 8 : 16;
-  const int b_fit = (int)std::min<long long>(kMaxBatch, (1ll << 30) / (c->slot_f2 * (long long)sizeof(float2)));
-  int B = d->radius_batch ? d->radius_batch : std::max(b_min, b_fit);
-  if (B > c->nr) B = c->nr;
-  c->B = B;
-  c->slots_b = B;
   const double dk = 2.0 * M_PI / d->box_mpc;
   const double n3 = (double)d->N * d->N * d->N;
   c->as = (float)(d->barrier_a / n3);
@@ -941,12 +991,12 @@ int prc_d2z_create(const prc_d2z_desc* d, prc_d2z_ctx** out) {
     return cuda_fail(e, "prc_d2z_create: device set-up");
   }
   const long long n3l = (long long)c->NN * c->N;
+  const SlotPlan plan = slot_plan(*ks, c->nr, d->radius_batch, level);
+  c->B = plan.B;
+  c->slots_b = plan.n;
   auto slots = [&]() {
-    int s = alloc_slots(c, c->B, &c->slots, &c->slots_b);
-    if (s != PRC_OK && !d->radius_batch && c->B > b_min) {  // the default: fewer will do
-      c->B = b_min;
-      s = alloc_slots(c, c->B, &c->slots, &c->slots_b);
-    }
+    const int s = alloc_slots(c, plan, &c->slots);
+    if (s == PRC_OK) c->spare = plan.spare;
     return s;
   };
   if ((st = dalloc(&c->spec, (size_t)c->slot_f2, "spectrum")) != PRC_OK || (st = slots()) != PRC_OK ||
@@ -981,6 +1031,29 @@ int prc_d2z_create(const prc_d2z_desc* d, prc_d2z_ctx** out) {
   }
   *out = c;
   return PRC_OK;
+}
+
+// n contexts at one level of slots for all of them: the largest whose spare
+// slots the reserve and the device have room for together.
+int create_levels(const prc_d2z_desc* d, int n, const std::function<int(Spare)>& create) {
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess) cudaGetLastError();
+  for (int level = kFull; level > kLean; --level) {
+    long long spare = 0;
+    for (int i = 0; i < n; ++i)
+      if (const KernelSet* ks = kernel_set(d[i].N))
+        spare += slot_plan(*ks, d[i].n_radii, d[i].radius_batch, (Spare)level).spare;
+    if (spare <= 0 || dev < 0 || dev >= kReserveDevices || g_reserve[dev].load() + spare > kReserveBytes) continue;
+    const int st = create((Spare)level);
+    if (st != PRC_ERR_ALLOC) return st;
+  }
+  return create(kLean);
+}
+}  // namespace
+
+int prc_d2z_create(const prc_d2z_desc* d, prc_d2z_ctx** out) {
+  if (!d || !out) return create_at(d, kLean, out);
+  return create_levels(d, 1, [&](Spare level) { return create_at(d, level, out); });
 }
 
 namespace {
@@ -1527,11 +1600,17 @@ int prc_d2z_tune(prc_d2z_ctx* c, int radius_batch, int win_variant) {
     if ((st = set_device(c)) != PRC_OK) return st;
     PRC_CU(cudaStreamSynchronize(c->st), "prc_d2z_tune");
     float2* ns = nullptr;
-    int n = 0;
-    if ((st = alloc_slots(c, B, &ns, &n)) != PRC_OK) return st;
+    SlotPlan p = slot_plan(c->ksl, c->nr, B, kOdd);
+    if (p.n > B && alloc_slots(c, p, &ns) != PRC_OK) ns = nullptr;
+    if (!ns) {
+      p = slot_plan(c->ksl, c->nr, B, kLean);
+      if ((st = alloc_slots(c, p, &ns)) != PRC_OK) return st;
+    }
     cudaFree(c->slots);
+    reserve_give(c->dev, c->spare);
     c->slots = ns;
-    c->slots_b = n;
+    c->slots_b = p.n;
+    c->spare = p.spare;
   }
   c->B = B;
   c->win_var = win_variant;
@@ -1584,18 +1663,26 @@ int prc_d2z_batch_create(int n_boxes, const prc_d2z_desc* descs, int n_streams, 
   std::vector<int> order(n_boxes);
   for (int i = 0; i < n_boxes; ++i) order[i] = i;
   std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return descs[x].N > descs[y].N; });
-  b->ctx.assign(n_boxes, nullptr);
-  for (int k = 0; k < n_boxes; ++k) {
-    const int i = order[k];
-    prc_d2z_desc d = descs[i];
-    d.stream = b->streams[k % n_streams];
-    int st = prc_d2z_create(&d, &b->ctx[i]);
-    if (st == PRC_OK && n_streams > 1) b->ctx[i]->waves = kBatchWaves;
-    if (st != PRC_OK) {
-      batch_free(b);
-      delete b;
-      return st;
+  const int st = create_levels(descs, n_boxes, [&](Spare level) {
+    b->ctx.assign(n_boxes, nullptr);
+    int s = PRC_OK;
+    for (int k = 0; k < n_boxes && s == PRC_OK; ++k) {
+      prc_d2z_desc d = descs[order[k]];
+      d.stream = b->streams[k % n_streams];
+      s = create_at(&d, level, &b->ctx[order[k]]);
+      if (s == PRC_OK && n_streams > 1) b->ctx[order[k]]->waves = kBatchWaves;
     }
+    if (s != PRC_OK)
+      for (prc_d2z_ctx*& c : b->ctx) {
+        prc_d2z_destroy(c);
+        c = nullptr;
+      }
+    return s;
+  });
+  if (st != PRC_OK) {
+    batch_free(b);
+    delete b;
+    return st;
   }
   *out = b;
   return PRC_OK;
