@@ -117,7 +117,8 @@ typedef struct {
  * spectrum (one slot more) and small tables.  The default radius batch is 16 (8
  * for N >= 1024), or more, up to what 1 GB of slots holds, while a reserve lasts:
  * all contexts and batches of the process together hold at most 6 GB a device
- * beyond the slots named here (an odd batch's extra slot comes out of it too).
+ * beyond the slots named here.  Out of it comes one slot more for an odd default
+ * batch and for an odd radius_batch below N = 256, or of 3 and more up to N = 512.
  * A batch's boxes all get their share of it or none does.  zreion does not depend on the
  * radius batch; sigma_grid and the adjoint do in their rounding. */
 

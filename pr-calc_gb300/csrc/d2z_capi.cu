@@ -321,17 +321,11 @@ template <class T> int dalloc(T** p, size_t count, const char* what) {
   return PRC_OK;
 }
 
-// Radii per sweep.  Sweeps on pairs of radii (fft2.cuh) take an even number:
-// an odd radius batch is rounded up, or down when the extra slot could not be
-// allocated.  The pair kernels are left for the single-radius ones by the
-// faithful window, by a tuned window variant, and where there is one radius
-// or one slot.
+// The pair kernels (fft2.cuh) are left for the single-radius ones by the
+// faithful window, by a tuned window variant, and where there is one radius or
+// one slot.
 bool paired(const prc_d2z_ctx* c) {
   return c->ksl.pair && !(c->flags & PRC_FLAG_FAITHFUL_WINDOW) && c->win_var == 0 && c->nr > 1 && c->slots_b > 1;
-}
-int sweep_len(const prc_d2z_ctx* c) {
-  if (!paired(c) || c->B % 2 == 0) return c->B;
-  return c->B + 1 <= c->slots_b ? c->B + 1 : c->B - 1;
 }
 
 // Whether a sweep of nb radii runs in pairs.  The last pair of an odd sweep is
@@ -350,6 +344,32 @@ bool in_pairs(const prc_d2z_ctx* c, int nb, bool adjoint) {
   if (adjoint) return nb % 2 == 0 || nb >= 5;
   if (N == 512) return nb >= (nb % 2 ? 21 : 6);
   return nb % 2 == 0 || nb >= (N == 256 ? 11 : 7);
+}
+
+// The next sweep of a context with `left` radii to go: its number of radii, and
+// whether it runs in pairs.  Pairs take an even number, so an odd radius batch is
+// rounded up where its context has the slot for that.  Without it, an odd sweep
+// leaves its last radius to a sweep of its own (the single-radius kernels), or
+// runs on single radii altogether: that is where whole steps took the same time
+// (all but one in pairs against single radii: 64^3 x 15 53 / 52 us; 128^3 x 15 152
+// / 154; 192^3 x 7 260 / 266; 256^3 x 13 785 / 791; 384^3 x 7 1948 / 2033; 512^3 x
+// 17 8.23 / 8.28 ms; 768^3 x 5 14.5 / 14.6; 1024^3 x 5 31.7 / 32.4; the adjoint:
+// 128^3 x 11 119 / 134 us; 192^3 x 7 284 / 291; 256^3 x 7 545 / 550; 384^3 x 7
+// 2162 / 2207; 512^3 x 9 5.11 / 5.24 ms; 768^3 x 5 15.9 / 16.2; 1024^3 x 5 33.5 /
+// 35.1).
+int next_sweep(const prc_d2z_ctx* c, int left, bool adjoint, bool* pair) {
+  *pair = false;
+  if (!paired(c)) return std::min(left, c->B);
+  const int N = c->N;
+  int nb = std::min(left, c->B % 2 && c->B < c->slots_b ? c->B + 1 : c->B);
+  if (nb % 2 && nb >= c->slots_b) {
+    const int line = N >= 768 ? 5 : N == 512 ? (adjoint ? 9 : 17) : N == 384 || N == 192 ? 7
+                   : N == 256 ? (adjoint ? 7 : 13) : adjoint ? 11 : 15;
+    if (!in_pairs(c, nb - 1, adjoint) || (left == nb && nb < line)) return nb;
+    --nb;
+  }
+  *pair = in_pairs(c, nb, adjoint);
+  return nb;
 }
 
 // Radius slots beyond those that a context cannot do without (the radius batch
@@ -375,8 +395,11 @@ void reserve_give(int dev, long long bytes) {
   if (bytes > 0) g_reserve[dev].fetch_sub(bytes);
 }
 
-// What a context takes beyond its need: nothing, the odd batch's slot, or that
-// and the full default width.
+// What a context takes beyond its need: nothing, one slot to fill up the last
+// pair of an odd batch, or that and the full default width.  The extra slot is for
+// the default batch and for grids where it is small beside what was asked for (up
+// to 29 MB below 256^3; up to 512^3 at most a third more); a larger one is left
+// out, and sweeps do without (next_sweep).
 enum Spare { kLean = 0, kOdd = 1, kFull = 2 };
 
 struct SlotPlan {
@@ -390,7 +413,7 @@ struct SlotPlan {
 // and fewer re-reads of the spectrum and of zreion: 64^3 x 64 radii in one
 // sweep instead of four, 122 -> 92 us; 192^3 x 41 1127 -> 1087.  Without reserve
 // the default is those 16 (8).
-SlotPlan slot_plan(const KernelSet& ks, int nr, int radius_batch, Spare level) {
+SlotPlan slot_plan(const KernelSet& ks, int nr, int radius_batch, int flags, Spare level) {
   const long long bytes = (long long)ks.N * ks.N * (ks.N / 2 + 2) * sizeof(float2);
   const int b_min = ks.N >= 1024 ? 8 : 16;
   const int need = std::min(radius_batch ? radius_batch : b_min, nr);
@@ -398,8 +421,9 @@ SlotPlan slot_plan(const KernelSet& ks, int nr, int radius_batch, Spare level) {
   p.B = need;
   if (!radius_batch && level == kFull)
     p.B = std::min(nr, std::max(b_min, (int)std::min<long long>(kMaxBatch, (1ll << 30) / bytes)));
-  p.n = p.B;
-  if (level >= kOdd && ks.pair && nr > 1 && p.B % 2 == 1) p.n = p.B + 1;
+  const bool small = !radius_batch || ks.N < 256 || (ks.N <= 512 && p.B > 1);
+  const bool odd = p.B % 2 && nr > 1 && ks.pair && !(flags & PRC_FLAG_FAITHFUL_WINDOW);
+  p.n = p.B + (level >= kOdd && odd && small ? 1 : 0);
   p.spare = (p.n - need) * bytes;
   return p;
 }
@@ -584,10 +608,9 @@ void enqueue_sweeps(prc_d2z_ctx* c, float* d_z, uint8_t* d_am, double* sig, floa
                     uint8_t* am_out = nullptr, bool withhold = false) {
   const int N = c->N, H = c->H;
   const long long NN = c->NN;
-  const int B = sweep_len(c);
-  for (int r0 = 0; r0 < c->nr; r0 += B) {
-    const int nb = (c->nr - r0 < B) ? c->nr - r0 : B;
-    const bool pair = in_pairs(c, nb, false);
+  for (int r0 = 0, nb; r0 < c->nr; r0 += nb) {
+    bool pair;
+    nb = next_sweep(c, c->nr - r0, false, &pair);
     SweepArgs sa;
     memset(&sa, 0, sizeof(sa));
     sa.slots = c->slots;
@@ -991,7 +1014,7 @@ int create_at(const prc_d2z_desc* d, Spare level, prc_d2z_ctx** out) {
     return cuda_fail(e, "prc_d2z_create: device set-up");
   }
   const long long n3l = (long long)c->NN * c->N;
-  const SlotPlan plan = slot_plan(*ks, c->nr, d->radius_batch, level);
+  const SlotPlan plan = slot_plan(*ks, c->nr, d->radius_batch, d->flags, level);
   c->B = plan.B;
   c->slots_b = plan.n;
   auto slots = [&]() {
@@ -1042,7 +1065,7 @@ int create_levels(const prc_d2z_desc* d, int n, const std::function<int(Spare)>&
     long long spare = 0;
     for (int i = 0; i < n; ++i)
       if (const KernelSet* ks = kernel_set(d[i].N))
-        spare += slot_plan(*ks, d[i].n_radii, d[i].radius_batch, (Spare)level).spare;
+        spare += slot_plan(*ks, d[i].n_radii, d[i].radius_batch, d[i].flags, (Spare)level).spare;
     if (spare <= 0 || dev < 0 || dev >= kReserveDevices || g_reserve[dev].load() + spare > kReserveBytes) continue;
     const int st = create((Spare)level);
     if (st != PRC_ERR_ALLOC) return st;
@@ -1434,10 +1457,9 @@ int prc_d2z_backward(prc_d2z_ctx* c, const float* dL_dz, const uint8_t* argmax, 
   PRC_CU(cudaEventRecord(c->ev[0], c->st), "event");
   float2* U = c->slots;
   float2* acc = c->spec;
-  const int B = sweep_len(c);
-  for (int r0 = 0; r0 < c->nr; r0 += B) {
-    const int nb = (c->nr - r0 < B) ? c->nr - r0 : B;
-    const bool pair = in_pairs(c, nb, true);
+  for (int r0 = 0, nb; r0 < c->nr; r0 += nb) {
+    bool pair;
+    nb = next_sweep(c, c->nr - r0, true, &pair);
     AdjArgs aa;
     memset(&aa, 0, sizeof(aa));
     aa.g = d_g;
@@ -1600,10 +1622,10 @@ int prc_d2z_tune(prc_d2z_ctx* c, int radius_batch, int win_variant) {
     if ((st = set_device(c)) != PRC_OK) return st;
     PRC_CU(cudaStreamSynchronize(c->st), "prc_d2z_tune");
     float2* ns = nullptr;
-    SlotPlan p = slot_plan(c->ksl, c->nr, B, kOdd);
+    SlotPlan p = slot_plan(c->ksl, c->nr, B, c->flags, kOdd);
     if (p.n > B && alloc_slots(c, p, &ns) != PRC_OK) ns = nullptr;
     if (!ns) {
-      p = slot_plan(c->ksl, c->nr, B, kLean);
+      p = slot_plan(c->ksl, c->nr, B, c->flags, kLean);
       if ((st = alloc_slots(c, p, &ns)) != PRC_OK) return st;
     }
     cudaFree(c->slots);

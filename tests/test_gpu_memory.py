@@ -34,8 +34,9 @@ COUNT, N, NR = 40, 128, 64
 LEAN = COUNT * 17 * _slot(N)
 
 
-def _warm():
-    with prc_d2z.Delta2Zreion(**_box(N, 2)):
+def _warm(n=N):
+    """Loads the kernels of a size (device memory that no context owns)."""
+    with prc_d2z.Delta2Zreion(**_box(n, 1)):
         pass
 
 
@@ -82,3 +83,36 @@ def test_boxes_without_reserve_give_the_same_results():
     batch.close()
     for c in ctx:
         c.close()
+
+
+# (N, radius_batch, slots beyond the spectrum's): a batch that bounds the memory of
+# a large grid gets the slots it asks for; below 256^3, and up to 512^3 from three on,
+# an odd one takes one more, but not for the faithful window, which runs no pairs
+@pytest.mark.parametrize("N,B,slots,faithful", [(192, 1, 2, False), (256, 1, 1, False), (256, 3, 4, False), (256, 5, 5, True),
+                                                (512, 1, 1, False), (768, 1, 1, False), (768, 3, 3, False),
+                                                (1024, 1, 1, False)])
+def test_an_odd_radius_batch(N, B, slots, faithful):
+    _warm(N)
+    c, used = _used(lambda: prc_d2z.Delta2Zreion(**_box(N, 2 * B + 2, radius_batch=B), faithful_window=faithful))
+    assert (slots + 1) * _slot(N) <= used <= (slots + 1.5) * _slot(N) + 2 ** 24, used / _slot(N)
+    c.close()
+
+
+# without that slot the sweeps of an odd batch are its pairs and the last radius
+# (sweeps counted by launches: 3 forward passes, 3 a sweep)
+@pytest.mark.parametrize("N,nr,B,sweeps", [(256, 4, 1, 4), (768, 3, 3, 1), (768, 5, 5, 2), (768, 7, 3, 3), (1024, 3, 1, 3)])
+def test_odd_sweeps_without_the_extra_slot(N, nr, B, sweeps):
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(N + nr)
+    delta = 3.0 * torch.randn((N, N, N), device="cuda", generator=gen)
+    with prc_d2z.Delta2Zreion(**_box(N, nr)) as ctx:
+        z0, am0, _ = ctx.forward(delta)
+        g0, db0 = ctx.backward(delta, am0)
+    with prc_d2z.Delta2Zreion(**_box(N, nr, radius_batch=B)) as ctx:
+        z, am, _ = ctx.forward(delta)
+        assert ctx.last_launches() == 3 + 3 * sweeps
+        g, db = ctx.backward(delta, am0)
+    assert torch.equal(z, z0) and torch.equal(am, am0)
+    # the sums over the radii meet in another order: a few roundings of float sums
+    assert float((g - g0).abs().max()) <= 1e-6 * float(g0.abs().max())
+    np.testing.assert_allclose(db, db0, rtol=1e-10, atol=1e-10 * N ** 1.5)
