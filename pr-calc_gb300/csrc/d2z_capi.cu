@@ -664,6 +664,7 @@ void enqueue_sweeps(prc_d2z_ctx* c, float* d_z, uint8_t* d_am, double* sig, floa
 // share out the batch's n_streams streams, largest grid size first.
 struct BatchGroup {
   int N = 0, nsweeps = 0;
+  bool pair = false;             // sweeps on pairs of radii (boxes of one size may form two groups)
   std::vector<int> boxes;        // batch indices
   cudaStream_t st = nullptr;    // one of the batch's streams (groups round-robin, largest first)
   // table offsets (bytes) in the batch's table buffer
@@ -724,18 +725,38 @@ void batch_enqueue(prc_d2z_batch* b, const float* const* delta, float* const* zr
 
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-// A box joins a grouped launch when its size has grouped kernels and it asks
-// for nothing they leave out: the faithful window, a single radius (or slot)
-// and the few odd radii at 256^3 that in_pairs leaves to the single-radius
-// kernels run per box.  (A tuned window variant is not used there.)
-bool groupable(const prc_d2z_ctx* c) {
-  return c->ksl.grouped && !(c->flags & PRC_FLAG_FAITHFUL_WINDOW) && c->nr > 1 && c->slots_b > 1 &&
-         !(c->N >= 256 && c->nr % 2 && c->nr < 11);
-}
-// radii per sweep of a grouped box (its window variant does not matter)
-int grouped_len(const prc_d2z_ctx* c) {
+// A box joins a grouped launch when its size has grouped kernels and it does
+// not ask for the faithful window.  (A tuned window variant is not used there.)
+bool groupable(const prc_d2z_ctx* c) { return c->ksl.grouped && !(c->flags & PRC_FLAG_FAITHFUL_WINDOW); }
+// Radii per sweep of a grouped box on pairs (its window variant does not matter).
+int pair_len(const prc_d2z_ctx* c) {
   return c->B % 2 == 0 ? c->B : c->B + 1 <= c->slots_b ? c->B + 1 : c->B - 1;
 }
+// Whether a grouped box is better run in pairs (all its sweeps are, a last one of
+// an odd number filled up): not with one radius or slot, nor where single radii
+// do its first sweep faster.  A whole grouped call in pairs against single radii, us: 24
+// boxes of 96^3 x 3 505 / 475, x 5 630 / 629; 16 of 128^3 x 3 674 / 584, x 7 1025
+// / 1009, x 9 1193 / 1218; 8 of 192^3 x 3 1130 / 1059, x 5 1470 / 1494; 6 of 256^3 x
+// 2 1274 / 1223, x 4 1847 / 1844, x 13 4545 / 4589; 32 of 64^3 x 3 286 / 281, x 5
+// 334 / 333, x 9 432 / 451.
+bool pairs_first(const prc_d2z_ctx* c) {
+  const int N = c->N, nb = std::min(pair_len(c), c->nr);
+  if (nb % 2 == 0) return N < 256 || nb >= 4;
+  return nb >= (N >= 256 ? 13 : N == 128 ? 9 : N >= 96 ? 5 : 3);
+}
+// Where pairs are better for half of a size's boxes or more, the others that can
+// join them do: a second group's launches cost more than their filled halves.
+bool grouped_pair(const prc_d2z_batch* b, const prc_d2z_ctx* c) {
+  if (c->nr < 2 || c->slots_b < 2) return false;
+  int boxes = 0, first = 0;
+  for (const prc_d2z_ctx* o : b->ctx)
+    if (o->N == c->N && groupable(o) && o->nr > 1 && o->slots_b > 1) {
+      ++boxes;
+      first += pairs_first(o);
+    }
+  return pairs_first(c) || (c->N < 256 && 2 * first >= boxes);
+}
+int grouped_len(const BatchGroup& g, const prc_d2z_ctx* c) { return g.pair ? pair_len(c) : c->B; }
 
 // Groups of equal grid size, their sweeps and the layout of their tables.
 // Sizes without grouped kernels keep per-box launches (no group).
@@ -748,30 +769,34 @@ int batch_group_setup(prc_d2z_batch* b) {
   if (b->h_tab) cudaFreeHost(b->h_tab);
   b->h_tab = nullptr;
   b->tab_bytes = 0;
-  std::vector<int> sizes;
-  for (auto* c : b->ctx)
-    if (groupable(c) && std::find(sizes.begin(), sizes.end(), c->N) == sizes.end()) sizes.push_back(c->N);
-  std::sort(sizes.begin(), sizes.end(), [](int x, int y) { return x > y; });
+  std::vector<std::pair<int, bool>> sizes;  // (N, on pairs)
+  for (auto* c : b->ctx) {
+    const std::pair<int, bool> k(c->N, grouped_pair(b, c));
+    if (groupable(c) && std::find(sizes.begin(), sizes.end(), k) == sizes.end()) sizes.push_back(k);
+  }
+  std::sort(sizes.begin(), sizes.end(), [](const auto& x, const auto& y) { return x > y; });
   size_t off = 0;
-  for (int N : sizes) {
+  for (const auto& size : sizes) {
     BatchGroup g;
+    const int N = size.first;
     g.N = N;
+    g.pair = size.second;
     for (int i = 0; i < b->n; ++i)
-      if (b->ctx[i]->N == N && groupable(b->ctx[i])) {
+      if (b->ctx[i]->N == N && groupable(b->ctx[i]) && grouped_pair(b, b->ctx[i]) == g.pair) {
         g.boxes.push_back(i);
         const prc_d2z_ctx* c = b->ctx[i];
-        g.nsweeps = std::max(g.nsweeps, (c->nr + grouped_len(c) - 1) / grouped_len(c));
+        g.nsweeps = std::max(g.nsweeps, (c->nr + grouped_len(g, c) - 1) / grouped_len(g, c));
       }
     for (int sw = 0; sw < g.nsweeps; ++sw) {
       std::vector<int> bx;
       for (int i : g.boxes)
-        if (b->ctx[i]->nr > sw * grouped_len(b->ctx[i])) bx.push_back(i);
+        if (b->ctx[i]->nr > sw * grouped_len(g, b->ctx[i])) bx.push_back(i);
       auto nb_of = [&](int i) {
-        const int B = grouped_len(b->ctx[i]);
+        const int B = grouped_len(g, b->ctx[i]);
         return std::min(B, b->ctx[i]->nr - sw * B);
       };
-      // most radii first: the boxes with more than y pairs in the sweep are a
-      // prefix, which the inverse y pass's pair y takes
+      // most radii first: the boxes with more than y radii (pairs) in the sweep
+      // are a prefix, which the inverse y pass's slot (pair) y takes
       std::stable_sort(bx.begin(), bx.end(), [&](int x, int y) { return nb_of(x) > nb_of(y); });
       std::vector<int> nbs;
       for (int i : bx) nbs.push_back(nb_of(i));
@@ -841,15 +866,16 @@ void batch_group_fill(prc_d2z_batch* b, const float* const* delta, float* const*
         const int i = g.sw_box[sw][k];
         const prc_d2z_ctx* c = b->ctx[i];
         const long long NN = c->NN, H = c->H;
-        const int r0 = sw * grouped_len(c), nb = g.sw_nb[sw][k];
+        const int r0 = sw * grouped_len(g, c), nb = g.sw_nb[sw][k];
         float2* U = c->slots;
+        float2* UQ = U + NN * H * (g.pair ? 2 : 1);
         BoxCol w, v;
         memset(&w, 0, sizeof w);
         memset(&v, 0, sizeof v);
-        w.in0 = c->spec, w.out0 = U, w.in1 = c->spec + NN * H, w.out1 = U + 2 * NN * H, w.nb = nb;
+        w.in0 = c->spec, w.out0 = U, w.in1 = c->spec + NN * H, w.out1 = UQ, w.nb = nb;
         for (int q = 0; q < nb; ++q) w.kr[q] = c->kr[r0 + q];
-        if (nb % 2) w.kr[nb] = w.kr[nb - 1];  // as in run_tile
-        v.in0 = U, v.out0 = U, v.in1 = U + 2 * NN * H, v.out1 = U + 2 * NN * H, v.nb = nb;
+        if (g.pair && nb % 2) w.kr[nb] = w.kr[nb - 1];  // as in run_tile
+        v.in0 = U, v.out0 = U, v.in1 = UQ, v.out1 = UQ, v.nb = nb;
         memcpy(h + g.o_win[sw] + k * sizeof(BoxCol), &w, sizeof w);
         memcpy(h + g.o_inv[sw] + k * sizeof(BoxCol), &v, sizeof v);
         BoxLine L;
@@ -859,7 +885,7 @@ void batch_group_fill(prc_d2z_batch* b, const float* const* delta, float* const*
         L.argmax = L.argmax_out = argmax ? argmax[i] : nullptr;
         L.nb = nb, L.r0 = r0, L.first = (sw == 0), L.as = c->as;
         for (int q = 0; q < nb; ++q) L.cb[q] = c->cb[r0 + q];
-        if (nb % 2) L.cb[nb] = NAN;  // never wins
+        if (g.pair && nb % 2) L.cb[nb] = NAN;  // never wins
         memcpy(h + g.o_line[sw] + k * sizeof(BoxLine), &L, sizeof L);
       }
     }
@@ -884,14 +910,16 @@ void batch_enqueue_grouped(prc_d2z_batch* b, const float* const* delta, float* c
     float2* U0 = c0->slots;
     ks.r2c_z_mb(ks, grid_for(N * N * nbox, ks.line_groups, ks.occ_mb_r2c, sms), g.st,
                 reinterpret_cast<const BoxR2c*>(b->d_tab + g.o_r2c), nbox, c0->tw);
+    const KernelSet::Grouped& mb = ks.mb[g.pair];
+    const int step = g.pair ? 2 : 1;  // radii per slot of the y pass
     auto cols = [&](int mode, TileSeg s0, TileSeg s1, size_t o, int nboxes, int gy, const int* nvb) {
       TileArgs a;
       memset(&a, 0, sizeof(a));
       if (mode != TM_FWD) {
-        const int tw = mode == TM_WIN ? ks.pair_tile_w_win : ks.pair_tile_w;
+        const int tw = mode == TM_WIN ? mb.tile_w_win : mb.tile_w_inv;
         s0.tpo = H / tw;
         s1.tpo = N / tw;
-        if (mode == TM_INV) pair_rows(ks, &s0);
+        if (mode == TM_INV && g.pair) pair_rows(ks, &s0);
       }
       a.seg[0] = s0;
       a.seg[1] = s1;
@@ -902,9 +930,10 @@ void batch_enqueue_grouped(prc_d2z_batch* b, const float* const* delta, float* c
       if (nvb)
         for (int y = 0; y < gy; ++y) a.nvb[y] = nvb[y];
       const int tpb = s0.n_outer * s0.tpo + s1.n_outer * s1.tpo;
-      const int occ = mode == TM_WIN ? ks.occ_mb_win : mode == TM_INV ? ks.occ_mb_inv : ks.occ_mb_tile;
-      ks.tile_mb(ks, mode, dim3(grid_for(tpb * (nvb ? nvb[0] : nboxes), 1, occ * (mode == TM_WIN ? waves : 1), sms), gy, 1),
-                 g.st, a);
+      const int occ = mode == TM_WIN ? mb.occ_win * (g.pair ? waves : 1) : mode == TM_INV ? mb.occ_inv : ks.occ_mb_tile;
+      const dim3 grid(grid_for(tpb * (nvb ? nvb[0] : nboxes), 1, occ, sms), gy, 1);
+      if (mode == TM_FWD) ks.tile_mb(ks, grid, g.st, a);
+      else mb.tile(ks, mode, grid, g.st, a);
       ++launches;
     };
     cols(TM_FWD, mseg(c0, S0, S0, false), qseg(c0, S0 + NN * (H + 1), S0 + NN * H, true), g.o_fy, nbox, 1, nullptr);
@@ -912,13 +941,13 @@ void batch_enqueue_grouped(prc_d2z_batch* b, const float* const* delta, float* c
     for (int sw = 0; sw < g.nsweeps; ++sw) {
       const int ns = (int)g.sw_box[sw].size();
       const std::vector<int>& nbs = g.sw_nb[sw];
-      float2* UQ = U0 + 2 * NN * H;
+      float2* UQ = U0 + step * NN * H;
       cols(TM_WIN, mseg(c0, S0, U0, true), qseg(c0, S0 + NN * H, UQ, true), g.o_win[sw], ns, 1, nullptr);
-      const int np = (nbs[0] + 1) / 2;
+      const int np = (nbs[0] + step - 1) / step;
       int nvb[kMaxBatch];
       for (int y = 0; y < np; ++y) {
         int k = 0;
-        while (k < ns && nbs[k] > 2 * y) ++k;
+        while (k < ns && nbs[k] > step * y) ++k;
         nvb[y] = k;
       }
       cols(TM_INV, mseg(c0, U0, U0, false), qseg(c0, UQ, UQ, false), g.o_inv[sw], ns, np, nvb);
@@ -930,7 +959,7 @@ void batch_enqueue_grouped(prc_d2z_batch* b, const float* const* delta, float* c
       sa.argmax = argmax ? argmax[g.sw_box[sw][0]] : nullptr;
       sa.box = reinterpret_cast<const BoxLine*>(b->d_tab + g.o_line[sw]);
       sa.nbox = ns;
-      ks.c2r_z_mb(ks, grid_for(N * N * ns, ks.mb_lines, ks.occ_mb_c2r * waves, sms), g.st, sa);
+      mb.c2r_z(ks, grid_for(N * N * ns, mb.lines, mb.occ_c2r * (g.pair ? waves : 1), sms), g.st, sa);
       launches += 2;
     }
     launches += 1;

@@ -163,9 +163,11 @@ template <int N, int MODE, int V> struct ColK {
                                          CK<N, CCfg<N>::T, typename CCfg<N>::P>>::type;
 };
 
-// MB (grouped launch, TM_FWD only): the tiles of a.nbox boxes of this grid
-// size, box i's segment pointers from a.box[i]; tile ti is tile ti mod (tiles
-// of one box) of box ti / (tiles of one box).
+// MB (grouped launch): the tiles of a.nbox boxes of this grid size, box i's
+// segment pointers, radius count and dk * R_b from a.box[i]; tile ti is tile
+// ti mod (tiles of one box) of box ti / (tiles of one box).  The inverse y
+// pass takes slot blockIdx.y of the first a.nvb[blockIdx.y] boxes (those with
+// more than blockIdx.y slots: the boxes are sorted by nb, largest first).
 template <int N, int MODE, int V = 0, bool MB = false>
 __global__ void __launch_bounds__(ColK<N, MODE, V>::type::THREADS, ColK<N, MODE, V>::type::MINB) k_col(TileArgs a) {
   using KK = typename ColK<N, MODE, V>::type;
@@ -191,11 +193,11 @@ __global__ void __launch_bounds__(ColK<N, MODE, V>::type::THREADS, ColK<N, MODE,
   }
   PPCol<T, G, FirstRadix<P>::v> buf{tws + KK::TW + c, KK::BUF};
   const CtaSync sync;
-  static_assert(!MB || MODE == TM_FWD, "grouped: the forward passes");
+  static_assert(!MB || MODE != TM_ACC, "no grouped adjoint pass");
   const long long yoff = (MODE == TM_FWD || MODE == TM_INV) ? (long long)blockIdx.y * a.slot_stride : 0;
   const int tiles0 = a.seg[0].n_outer * a.seg[0].tpo;
   const int tpb = tiles0 + a.seg[1].n_outer * a.seg[1].tpo;  // tiles of one box
-  const int tiles = MB ? tpb * a.nbox : tpb;
+  const int tiles = !MB ? tpb : tpb * (MODE == TM_INV ? a.nvb[blockIdx.y] : a.nbox);
 
   // A tile: its segment (0 main, 1 Nyquist plane), outer index, column
   // block and offset; the segment's fields are read from the kernel
@@ -367,7 +369,9 @@ __global__ void __launch_bounds__(ColK<N, MODE, V>::type::THREADS, ColK<N, MODE,
       }
       auto radius = [&](int b, bool last) {
         float wv[E];
-        const float krb = s_kr[b];
+        float krb;
+        if constexpr (MB) krb = __ldg(&a.box[w.bx].kr[b]);
+        else krb = s_kr[b];
         if constexpr (FW) {
 #pragma unroll
           for (int m = 0; m < E; ++m) wv[m] = window_faithful(kq[m], krb);
@@ -390,8 +394,10 @@ __global__ void __launch_bounds__(ColK<N, MODE, V>::type::THREADS, ColK<N, MODE,
         gstore(w, sg_out(w) + (long long)b * a.slot_stride, v);
       };
       // the last radius is peeled so that kq's and raw's live ranges end before it
-      int b0 = 0, b1 = a.nb;
-      if constexpr (kWinRadiusSplit<N>) radius_range(a.nb, b0, b1);
+      int b0 = 0, b1;
+      if constexpr (MB) b1 = __ldg(&a.box[w.bx].nb);
+      else if constexpr (kWinRadiusSplit<N>) radius_range(a.nb, b0, b1);
+      else b1 = a.nb;
       for (int b = b0; b < b1 - 1; ++b) radius(b, false);
       radius(b1 - 1, true);
     }

@@ -45,13 +45,20 @@ struct KernelSet {
   void (*pair_c2r)(const KernelSet&, int grid, cudaStream_t, const SweepArgs&);
   // grouped launches (several boxes of this size per launch), when compiled
   // for this size (grouped = 1): forward z pass, forward column passes, and
-  // the sweep's passes on pairs of radii (TM_WIN, TM_INV, inverse z)
+  // the sweep's passes (TM_WIN, TM_INV, inverse z) on single radii [0] and on
+  // pairs [1]
+  struct Grouped {
+    int tile_w_win, tile_w_inv;
+    int lines;  // lines per CTA step of the inverse z pass
+    int occ_win, occ_inv, occ_c2r;
+    void (*tile)(const KernelSet&, int mode, dim3 grid, cudaStream_t, const TileArgs&);
+    void (*c2r_z)(const KernelSet&, int grid, cudaStream_t, const SweepArgs&);
+  };
   int grouped;
-  int mb_lines;  // lines per CTA step of the inverse z pass
-  int occ_mb_tile, occ_mb_inv, occ_mb_win, occ_mb_c2r, occ_mb_r2c;
+  Grouped mb[2];
+  int occ_mb_tile, occ_mb_r2c;
   void (*r2c_z_mb)(const KernelSet&, int grid, cudaStream_t, const BoxR2c* box, int nbox, const float2* tw);
-  void (*tile_mb)(const KernelSet&, int mode, dim3 grid, cudaStream_t, const TileArgs&);
-  void (*c2r_z_mb)(const KernelSet&, int grid, cudaStream_t, const SweepArgs&);
+  void (*tile_mb)(const KernelSet&, dim3 grid, cudaStream_t, const TileArgs&);
 };
 
 // nullptr when N has no compiled plan

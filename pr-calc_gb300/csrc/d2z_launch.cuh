@@ -129,11 +129,19 @@ template <int N> struct ColLaunch<N, true> {
       default: k_col<N, TM_ACC><<<grid, CA::THREADS, CSA, st>>>(a); break;
     }
   }
-  // grouped forward column passes (several boxes of this size per launch)
+  // grouped launches (several boxes of this size per launch; window variant 0)
   static constexpr bool GROUPED = N <= 256 && PCfg<N>::on;
-  static void* fn_mb() { return reinterpret_cast<void*>(&k_col<N, TM_FWD, 0, true>); }
-  static void launch_mb(dim3 grid, cudaStream_t st, const TileArgs& a) {
-    if constexpr (GROUPED) launch_pdl(&k_col<N, TM_FWD, 0, true>, grid, THREADS, CS, st, a);
+  using W0 = typename Win<0>::K;
+  static constexpr size_t WS0 = (size_t)W0::smem_f2 * sizeof(float2);
+  template <int MODE> static void* fn_mb() { return reinterpret_cast<void*>(&k_col<N, MODE, 0, true>); }
+  static void launch_mb(int mode, dim3 grid, cudaStream_t st, const TileArgs& a) {
+    if constexpr (GROUPED) {
+      switch (mode) {
+        case TM_FWD: launch_pdl(&k_col<N, TM_FWD, 0, true>, grid, THREADS, CS, st, a); break;
+        case TM_INV: k_col<N, TM_INV, 0, true><<<grid, THREADS, CS, st>>>(a); break;
+        default: k_col<N, TM_WIN, 0, true><<<grid, W0::THREADS, WS0, st>>>(a); break;
+      }
+    }
   }
 };
 
@@ -160,6 +168,12 @@ template <int N> struct C2rLaunch<N, true> {
       if (a.argmax) k_c2r_zp<N, true, false><<<grid, THREADS, BYTES, st>>>(a);
       else k_c2r_zp<N, false, false><<<grid, THREADS, BYTES, st>>>(a);
     }
+  }
+  // grouped: a.argmax != null means every box of the launch records its argmax
+  template <bool AM> static void* f_mb() { return reinterpret_cast<void*>(&k_c2r_zp<N, AM, false, true>); }
+  static void launch_mb(int grid, cudaStream_t st, const SweepArgs& a) {
+    if (a.argmax) k_c2r_zp<N, true, false, true><<<grid, THREADS, BYTES, st>>>(a);
+    else k_c2r_zp<N, false, false, true><<<grid, THREADS, BYTES, st>>>(a);
   }
 };
 
@@ -204,7 +218,6 @@ template <int N> struct PairLaunch<N, true> {
       else launch_pdl(&k_c2r_zp2<N, false, false>, grid, KZ::THREADS, KZ::bytes, st, a);
     }
   }
-  // grouped: a.argmax != null means every box of the launch records its argmax
   static void c2r_mb(int grid, cudaStream_t st, const SweepArgs& a) {
     if (a.argmax) launch_pdl(&k_c2r_zp2<N, true, false, true>, grid, KZM::THREADS, KZM::bytes, st, a);
     else launch_pdl(&k_c2r_zp2<N, false, false, true>, grid, KZM::THREADS, KZM::bytes, st, a);
@@ -268,21 +281,31 @@ template <int N> struct Launchers {
       if ((e = occ(&ks->occ_pair_c2r, z[1], PL::KZ::THREADS, PL::KZ::bytes)) != cudaSuccess) return e;
     }
     if constexpr (CL::GROUPED) {
-      void* fm = CL::fn_mb();
-      void* im = PL::template inv_fn<true>();
-      void* wm = PL::template win_fn<true>();
-      void* z0 = PL::template z_fn<false, false, true>();
-      void* z1 = PL::template z_fn<true, false, true>();
+      KernelSet::Grouped &one = ks->mb[0], &two = ks->mb[1];
+      void* fm = CL::template fn_mb<TM_FWD>();
+      void* i1 = CL::template fn_mb<TM_INV>();
+      void* w1 = CL::template fn_mb<TM_WIN>();
+      void* i2 = PL::template inv_fn<true>();
+      void* w2 = PL::template win_fn<true>();
+      void* z1[2] = {CR::template f_mb<false>(), CR::template f_mb<true>()};
+      void* z2[2] = {PL::template z_fn<false, false, true>(), PL::template z_fn<true, false, true>()};
       if ((e = smem(fm, CL::CS)) != cudaSuccess) return e;
-      if ((e = smem(im, PL::KI::bytes)) != cudaSuccess) return e;
-      if ((e = smem(wm, PL::KW::bytes)) != cudaSuccess) return e;
-      if ((e = smem(z0, PL::KZM::bytes)) != cudaSuccess) return e;
-      if ((e = smem(z1, PL::KZM::bytes)) != cudaSuccess) return e;
+      if ((e = smem(i1, CL::CS)) != cudaSuccess) return e;
+      if ((e = smem(w1, CL::WS0)) != cudaSuccess) return e;
+      if ((e = smem(i2, PL::KI::bytes)) != cudaSuccess) return e;
+      if ((e = smem(w2, PL::KW::bytes)) != cudaSuccess) return e;
+      for (int k = 0; k < 2; ++k) {
+        if ((e = smem(z1[k], CR::BYTES)) != cudaSuccess) return e;
+        if ((e = smem(z2[k], PL::KZM::bytes)) != cudaSuccess) return e;
+      }
       if ((e = smem(&k_r2c_z<N, true>, LS)) != cudaSuccess) return e;
       if ((e = occ(&ks->occ_mb_tile, fm, CL::THREADS, CL::CS)) != cudaSuccess) return e;
-      if ((e = occ(&ks->occ_mb_inv, im, PL::KI::THREADS, PL::KI::bytes)) != cudaSuccess) return e;
-      if ((e = occ(&ks->occ_mb_win, wm, PL::KW::THREADS, PL::KW::bytes)) != cudaSuccess) return e;
-      if ((e = occ(&ks->occ_mb_c2r, z1, PL::KZM::THREADS, PL::KZM::bytes)) != cudaSuccess) return e;
+      if ((e = occ(&one.occ_inv, i1, CL::THREADS, CL::CS)) != cudaSuccess) return e;
+      if ((e = occ(&one.occ_win, w1, CL::W0::THREADS, CL::WS0)) != cudaSuccess) return e;
+      if ((e = occ(&one.occ_c2r, z1[1], CR::THREADS, CR::BYTES)) != cudaSuccess) return e;
+      if ((e = occ(&two.occ_inv, i2, PL::KI::THREADS, PL::KI::bytes)) != cudaSuccess) return e;
+      if ((e = occ(&two.occ_win, w2, PL::KW::THREADS, PL::KW::bytes)) != cudaSuccess) return e;
+      if ((e = occ(&two.occ_c2r, z2[1], PL::KZM::THREADS, PL::KZM::bytes)) != cudaSuccess) return e;
       if ((e = occ(&ks->occ_mb_r2c, &k_r2c_z<N, true>, LL::THREADS, LS)) != cudaSuccess) return e;
     }
     if ((e = smem(CL::faithful_fn(), CL::FS)) != cudaSuccess) return e;
@@ -308,14 +331,20 @@ template <int N> struct Launchers {
     if constexpr (CL::GROUPED) launch_pdl(&k_r2c_z<N, true>, grid, LL::THREADS, LS, st, (const float*)nullptr, 1.f, (float2*)nullptr, (float2*)nullptr,
                                                tw, box, nbox);
   }
-  static void tile_mb(const KernelSet&, int mode, dim3 grid, cudaStream_t st, const TileArgs& a) {
+  static void tile_mb(const KernelSet&, dim3 grid, cudaStream_t st, const TileArgs& a) {
+    if constexpr (CL::GROUPED) CL::launch_mb(TM_FWD, grid, st, a);
+  }
+  template <bool PAIR> static void sweep_mb(const KernelSet&, int mode, dim3 grid, cudaStream_t st, const TileArgs& a) {
     if constexpr (CL::GROUPED) {
-      if (mode == TM_FWD) CL::launch_mb(grid, st, a);
-      else PL::template tile<true>(mode, grid, st, a);
+      if constexpr (PAIR) PL::template tile<true>(mode, grid, st, a);
+      else CL::launch_mb(mode, grid, st, a);
     }
   }
-  static void c2r_z_mb(const KernelSet&, int grid, cudaStream_t st, const SweepArgs& a) {
-    if constexpr (CL::GROUPED) PL::c2r_mb(grid, st, a);
+  template <bool PAIR> static void c2r_z_mb(const KernelSet&, int grid, cudaStream_t st, const SweepArgs& a) {
+    if constexpr (CL::GROUPED) {
+      if constexpr (PAIR) PL::c2r_mb(grid, st, a);
+      else CR::launch_mb(grid, st, a);
+    }
   }
   static void pair_tile(const KernelSet&, int mode, dim3 grid, cudaStream_t st, const TileArgs& a) {
     if constexpr (PL::on) {
@@ -370,10 +399,10 @@ template <int N> struct Launchers {
     }
     if constexpr (CL::GROUPED) {
       ks.grouped = 1;
-      ks.mb_lines = PL::KZM::NG;
+      ks.mb[0] = {CL::W0::T, CL::T, CR::NG, 0, 0, 0, &sweep_mb<false>, &c2r_z_mb<false>};
+      ks.mb[1] = {PL::KW::T, PL::KI::T, PL::KZM::NG, 0, 0, 0, &sweep_mb<true>, &c2r_z_mb<true>};
       ks.r2c_z_mb = &r2c_z_mb;
       ks.tile_mb = &tile_mb;
-      ks.c2r_z_mb = &c2r_z_mb;
     }
     return ks;
   }
