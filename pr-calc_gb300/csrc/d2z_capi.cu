@@ -204,7 +204,7 @@ struct prc_d2z_ctx {
   int win_var = 0;   // window-pass variant (prc_d2z_tune)
   int slots_b = 0;   // radius slots allocated (one more than B for an odd B of paired sweeps)
   long long spare = 0;  // bytes of them taken from the reserve (SlotPlan)
-  int waves = 1;     // CTA waves of the window and z passes (batches: kBatchWaves)
+  bool shared = false;  // a batch's box: other streams' kernels share the GPU
   long long NN = 0, slot_f2 = 0;
   double box = 0, A = 0, dinit = 1;
   std::vector<double> R, Bb;
@@ -305,10 +305,14 @@ int grid_for(int items, int per_cta, int occ, int sms) {
   return (int)(need < cap ? need : cap);
 }
 
-// A context alone runs its passes as one wave of resident CTAs.  Where kernels
-// of several streams share the GPU, a CTA that has to wait for its place
-// would start its whole share late; smaller shares even that out.
-constexpr int kBatchWaves = 4;
+// A pass is one wave of resident CTAs, but for the window and z passes of groups
+// on pairs where several streams share the GPU: there a CTA that has to wait for
+// its place would start its whole share late, and smaller shares even that out
+// (grouped launches with 1, 2, 4, 8 waves: 16 mixed boxes of 64-256^3 9105, 9008,
+// 9005, 9020 us, 48 of 64^3 1221, 1201, 1197, 1201).  Per-box launches have no
+// use for it (8 of 192^3 x 3 in one graph 1174 us with one wave, 1217 with four; 16
+// of 128^3 x 3 760 / 836; with 16 radii and more the same either way).
+constexpr int kGroupWaves = 4;
 
 template <class T> int dalloc(T** p, size_t count, const char* what) {
   cudaError_t e = cudaMalloc((void**)p, count * sizeof(T));
@@ -336,10 +340,16 @@ bool paired(const prc_d2z_ctx* c) {
 // 2573 / 2528, x 6 3355 / 3394, x 7 4169 / 3831, x 15 7.40 / 7.25 ms; 1024^3 x 3
 // 26.3 / 22.6); smaller grids win with any number.  The adjoint gains more from
 // pairs (256^3 x 3 343 / 338 us, 384^3 x 3 1271 / 1209, 512^3 x 3 2502 / 2276,
-// x 5 3258 / 3271, 1024^3 x 3 24.7 / 24.3 ms, x 5 31.8 / 35.1).
+// x 5 3258 / 3271, 1024^3 x 3 24.7 / 24.3 ms, x 5 31.8 / 35.1).  A box of a batch
+// shares the GPU with other streams' kernels: a filled half is then no longer
+// hidden by idle SMs, and costs its share (per-box launches in one graph, pairs
+// against single radii, us: 24 boxes of 96^3 x 3 582 / 553, x 5 720 / 770; 16 of
+// 128^3 x 3 760 / 623, x 15 1981 / 1904, x 31 3581 / 3524; 8 of 192^3 x 3 1174 / 999,
+// x 9 2280 / 2214, x 15 3394 / 3424; 6 of 256^3 x 5 2285 / 2193, x 7 2802 / 2808).
 bool in_pairs(const prc_d2z_ctx* c, int nb, bool adjoint) {
   if (!paired(c) || nb < 2) return false;
   const int N = c->N;
+  if (c->shared && nb % 2 && N >= 96 && N <= 256) return nb >= (N == 96 ? 5 : N == 128 ? 33 : N == 192 ? 13 : 7);
   if (N < 256) return true;
   if (adjoint) return nb % 2 == 0 || nb >= 5;
   if (N == 512) return nb >= (nb % 2 ? 21 : 6);
@@ -551,7 +561,7 @@ void run_tile(prc_d2z_ctx* c, int mode, TileSeg s0, TileSeg s1, int gy, int nb =
                 : (mode == TM_ACC) ? c->ksl.occ_tile_acc
                 : faithful         ? c->ksl.occ_win_faithful
                 : (mode == TM_WIN) ? c->ksl.occ_winv[wv] : c->ksl.occ_tile;
-  dim3 grid(grid_for(tiles, 1, occ * (mode == TM_WIN ? c->waves : 1), c->sms), gy, 1);
+  dim3 grid(grid_for(tiles, 1, occ, c->sms), gy, 1);
   if (mode == TM_WIN && c->N <= 128) {
     // fewer tiles than two waves of resident CTAs: the sweep's radii are
     // split over blockIdx.y as well (the kernels of grids up to 128 read
@@ -639,7 +649,7 @@ void enqueue_sweeps(prc_d2z_ctx* c, float* d_z, uint8_t* d_am, double* sig, floa
     {
       Prof pf(c, PRC_KIND_C2R_Z);
       if (pair)
-        c->ks->pair_c2r(c->ksl, grid_for(N * N, c->ksl.pair_lines, c->ksl.occ_pair_c2r * c->waves, c->sms), c->st, sa);
+        c->ks->pair_c2r(c->ksl, grid_for(N * N, c->ksl.pair_lines, c->ksl.occ_pair_c2r, c->sms), c->st, sa);
       else
         c->ks->c2r_z(c->ksl, grid_for(N * N, c->ksl.c2r_lines, c->ksl.occ_c2r, c->sms), c->st, sa);
     }
@@ -904,13 +914,14 @@ void batch_enqueue_grouped(prc_d2z_batch* b, const float* const* delta, float* c
     const BatchGroup& g = b->groups[gi];
     const prc_d2z_ctx* c0 = b->ctx[g.boxes[0]];
     const KernelSet& ks = c0->ksl;
-    const int N = g.N, H = N / 2, sms = c0->sms, nbox = (int)g.boxes.size(), waves = c0->waves;
+    const int N = g.N, H = N / 2, sms = c0->sms, nbox = (int)g.boxes.size();
     const long long NN = c0->NN;
     float2* S0 = c0->spec;
     float2* U0 = c0->slots;
     ks.r2c_z_mb(ks, grid_for(N * N * nbox, ks.line_groups, ks.occ_mb_r2c, sms), g.st,
                 reinterpret_cast<const BoxR2c*>(b->d_tab + g.o_r2c), nbox, c0->tw);
     const KernelSet::Grouped& mb = ks.mb[g.pair];
+    const int waves = g.pair && b->streams.size() > 1 ? kGroupWaves : 1;
     const int step = g.pair ? 2 : 1;  // radii per slot of the y pass
     auto cols = [&](int mode, TileSeg s0, TileSeg s1, size_t o, int nboxes, int gy, const int* nvb) {
       TileArgs a;
@@ -930,7 +941,7 @@ void batch_enqueue_grouped(prc_d2z_batch* b, const float* const* delta, float* c
       if (nvb)
         for (int y = 0; y < gy; ++y) a.nvb[y] = nvb[y];
       const int tpb = s0.n_outer * s0.tpo + s1.n_outer * s1.tpo;
-      const int occ = mode == TM_WIN ? mb.occ_win * (g.pair ? waves : 1) : mode == TM_INV ? mb.occ_inv : ks.occ_mb_tile;
+      const int occ = mode == TM_WIN ? mb.occ_win * waves : mode == TM_INV ? mb.occ_inv : ks.occ_mb_tile;
       const dim3 grid(grid_for(tpb * (nvb ? nvb[0] : nboxes), 1, occ, sms), gy, 1);
       if (mode == TM_FWD) ks.tile_mb(ks, grid, g.st, a);
       else mb.tile(ks, mode, grid, g.st, a);
@@ -959,7 +970,7 @@ void batch_enqueue_grouped(prc_d2z_batch* b, const float* const* delta, float* c
       sa.argmax = argmax ? argmax[g.sw_box[sw][0]] : nullptr;
       sa.box = reinterpret_cast<const BoxLine*>(b->d_tab + g.o_line[sw]);
       sa.nbox = ns;
-      mb.c2r_z(ks, grid_for(N * N * ns, mb.lines, mb.occ_c2r * (g.pair ? waves : 1), sms), g.st, sa);
+      mb.c2r_z(ks, grid_for(N * N * ns, mb.lines, mb.occ_c2r * waves, sms), g.st, sa);
       launches += 2;
     }
     launches += 1;
@@ -1721,7 +1732,7 @@ int prc_d2z_batch_create(int n_boxes, const prc_d2z_desc* descs, int n_streams, 
       prc_d2z_desc d = descs[order[k]];
       d.stream = b->streams[k % n_streams];
       s = create_at(&d, level, &b->ctx[order[k]]);
-      if (s == PRC_OK && n_streams > 1) b->ctx[order[k]]->waves = kBatchWaves;
+      if (s == PRC_OK) b->ctx[order[k]]->shared = n_streams > 1;
     }
     if (s != PRC_OK)
       for (prc_d2z_ctx*& c : b->ctx) {

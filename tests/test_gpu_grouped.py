@@ -1,5 +1,6 @@
-"""Grouped launches on single radii and on pairs: every box of a grouped size
-joins one, whatever its radius count and batch, and gets the per-box result."""
+"""Batches on single radii and on pairs: every box of a grouped size joins a
+grouped launch, whatever its radius count and batch, and a box gets the per-box
+result in grouped and in per-box launches on either side of their lines."""
 import numpy as np
 import pytest
 
@@ -28,8 +29,8 @@ SPEC = {
 
 
 @pytest.mark.parametrize("name", list(SPEC))
-@pytest.mark.parametrize("with_argmax", [False, True])
-def test_grouped_boxes_match_per_box(name, with_argmax):
+@pytest.mark.parametrize("mode,with_argmax", [("grouped", False), ("grouped", True), ("graph", True), ("loop", False)])
+def test_boxes_match_per_box(name, mode, with_argmax):
     import torch
     boxes = [_box(*s) for s in SPEC[name]]
     gen = torch.Generator(device="cuda").manual_seed(len(name))
@@ -42,7 +43,7 @@ def test_grouped_boxes_match_per_box(name, with_argmax):
     for _ in range(2):  # the second call replays the captured graph
         out = [torch.full_like(d, -3.0) for d in fields]
         am = [torch.full(d.shape, 7, dtype=torch.uint8, device="cuda") for d in fields] if with_argmax else None
-        batch.forward(fields, out, am, mode="grouped")
+        batch.forward(fields, out, am, mode=mode)
         for i, (z, a) in enumerate(ref):
             assert torch.equal(out[i], z), SPEC[name][i]
             assert not with_argmax or torch.equal(am[i], a), SPEC[name][i]
