@@ -333,27 +333,28 @@ bool paired(const prc_d2z_ctx* c) {
 }
 
 // Whether a sweep of nb radii runs in pairs.  The last pair of an odd sweep is
-// filled up, and a pair of radii costs nearly two, so from 256^3 on few and odd
-// radii stay with the single-radius kernels.  The lines are where one whole
-// step took the same time either way (pairs against single radii: 256^3 x 5
-// 435 / 396 us, x 11 705 / 704; 384^3 x 5 1654 / 1603, x 7 2064 / 2089; 512^3 x 4
-// 2573 / 2528, x 6 3355 / 3394, x 7 4169 / 3831, x 15 7.40 / 7.25 ms; 1024^3 x 3
-// 26.3 / 22.6); smaller grids win with any number.  The adjoint gains more from
-// pairs (256^3 x 3 343 / 338 us, 384^3 x 3 1271 / 1209, 512^3 x 3 2502 / 2276,
-// x 5 3258 / 3271, 1024^3 x 3 24.7 / 24.3 ms, x 5 31.8 / 35.1).  A box of a batch
-// shares the GPU with other streams' kernels: a filled half is then no longer
-// hidden by idle SMs, and costs its share (per-box launches in one graph, pairs
-// against single radii, us: 24 boxes of 96^3 x 3 582 / 553, x 5 720 / 770; 16 of
+// filled up, and a pair of radii costs nearly two, so few and odd radii stay with
+// the single-radius kernels.  The lines are where one whole step took the same
+// time either way.  Pairs against single radii, forward: 128^3 x 3 60.8 / 59.5 us, x 5
+// 71.7 / 74.8; 192^3 x 3 155 / 150, x 5 202 / 208; 256^3 x 9 595 / 584, x 11 688 / 688,
+// x 13 778 / 791; 384^3 x 5 1620 / 1552, x 7 2020 / 2033; 512^3 x 2 1753 / 1682, x 4
+// 2527 / 2550, x 15 7.42 / 7.39 ms, x 17 8.19 / 8.28; 768^3 x 5 15.1 / 14.6, x 7 18.8 /
+// 19.0; 1024^3 x 3 24.4 / 23.0, x 5 31.7 / 32.4; smaller grids win with any number
+// (64^3 x 3 29.7 / 31.5 us).  The adjoint gains more from pairs: 192^3 x 3 162 / 160
+// us; 256^3 x 3 306 / 302, x 5 397 / 425; 384^3 x 3 1208 / 1163, x 5 1619 / 1683; 512^3
+// x 3 2462 / 2231, x 5 3224 / 3227; 768^3 x 3 11.3 / 11.1 ms, x 5 15.0 / 16.2; 1024^3 x
+// 3 23.3 / 24.3.  A box of a batch shares the GPU with other streams' kernels: a
+// filled half is then no longer hidden by idle SMs, and costs its share (per-box
+// launches in one graph, us: 24 boxes of 96^3 x 3 582 / 553, x 5 720 / 770; 16 of
 // 128^3 x 3 760 / 623, x 15 1981 / 1904, x 31 3581 / 3524; 8 of 192^3 x 3 1174 / 999,
 // x 9 2280 / 2214, x 15 3394 / 3424; 6 of 256^3 x 5 2285 / 2193, x 7 2802 / 2808).
 bool in_pairs(const prc_d2z_ctx* c, int nb, bool adjoint) {
   if (!paired(c) || nb < 2) return false;
   const int N = c->N;
-  if (c->shared && nb % 2 && N >= 96 && N <= 256) return nb >= (N == 96 ? 5 : N == 128 ? 33 : N == 192 ? 13 : 7);
-  if (N < 256) return true;
-  if (adjoint) return nb % 2 == 0 || nb >= 5;
-  if (N == 512) return nb >= (nb % 2 ? 21 : 6);
-  return nb % 2 == 0 || nb >= (N == 256 ? 11 : 7);
+  if (nb % 2 == 0) return N != 512 || adjoint || nb >= 4;
+  if (adjoint) return nb >= (N < 256 || N == 1024 ? 3 : 5);
+  if (c->shared && N >= 96 && N <= 256) return nb >= (N == 96 ? 5 : N == 128 ? 33 : N == 192 ? 13 : 7);
+  return nb >= (N < 128 ? 3 : N < 256 || N == 1024 ? 5 : N == 256 ? 11 : N == 512 ? 17 : 7);
 }
 
 // The next sweep of a context with `left` radii to go: its number of radii, and
