@@ -326,10 +326,11 @@ template <class T> int dalloc(T** p, size_t count, const char* what) {
 }
 
 // The pair kernels (fft2.cuh) are left for the single-radius ones by the
-// faithful window, by a tuned window variant, and where there is one radius or
-// one slot.
-bool paired(const prc_d2z_ctx* c) {
-  return c->ksl.pair && !(c->flags & PRC_FLAG_FAITHFUL_WINDOW) && c->win_var == 0 && c->nr > 1 && c->slots_b > 1;
+// faithful window, by a tuned window variant (the adjoint has none: 256^3 x 16
+// 914 us in pairs, 1157 without), and where there is one radius or one slot.
+bool paired(const prc_d2z_ctx* c, bool adjoint) {
+  return c->ksl.pair && !(c->flags & PRC_FLAG_FAITHFUL_WINDOW) && (adjoint || c->win_var == 0) && c->nr > 1 &&
+         c->slots_b > 1;
 }
 
 // Whether a sweep of nb radii runs in pairs.  The last pair of an odd sweep is
@@ -349,7 +350,7 @@ bool paired(const prc_d2z_ctx* c) {
 // 128^3 x 3 760 / 623, x 15 1981 / 1904, x 31 3581 / 3524; 8 of 192^3 x 3 1174 / 999,
 // x 9 2280 / 2214, x 15 3394 / 3424; 6 of 256^3 x 5 2285 / 2193, x 7 2802 / 2808).
 bool in_pairs(const prc_d2z_ctx* c, int nb, bool adjoint) {
-  if (!paired(c) || nb < 2) return false;
+  if (!paired(c, adjoint) || nb < 2) return false;
   const int N = c->N;
   if (nb % 2 == 0) return N != 512 || adjoint || nb >= 4;
   if (adjoint) return nb >= (N < 256 || N == 1024 ? 3 : 5);
@@ -370,7 +371,7 @@ bool in_pairs(const prc_d2z_ctx* c, int nb, bool adjoint) {
 // 35.1).
 int next_sweep(const prc_d2z_ctx* c, int left, bool adjoint, bool* pair) {
   *pair = false;
-  if (!paired(c)) return std::min(left, c->B);
+  if (!paired(c, adjoint)) return std::min(left, c->B);
   const int N = c->N;
   int nb = std::min(left, c->B % 2 && c->B < c->slots_b ? c->B + 1 : c->B);
   if (nb % 2 && nb >= c->slots_b) {
