@@ -4,7 +4,8 @@ For a grid side N and a radius count it times every compiled window-pass
 variant (tile width and radix plan, prc_d2z_win_variants) at several radius
 batches (radii per sweep) on a synthetic field of this library's generator,
 and keeps the fastest pair in a JSON cache keyed by the device name, its SM
-count, N and the radius count.  For batches of boxes it also picks the number
+count, the library's contents (another build's kernels have other times), N and
+the radius count.  For batches of boxes it also picks the number
 of streams by timing the whole captured batch.
 
     from prc_d2z import autotune
@@ -17,12 +18,15 @@ transforms (the tests check every variant against the default).
 """
 from __future__ import annotations
 
+import functools
+import hashlib
 import json
 import os
 import statistics
 
 import numpy as np
 
+from . import _lib
 from . import CLParameters, Delta2Zreion, Parameters, compute_tables, fields, win_variants
 
 __all__ = ["tuned", "tune", "tune_batch_streams", "cache_path", "candidates"]
@@ -37,6 +41,12 @@ def _device_key() -> str:
     import torch
     props = torch.cuda.get_device_properties(torch.cuda.current_device())
     return f"{props.name}|sm{props.multi_processor_count}"
+
+
+@functools.lru_cache(maxsize=None)
+def _library_key(path: str) -> str:
+    with open(path, "rb") as fh:
+        return hashlib.sha256(fh.read()).hexdigest()[:16]
 
 
 def _load(path):
@@ -85,7 +95,7 @@ def tune(N: int, n_radii: int, reps: int = 5, force: bool = False, path: str | N
     import torch
     path = path or cache_path()
     data = _load(path)
-    key = f"{_device_key()}|N={N}|nr={n_radii}"
+    key = f"{_device_key()}|lib={_library_key(_lib.load()._name)}|N={N}|nr={n_radii}"
     if key in data and not force:
         return data[key]
     box = 1.5 * N
