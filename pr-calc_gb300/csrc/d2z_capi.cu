@@ -973,7 +973,7 @@ void batch_enqueue_grouped(prc_d2z_batch* b, const float* const* delta, float* c
       sa.box = reinterpret_cast<const BoxLine*>(b->d_tab + g.o_line[sw]);
       sa.nbox = ns;
       mb.c2r_z(ks, grid_for(N * N * ns, mb.lines, mb.occ_c2r * waves, sms), g.st, sa);
-      launches += 2;
+      launches += 1;
     }
     launches += 1;
     cudaEventRecord(b->gev[gi], g.st);

@@ -63,3 +63,14 @@ def test_few_radii_keep_grouped_launches(N, nr):
         counts.append(batch.launches())
         batch.close()
     assert counts[0] == counts[1]
+
+
+@pytest.mark.parametrize("radius_batch,sweeps", [(8, 1), (4, 2)])
+def test_grouped_launch_count(radius_batch, sweeps):
+    """Three forward passes and three passes a sweep."""
+    import torch
+    d = [torch.zeros((32, 32, 32), device="cuda") for _ in range(3)]
+    batch = prc_d2z.Batch([_box(32, 8, radius_batch)] * 3, n_streams=1)
+    batch.forward(d, [torch.empty_like(x) for x in d], mode="grouped")
+    assert batch.launches() == 3 + 3 * sweeps
+    batch.close()
