@@ -17,23 +17,30 @@
 namespace prc {
 
 // Tile width and resident CTAs per SM of the pair passes (plans as in CCfg).
-// Twelve elements a lane leave room for a third y CTA of 256 threads (85
+// Twelve elements a lane leave room for a third y CTA of 256 threads (80
 // registers): 384^3 x 24 1.98 -> 1.83 ms, 768^3 x 16 12.6 -> 11.6; a fifth window CTA
-// of 128 at 192 (x 41 0.305 -> 0.294 ms).  (Ten at 128 would gain 0.001 ms there
-// and lose 0.02 in TM_ACC.)  At 1024 shared memory holds two y CTAs whatever MINB
-// says; 85 registers took 18.1 ms for 12 radii, 128 18.5.  With sixteen elements
-// elsewhere the same only spills (512^3 x 32: y 5.44 -> 5.51, window 4.12 -> 4.27).
+// of 128 at 192 (x 41 0.306 -> 0.295 ms).  (Ten at 128 would gain 0.001 ms there.)
+// At 1024 shared memory holds two y CTAs whatever MINB says; 80 registers took
+// 18.0 ms for 12 radii, 128 18.4.  With sixteen elements elsewhere the same only
+// spills (512^3 x 32: y 5.44 -> 5.51, window 4.12 -> 4.27).
+// The accumulating x pass (MINBACC) holds a tile's values and windows at once:
+// sixteen CTAs spill it at 32 and 64, and eight take 42.9 us against 55.2 (32^3 x
+// 64) and 45.0 against 59.9 (64^3 x 64; twelve 47.1).  Elsewhere it takes what the
+// window pass does, also where that spills: 192^3 x 41 five CTAs (52 bytes) 303.9,
+// four 308.6; 512^3 x 32 four (16 bytes) 3753, three 3891; 96^3 x 32 eight or six
+// 42.9; 128^3 x 32 eight 61.9, seven 63.5; 256^3 x 32 four 418, three 441; 384^3 x
+// 24 four 1842, three 1930.
 template <int N> struct C2Cfg { static constexpr bool on = false; };
-template <> struct C2Cfg<32> { static constexpr bool on = true; static constexpr int T = 16, MINB = 16, TWIN = 16, MINBWIN = 16, XB = 8; };
-template <> struct C2Cfg<64> { static constexpr bool on = true; static constexpr int T = 8, MINB = 16, TWIN = 8, MINBWIN = 16, XB = 8; };
-template <> struct C2Cfg<96> { static constexpr bool on = true; static constexpr int T = 8, MINB = 8, TWIN = 8, MINBWIN = 8, XB = 8; };
-template <> struct C2Cfg<128> { static constexpr bool on = true; static constexpr int T = 8, MINB = 8, TWIN = 8, MINBWIN = 8, XB = 8; };
-template <> struct C2Cfg<192> { static constexpr bool on = true; static constexpr int T = 8, MINB = 5, TWIN = 8, MINBWIN = 5, XB = 8; };
-template <> struct C2Cfg<256> { static constexpr bool on = true; static constexpr int T = 8, MINB = 4, TWIN = 8, MINBWIN = 4, XB = 8; };
-template <> struct C2Cfg<384> { static constexpr bool on = true; static constexpr int T = 8, MINB = 3, TWIN = 4, MINBWIN = 4, XB = 8; };
-template <> struct C2Cfg<512> { static constexpr bool on = true; static constexpr int T = 8, MINB = 2, TWIN = 4, MINBWIN = 4, XB = 4; };
-template <> struct C2Cfg<768> { static constexpr bool on = true; static constexpr int T = 4, MINB = 3, TWIN = 4, MINBWIN = 2, XB = 4; };
-template <> struct C2Cfg<1024> { static constexpr bool on = true; static constexpr int T = 4, MINB = 3, TWIN = 8, MINBWIN = 1, XB = 4; };
+template <> struct C2Cfg<32> { static constexpr bool on = true; static constexpr int T = 16, MINB = 16, TWIN = 16, MINBWIN = 16, MINBACC = 8, XB = 8; };
+template <> struct C2Cfg<64> { static constexpr bool on = true; static constexpr int T = 8, MINB = 16, TWIN = 8, MINBWIN = 16, MINBACC = 8, XB = 8; };
+template <> struct C2Cfg<96> { static constexpr bool on = true; static constexpr int T = 8, MINB = 8, TWIN = 8, MINBWIN = 8, MINBACC = 8, XB = 8; };
+template <> struct C2Cfg<128> { static constexpr bool on = true; static constexpr int T = 8, MINB = 8, TWIN = 8, MINBWIN = 8, MINBACC = 8, XB = 8; };
+template <> struct C2Cfg<192> { static constexpr bool on = true; static constexpr int T = 8, MINB = 5, TWIN = 8, MINBWIN = 5, MINBACC = 5, XB = 8; };
+template <> struct C2Cfg<256> { static constexpr bool on = true; static constexpr int T = 8, MINB = 4, TWIN = 8, MINBWIN = 4, MINBACC = 4, XB = 8; };
+template <> struct C2Cfg<384> { static constexpr bool on = true; static constexpr int T = 8, MINB = 3, TWIN = 4, MINBWIN = 4, MINBACC = 4, XB = 8; };
+template <> struct C2Cfg<512> { static constexpr bool on = true; static constexpr int T = 8, MINB = 2, TWIN = 4, MINBWIN = 4, MINBACC = 4, XB = 4; };
+template <> struct C2Cfg<768> { static constexpr bool on = true; static constexpr int T = 4, MINB = 3, TWIN = 4, MINBWIN = 2, MINBACC = 2, XB = 4; };
+template <> struct C2Cfg<1024> { static constexpr bool on = true; static constexpr int T = 4, MINB = 3, TWIN = 8, MINBWIN = 1, MINBACC = 1, XB = 4; };
 
 // Layout of a pair slot's main array: blocks of XB planes ix, in a block the
 // order (iy, kz / T, ix % XB, kz % T) with T the window pass's tile width, so
@@ -73,7 +80,7 @@ template <int N, int MODE> struct CK2 {
   static constexpr bool XP = MODE == TM_WIN || MODE == TM_ACC;  // an x pass: tiles of the slot's pieces
   static constexpr int H = N / 2, T = XP ? C2Cfg<N>::TWIN : C2Cfg<N>::T;
   static constexpr int E = P::E, G = N / E, THREADS = T * G, EH = E / 2;
-  static constexpr int MINB = XP ? C2Cfg<N>::MINBWIN : C2Cfg<N>::MINB;
+  static constexpr int MINB = MODE == TM_ACC ? C2Cfg<N>::MINBACC : XP ? C2Cfg<N>::MINBWIN : C2Cfg<N>::MINB;
   static_assert(T == 16 || (T == 8 && G >= 4) || (T == 4 && G >= 8), "lane layouts");
   static_assert(THREADS % 32 == 0 && H % T == 0, "whole warps, whole tiles");
   static constexpr int TW = (PlanRun<P>::TW + 1) & ~1;
