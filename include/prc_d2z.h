@@ -255,7 +255,7 @@ int prc_d2z_correct(prc_d2z_ctx* ctx, const float* zvz, float* zreion, int zreio
 /* Adjoint of prc_d2z_forward (no reference counterpart: the reference has no
  * gradient).  dL_dz (N^3) and argmax (N^3) -> dL/d delta_lin (N^3) and
  * dL/dB_r (n_radii doubles, optional).  The host maps dL/dB_r to dL/dzeta and
- * dL/dM_min with prc_barrier_grad. */
+ * dL/dM_min (prc_d2z.autograd.param_gradients). */
 int prc_d2z_backward(prc_d2z_ctx* ctx, const float* dL_dz, const uint8_t* argmax,
                      int in_on_device, float* dL_ddelta, int out_on_device,
                      double* dL_dB);
@@ -279,13 +279,14 @@ int prc_d2z_last_launches(prc_d2z_ctx* ctx, int* n);
  *   PRC_BATCH_GRAPH    the same launches captured once into a CUDA graph and
  *                      replayed with one launch per call (captured again when
  *                      the pointers change);
- *   PRC_BATCH_GROUPED  the boxes of each grid size form a group and every pass
+ *   PRC_BATCH_GROUPED  the boxes of each grid size form a group (or two, one on
+ *                      single radii, one on pairs of radii) and every pass
  *                      of the step runs as ONE launch over all boxes of the
  *                      group: resident CTAs walk the (box, tile) or (box, line
  *                      group) items of that pass, with each box's pointers,
  *                      radius count and constants read from device tables;
  *                      the groups share out the n_streams streams (largest
- *                      grid size first), all captured once into a CUDA graph (about 3 + 3 x sweeps launches per grid size
+ *                      grid size first), all captured once into a CUDA graph (3 + 3 x sweeps launches per group
  *                      instead of as many per box).  The tables are rewritten
  *                      at every call, so new pointers need no new capture.
  *                      Grid sizes up to 256 except 8..24 and 48 have grouped

@@ -93,8 +93,10 @@ template <int N, int MODE> struct CK2 {
   // the pass from 0.635 to 0.94 ms for 32 radii, and at 1024^3 two CTAs' shared
   // memory leaves too little of it alone (22.1 ms against 18.5 for 12 radii).
   // The copies take one more trip through shared memory: 0.642 against 0.635
-  // ms at 256, 0.381 against 0.356 at 192^3 x 41, 1.404 against 1.364 at 384 x
-  // 16, so those sizes and the smaller ones load into registers.
+  // ms at 256 with the GPU to itself, 0.381 against 0.356 at 192^3 x 41, so 192
+  // and the smaller ones load into registers; so does 384, where the two are
+  // equal (three CTAs an SM, 24 radii: 1.822 against 1.830 ms, the adjoint's y
+  // pass 1.827 against 1.825).
   static constexpr bool ASYNC = (MODE == TM_INV || MODE == TM_FWD) && N >= 256 && N != 384;
   // stage twiddles, exchange buffer, (x passes) the spectrum tile or the sums
   static constexpr size_t bytes = (size_t)TW * 8 + (size_t)ROWS * T * 16 + (XP ? (size_t)N * T * 8 : 0);

@@ -130,7 +130,7 @@ struct TileArgs {
   float dk, kmax;          // faithful window: dk = 2 pi / box and kmax = dk * N, in float
   float kr[kMaxBatch];     // dk * R_b (faithful window: R_b)
   // grouped launches: the boxes (sorted by nb, largest first), their count,
-  // and per pair y of the inverse y pass the number of boxes with more pairs
+  // and per slot (pair) y of the inverse y pass the number of boxes with more
   const BoxCol* box;
   int nbox;
   int nvb[kMaxBatch];
