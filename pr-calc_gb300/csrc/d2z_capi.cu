@@ -204,7 +204,7 @@ struct prc_d2z_ctx {
   int win_var = 0;   // window-pass variant (prc_d2z_tune)
   int slots_b = 0;   // radius slots allocated (one more than B for an odd B of paired sweeps)
   long long spare = 0;  // bytes of them taken from the reserve (SlotPlan)
-  bool shared = false;  // a batch's box: other streams' kernels share the GPU
+  int shared = 0;    // a box of a batch on several streams: its boxes of this size
   long long NN = 0, slot_f2 = 0;
   double box = 0, A = 0, dinit = 1;
   std::vector<double> R, Bb;
@@ -305,14 +305,20 @@ int grid_for(int items, int per_cta, int occ, int sms) {
   return (int)(need < cap ? need : cap);
 }
 
-// A pass is one wave of resident CTAs, but for the window and z passes of groups
-// on pairs where several streams share the GPU: there a CTA that has to wait for
-// its place would start its whole share late, and smaller shares even that out
-// (grouped launches with 1, 2, 4, 8 waves: 16 mixed boxes of 64-256^3 9105, 9008,
-// 9005, 9020 us, 48 of 64^3 1221, 1201, 1197, 1201).  Per-box launches have no
-// use for it (8 of 192^3 x 3 in one graph 1174 us with one wave, 1217 with four; 16
-// of 128^3 x 3 760 / 836; with 16 radii and more the same either way).
-constexpr int kGroupWaves = 4;
+// A pass is one wave of resident CTAs, but for the window and z passes on pairs
+// where several streams share the GPU: there a CTA that has to wait for its place
+// would start its whole share late, and smaller shares even that out (grouped
+// launches with 1, 2, 4, 8 waves: 16 mixed boxes of 64-256^3 9105, 9008, 9005, 9020
+// us, 48 of 64^3 1221, 1201, 1197, 1201).  Per-box launches gain from it beside boxes
+// of other sizes (five boxes of 32-256^3 x 8-15 in one graph 1299 -> 1237 us, six of x
+// 20-34 2307 -> 2254), and lose among many boxes of one size with few radii (8 of
+// 192^3 x 3 1174 us with one wave, 1217 with four; 16 of 128^3 x 3 760 / 836, x 16 1981
+// / 2020, x 24 2776 / 2796).
+constexpr int kSharedWaves = 4;
+constexpr int kManyBoxes = 6;
+int waves(const prc_d2z_ctx* c, int nb, bool pair) {
+  return c->shared && pair && (nb >= 20 || c->shared < kManyBoxes) ? kSharedWaves : 1;
+}
 
 template <class T> int dalloc(T** p, size_t count, const char* what) {
   cudaError_t e = cudaMalloc((void**)p, count * sizeof(T));
@@ -348,13 +354,19 @@ bool paired(const prc_d2z_ctx* c, bool adjoint) {
 // filled half is then no longer hidden by idle SMs, and costs its share (per-box
 // launches in one graph, us: 24 boxes of 96^3 x 3 582 / 553, x 5 720 / 770; 16 of
 // 128^3 x 3 760 / 623, x 15 1981 / 1904, x 31 3581 / 3524; 8 of 192^3 x 3 1174 / 999,
-// x 9 2280 / 2214, x 15 3394 / 3424; 6 of 256^3 x 5 2285 / 2193, x 7 2802 / 2808).
+// x 9 2280 / 2214, x 15 3394 / 3424; 6 of 256^3 x 5 2285 / 2193, x 7 2802 / 2808, x 9
+// 3338 / 3425).  It costs less beside boxes of other sizes (five boxes of 32 to 256^3,
+// one of 128^3 x 11 among them, 1237 / 1303), so the lines at 128 and 192 lie lower
+// with few boxes of the size.
 bool in_pairs(const prc_d2z_ctx* c, int nb, bool adjoint) {
   if (!paired(c, adjoint) || nb < 2) return false;
   const int N = c->N;
   if (nb % 2 == 0) return N != 512 || adjoint || nb >= 4;
   if (adjoint) return nb >= (N < 256 || N == 1024 ? 3 : 5);
-  if (c->shared && N >= 96 && N <= 256) return nb >= (N == 96 ? 5 : N == 128 ? 33 : N == 192 ? 13 : 7);
+  if (c->shared && N >= 96 && N <= 256) {
+    const bool many = c->shared >= kManyBoxes;
+    return nb >= (N == 96 ? 5 : N == 128 ? (many ? 21 : 9) : N == 192 ? (many ? 11 : 7) : 9);
+  }
   return nb >= (N < 128 ? 3 : N < 256 || N == 1024 ? 5 : N == 256 ? 11 : N == 512 ? 17 : 7);
 }
 
@@ -563,7 +575,7 @@ void run_tile(prc_d2z_ctx* c, int mode, TileSeg s0, TileSeg s1, int gy, int nb =
                 : (mode == TM_ACC) ? c->ksl.occ_tile_acc
                 : faithful         ? c->ksl.occ_win_faithful
                 : (mode == TM_WIN) ? c->ksl.occ_winv[wv] : c->ksl.occ_tile;
-  dim3 grid(grid_for(tiles, 1, occ, c->sms), gy, 1);
+  dim3 grid(grid_for(tiles, 1, occ * (mode == TM_WIN ? waves(c, nb, pair) : 1), c->sms), gy, 1);
   if (mode == TM_WIN && c->N <= 128) {
     // fewer tiles than two waves of resident CTAs: the sweep's radii are
     // split over blockIdx.y as well (the kernels of grids up to 128 read
@@ -651,7 +663,7 @@ void enqueue_sweeps(prc_d2z_ctx* c, float* d_z, uint8_t* d_am, double* sig, floa
     {
       Prof pf(c, PRC_KIND_C2R_Z);
       if (pair)
-        c->ks->pair_c2r(c->ksl, grid_for(N * N, c->ksl.pair_lines, c->ksl.occ_pair_c2r, c->sms), c->st, sa);
+        c->ks->pair_c2r(c->ksl, grid_for(N * N, c->ksl.pair_lines, c->ksl.occ_pair_c2r * waves(c, nb, true), c->sms), c->st, sa);
       else
         c->ks->c2r_z(c->ksl, grid_for(N * N, c->ksl.c2r_lines, c->ksl.occ_c2r, c->sms), c->st, sa);
     }
@@ -699,6 +711,7 @@ struct prc_d2z_batch {
   int exec_mode = -1;            // batch mode the graph was captured in
   // grouped launches
   std::vector<BatchGroup> groups;
+  std::vector<char> joined;      // box i runs in a group (else per box in the same graph)
   std::vector<cudaEvent_t> gev;  // one join event per group
   char* h_tab = nullptr;         // host image of the tables (pinned: the copy is asynchronous)
   size_t tab_bytes = 0;
@@ -737,7 +750,7 @@ void batch_enqueue(prc_d2z_batch* b, const float* const* delta, float* const* zr
 
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-// A box joins a grouped launch when its size has grouped kernels and it does
+// A box can join a grouped launch when its size has grouped kernels and it does
 // not ask for the faithful window.  (A tuned window variant is not used there.)
 bool groupable(const prc_d2z_ctx* c) { return c->ksl.grouped && !(c->flags & PRC_FLAG_FAITHFUL_WINDOW); }
 // Radii per sweep of a grouped box on pairs (its window variant does not matter).
@@ -749,15 +762,18 @@ int pair_len(const prc_d2z_ctx* c) {
 // do its first sweep faster.  A whole grouped call in pairs against single radii, us: 24
 // boxes of 96^3 x 3 505 / 475, x 5 630 / 629; 16 of 128^3 x 3 674 / 584, x 7 1025
 // / 1009, x 9 1193 / 1218; 8 of 192^3 x 3 1130 / 1059, x 5 1470 / 1494; 6 of 256^3 x
-// 2 1274 / 1223, x 4 1847 / 1844, x 13 4545 / 4589; 32 of 64^3 x 3 286 / 281, x 5
+// 2 1274 / 1223, x 4 1847 / 1844, x 9 - / 3428, x 12 4002 / -, x 13 4545 / 4589; 32 of 64^3 x 3 286 / 281, x 5
 // 334 / 333, x 9 432 / 451.
 bool pairs_first(const prc_d2z_ctx* c) {
   const int N = c->N, nb = std::min(pair_len(c), c->nr);
   if (nb % 2 == 0) return N < 256 || nb >= 4;
-  return nb >= (N >= 256 ? 13 : N == 128 ? 9 : N >= 96 ? 5 : 3);
+  return nb >= (N >= 256 ? 11 : N == 128 ? 9 : N >= 96 ? 5 : 3);
 }
 // Where pairs are better for half of a size's boxes or more, the others that can
-// join them do: a second group's launches cost more than their filled halves.
+// join them do: a second group's launches cost more than their filled halves.  At
+// 256^3 those of even sweeps do that have one to join, or are too few for a group
+// of single radii.
+constexpr int kFewBoxes = 4;
 bool grouped_pair(const prc_d2z_batch* b, const prc_d2z_ctx* c) {
   if (c->nr < 2 || c->slots_b < 2) return false;
   int boxes = 0, first = 0;
@@ -766,12 +782,13 @@ bool grouped_pair(const prc_d2z_batch* b, const prc_d2z_ctx* c) {
       ++boxes;
       first += pairs_first(o);
     }
-  return pairs_first(c) || (c->N < 256 && 2 * first >= boxes);
+  const bool even = std::min(pair_len(c), c->nr) % 2 == 0;
+  return pairs_first(c) || (c->N < 256 ? 2 * first >= boxes : even && (first > 0 || boxes < kFewBoxes));
 }
 int grouped_len(const BatchGroup& g, const prc_d2z_ctx* c) { return g.pair ? pair_len(c) : c->B; }
 
 // Groups of equal grid size, their sweeps and the layout of their tables.
-// Sizes without grouped kernels keep per-box launches (no group).
+// Boxes outside them (joined = 0) keep per-box launches.
 int batch_group_setup(prc_d2z_batch* b) {
   for (auto e : b->gev) cudaEventDestroy(e);
   b->groups.clear();
@@ -781,10 +798,29 @@ int batch_group_setup(prc_d2z_batch* b) {
   if (b->h_tab) cudaFreeHost(b->h_tab);
   b->h_tab = nullptr;
   b->tab_bytes = 0;
+  // Two groups of one size, one in pairs and one on single radii, run side by
+  // side up to 192^3; at 256^3, where each fills the GPU and its slots L2, the
+  // single ones run per box then (boxes of 5, 6, 7 and 9 radii on two streams
+  // 1810 us against 2076 in two groups; 8 of 64^3 x 1 and 8 x 8 140 us in two
+  // groups, 203 with the eight per box), and where they are few, too (two of 256^3
+  // x 2 and x 3 beside smaller boxes 568 us, 639 in a group; eight x 5 2973 and 2815).
+  std::vector<char> pair(b->n);
+  for (int i = 0; i < b->n; ++i) pair[i] = groupable(b->ctx[i]) && grouped_pair(b, b->ctx[i]);
+  b->joined.assign(b->n, 0);
+  for (int i = 0; i < b->n; ++i) {
+    int same = 0;
+    bool beside_pairs = false;
+    for (int j = 0; j < b->n; ++j)
+      if (b->ctx[j]->N == b->ctx[i]->N && groupable(b->ctx[j])) {
+        ++same;
+        beside_pairs |= pair[j];
+      }
+    b->joined[i] = groupable(b->ctx[i]) && (pair[i] || b->ctx[i]->N < 256 || (!beside_pairs && same >= kFewBoxes));
+  }
   std::vector<std::pair<int, bool>> sizes;  // (N, on pairs)
-  for (auto* c : b->ctx) {
-    const std::pair<int, bool> k(c->N, grouped_pair(b, c));
-    if (groupable(c) && std::find(sizes.begin(), sizes.end(), k) == sizes.end()) sizes.push_back(k);
+  for (int i = 0; i < b->n; ++i) {
+    const std::pair<int, bool> k(b->ctx[i]->N, pair[i]);
+    if (b->joined[i] && std::find(sizes.begin(), sizes.end(), k) == sizes.end()) sizes.push_back(k);
   }
   std::sort(sizes.begin(), sizes.end(), [](const auto& x, const auto& y) { return x > y; });
   size_t off = 0;
@@ -794,7 +830,7 @@ int batch_group_setup(prc_d2z_batch* b) {
     g.N = N;
     g.pair = size.second;
     for (int i = 0; i < b->n; ++i)
-      if (b->ctx[i]->N == N && groupable(b->ctx[i]) && grouped_pair(b, b->ctx[i]) == g.pair) {
+      if (b->joined[i] && b->ctx[i]->N == N && pair[i] == g.pair) {
         g.boxes.push_back(i);
         const prc_d2z_ctx* c = b->ctx[i];
         g.nsweeps = std::max(g.nsweeps, (c->nr + grouped_len(g, c) - 1) / grouped_len(g, c));
@@ -923,7 +959,7 @@ void batch_enqueue_grouped(prc_d2z_batch* b, const float* const* delta, float* c
     ks.r2c_z_mb(ks, grid_for(N * N * nbox, ks.line_groups, ks.occ_mb_r2c, sms), g.st,
                 reinterpret_cast<const BoxR2c*>(b->d_tab + g.o_r2c), nbox, c0->tw);
     const KernelSet::Grouped& mb = ks.mb[g.pair];
-    const int waves = g.pair && b->streams.size() > 1 ? kGroupWaves : 1;
+    const int gwaves = g.pair && b->streams.size() > 1 ? kSharedWaves : 1;
     const int step = g.pair ? 2 : 1;  // radii per slot of the y pass
     auto cols = [&](int mode, TileSeg s0, TileSeg s1, size_t o, int nboxes, int gy, const int* nvb) {
       TileArgs a;
@@ -943,7 +979,7 @@ void batch_enqueue_grouped(prc_d2z_batch* b, const float* const* delta, float* c
       if (nvb)
         for (int y = 0; y < gy; ++y) a.nvb[y] = nvb[y];
       const int tpb = s0.n_outer * s0.tpo + s1.n_outer * s1.tpo;
-      const int occ = mode == TM_WIN ? mb.occ_win * waves : mode == TM_INV ? mb.occ_inv : ks.occ_mb_tile;
+      const int occ = mode == TM_WIN ? mb.occ_win * gwaves : mode == TM_INV ? mb.occ_inv : ks.occ_mb_tile;
       const dim3 grid(grid_for(tpb * (nvb ? nvb[0] : nboxes), 1, occ, sms), gy, 1);
       if (mode == TM_FWD) ks.tile_mb(ks, grid, g.st, a);
       else mb.tile(ks, mode, grid, g.st, a);
@@ -972,17 +1008,17 @@ void batch_enqueue_grouped(prc_d2z_batch* b, const float* const* delta, float* c
       sa.argmax = argmax ? argmax[g.sw_box[sw][0]] : nullptr;
       sa.box = reinterpret_cast<const BoxLine*>(b->d_tab + g.o_line[sw]);
       sa.nbox = ns;
-      mb.c2r_z(ks, grid_for(N * N * ns, mb.lines, mb.occ_c2r * waves, sms), g.st, sa);
+      mb.c2r_z(ks, grid_for(N * N * ns, mb.lines, mb.occ_c2r * gwaves, sms), g.st, sa);
       launches += 1;
     }
     launches += 1;
     cudaEventRecord(b->gev[gi], g.st);
     cudaStreamWaitEvent(b->origin, b->gev[gi], 0);
   }
-  // sizes without grouped kernels: per-box launches
+  // boxes outside the groups: per-box launches
   for (int i = 0; i < b->n; ++i) {
     prc_d2z_ctx* c = b->ctx[i];
-    if (groupable(c)) continue;
+    if (b->joined[i]) continue;
     c->launches = 0;
     forward_r2c(c, delta[i], c->dinit);
     enqueue_sweeps(c, zreion[i], argmax ? argmax[i] : nullptr, nullptr);
@@ -1734,7 +1770,7 @@ int prc_d2z_batch_create(int n_boxes, const prc_d2z_desc* descs, int n_streams, 
       prc_d2z_desc d = descs[order[k]];
       d.stream = b->streams[k % n_streams];
       s = create_at(&d, level, &b->ctx[order[k]]);
-      if (s == PRC_OK) b->ctx[order[k]]->shared = n_streams > 1;
+      for (int i = 0; i < n_boxes && s == PRC_OK && n_streams > 1; ++i) b->ctx[order[k]]->shared += descs[i].N == d.N;
     }
     if (s != PRC_OK)
       for (prc_d2z_ctx*& c : b->ctx) {
@@ -1782,7 +1818,7 @@ int prc_d2z_batch_forward(prc_d2z_batch* b, const float* const* delta, float* co
              "batch tables");
     std::vector<const void*> key;
     for (int i = 0; i < b->n; ++i)
-      if (!groupable(b->ctx[i])) {
+      if (!b->joined[i]) {
         key.push_back(delta[i]);
         key.push_back(zreion[i]);
         key.push_back(argmax ? argmax[i] : nullptr);

@@ -57,7 +57,7 @@ def test_few_radii_keep_grouped_launches(N, nr):
     import torch
     d = [torch.zeros((N,) * 3, device="cuda") for _ in range(6)]
     counts = []
-    for n in (2, 6):
+    for n in (4, 6):
         batch = prc_d2z.Batch([_box(N, nr, 0)] * n, n_streams=2)
         batch.forward(d[:n], [torch.empty_like(x) for x in d[:n]], mode="grouped")
         counts.append(batch.launches())
